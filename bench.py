@@ -576,7 +576,7 @@ def run_ours(args, world, rank, local, collect=False):
             "roofline": ({"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                           "frac": achieved / peak, "peak_source": peak_kind,
                           "algorithmic_bytes_per_launch": per_launch_bytes,
-                          "kernel": ("cluster_sweep_kernel<POISSON>" if args.strategy != "grid_levels"
+                          "kernel": ("window_sweep_kernel<POISSON>" if args.strategy != "grid_levels"
                                      else "indep_sweep_kernel<POISSON>") + " (one launch per findMode attempt)",
                           "bytes": "per-coordinate algorithmic bytes (column entries and the row state they gather and update) of every sweep that ran, plus the objective checks",
                           "traffic": traffic} if WORKLOAD == "poisson_offset" else
@@ -712,8 +712,8 @@ def run_logistic_l1(args, world, rank, local, collect=False):
         "roofline": {"bound": "hbm", "achieved": total_bytes / ker_t / 1e9, "peak": peak, "unit": "GB/s",
                      "frac": total_bytes / ker_t / 1e9 / peak, "peak_source": peak_kind,
                      "algorithmic_bytes_per_launch": total_bytes / attempts,
-                     "kernel": ("resident_sweep_kernel<LOGISTIC> (one CTA, row state in shared memory)"
-                                if args.strategy in ("auto", "resident") else
+                     "kernel": ("window_sweep_kernel<LOGISTIC> (a cluster, row state in shared memory)"
+                                if args.strategy in ("auto", "resident", "levels") else
                                 f"{args.strategy} sweep of the independent-row engine"), "traffic": None,
                      "note": "1.1e5 entries per sweep: latency-bound, L2-resident"},
         "cpu_baseline": {"value": ref_fit["iterations"] * active * reps / t_ref, "unit": METRIC, "cores": 1,
@@ -1064,8 +1064,8 @@ def run_serve(args, world, rank, local, collect=False):
     if world > 1 and rank != 0:
         return  # one server per GPU box; replicas add nothing to a latency figure
     stream = synthetic.serving_stream(args.serve_requests, seed=11, **SERVE_RANGES)
-    # warm-up requests of every kind the trace holds (logistic fits on the resident and
-    # the cluster sweep, conditional logistic and Cox fits), so that each kernel has run once
+    # warm-up requests of every kind the trace holds (logistic fits on general and on fast
+    # slots, conditional logistic and Cox fits), so that each kernel has run once
     warm = synthetic.serving_stream(max(16, args.serve_slots + args.serve_fast_slots), seed=12, rate=1e3,
                                     K_range=(1e3, 3e4), J_range=(50, 200))
     srv = serve.Server(device=local, hbm_budget=150e9, slots=args.serve_slots, fast_slots=args.serve_fast_slots,
@@ -1155,8 +1155,8 @@ def serve_config(args, stream) -> dict:
             "fast_lane": "requests of at most 200,000 matrix entries, oldest first",
             "hbm_budget_bytes": 150e9,
             "step": "replay of the whole stream; latency = completion - arrival",
-            "strategy": "logistic: the resident sweep (one CTA) when the rows fit it, else the "
-                        "cluster sweep on the slot's share of the SMs; grouped models: the group sweep"}
+            "strategy": "logistic: the windowed sweep on the slot's share of the SMs; grouped models: "
+                        "the group sweep"}
 
 
 def _serve_cpu_latencies(stream, n: int):

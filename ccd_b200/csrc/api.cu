@@ -24,7 +24,6 @@
 #include "csr_device.h"
 #include "csr_host.h"
 #include "engine.h"
-#include "resident.h"
 
 namespace ccdb {
 
@@ -137,10 +136,10 @@ void Matrix::ensure_csr(cudaStream_t s) {
 Fit::~Fit() {
     for (void* p : {(void*)row, (void*)y, (void*)beta, (void*)hdelta, (void*)xjy, (void*)ptype,
                     (void*)pvar, (void*)st, (void*)grid_bar, (void*)red, (void*)xb_tmp, (void*)w,
-                    (void*)gh_parts, (void*)gh_out, (void*)d_batch_cols, (void*)d_batch_out,
-                    (void*)d_res_recs, (void*)d_res_rs})
+                    (void*)gh_parts, (void*)gh_out, (void*)d_batch_cols, (void*)d_batch_out})
         ctx->release(p);
     release_schedule();
+    release_window();
     if (group_engine()) cox_release();
 }
 
@@ -148,7 +147,7 @@ void Fit::release_schedule() {
     if (!sched) return;
     for (void* p : {(void*)sched->segs, (void*)sched->cta_seg, (void*)sched->tasks,
                     (void*)sched->level_need, (void*)sched->level_done, (void*)sched->col_arrive,
-                    (void*)sched->partials, (void*)sched->level_split})
+                    (void*)sched->partials})
         ctx->release(p);
     sched.reset();
 }
@@ -184,7 +183,6 @@ IndepParams Fit::params() const {
         P.level_need = sched->level_need;
         P.col_arrive = sched->col_arrive;
         P.partials = sched->partials;
-        P.level_split = sched->level_split;
     }
     return P;
 }
@@ -282,50 +280,9 @@ void Fit::download_beta() {
     check_cuda(ctx->wait(), "beta sync");
 }
 
-int Fit::sweep_kind(const ccdb_mode_args& a) const {
-    return a.strategy == CCDB_SWEEP_GRID_LEVELS ? kSchedGrid : kSchedCluster;
-}
-
-void Fit::ensure_schedule(int kind) {
-    int C = 0;  // the cluster sweep's size: the largest resident, within the context's CTA share
-    if (kind == kSchedCluster) {
-        if (ctx->sweep_cluster < 0) {
-            int c = 0;
-            check_cuda(cluster_sweep_max_size(model, &c), "cluster occupancy");
-            ctx->sweep_cluster = c;
-        }
-        C = ctx->sweep_cluster;
-        if (C < 1) throw Error(CCDB_ERR_CUDA, "the cluster sweep kernel cannot be resident");
-        while (ctx->max_ctas > 0 && C > ctx->max_ctas && C > 1) C /= 2;
-    }
-    if (sched && sched->fixed == fixed && sched->kind == kind && (kind != kSchedCluster || sched->cluster == C))
-        return;
+void Fit::ensure_schedule() {
+    if (sched && sched->fixed == fixed) return;
     release_schedule();
-    if (kind == kSchedCluster) {
-        ScheduleParams sp;
-        sp.n_cta = C;
-        sp.warps_per_cta = indep_threads() / 32;
-        sp.warp_max = 128;   // warp tasks stage 4 entries per lane
-        sp.cta_max = 4096;   // CTA tasks and chunks stage 8 entries per thread
-        sp.chunk = 1024;     // split columns: chunks of ~1024 entries spread a long column over more CTAs
-        std::vector<int64_t> entries(J);
-        for (int j = 0; j < J; ++j) entries[j] = m->entries(j);
-        auto s = std::make_unique<DevSchedule>();
-        s->fixed = fixed;
-        s->kind = kind;
-        s->cluster = C;
-        s->host = build_schedule(K, J, m->col_start.data(), m->rows_h.data(), m->fmt.data(),
-                                 fixed.data(), nullptr, K, entries.data(), sp);
-        if (s->host.max_split_per_seg > indep_max_split() || s->host.max_split_per_level > indep_max_split())
-            throw Error(CCDB_ERR_UNSUPPORTED, "too many split columns on one level");
-        s->segs = upload(ctx, s->host.segs.data(), s->host.segs.size(), stream);
-        s->cta_seg = upload(ctx, s->host.cta_seg.data(), s->host.cta_seg.size(), stream);
-        s->tasks = upload(ctx, s->host.tasks.data(), s->host.tasks.size(), stream);
-        s->level_split = upload(ctx, s->host.level_split.data(), s->host.level_split.size(), stream);
-        check_cuda(ctx->wait(), "schedule upload");
-        sched = std::move(s);
-        return;
-    }
     int bps = 0;
     check_cuda(indep_sweep_occupancy(model, &bps), "occupancy");
     if (bps < 1) throw Error(CCDB_ERR_CUDA, "sweep kernel does not fit on an SM");
@@ -338,7 +295,6 @@ void Fit::ensure_schedule(int kind) {
     for (int j = 0; j < J; ++j) entries[j] = m->entries(j);
     auto s = std::make_unique<DevSchedule>();
     s->fixed = fixed;
-    s->kind = kind;
     s->host = build_schedule(K, J, m->col_start.data(), m->rows_h.data(), m->fmt.data(),
                              fixed.data(), nullptr, K, entries.data(), sp);
     if (s->host.max_split_per_seg > indep_max_split())
@@ -498,8 +454,8 @@ void Fit::find_mode_once(const ccdb_mode_args& a, double bound, int* flag, int* 
         find_mode_group_sweep(a, flag, iters, obj, ms);
         return;
     }
-    if (use_resident(a)) {
-        find_mode_resident(a, flag, iters, obj, ms);
+    if (!group_engine() && a.strategy != CCDB_SWEEP_SPECULATIVE && a.strategy != CCDB_SWEEP_GRID_LEVELS) {
+        find_mode_window(a, flag, iters, obj, ms);
         return;
     }
     if (group_engine() || use_speculative(a)) {
@@ -508,8 +464,7 @@ void Fit::find_mode_once(const ccdb_mode_args& a, double bound, int* flag, int* 
         *ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
         return;
     }
-    const int kind = sweep_kind(a);
-    ensure_schedule(kind);
+    ensure_schedule();
     if (sched->host.n_levels == 0) {
         // every coordinate is fixed: each cycle changes nothing, so the first
         // convergence check sees conv = 0 (findMode with an empty cycle)
@@ -523,11 +478,9 @@ void Fit::find_mode_once(const ccdb_mode_args& a, double bound, int* flag, int* 
     DevStatus zero{};
     zero.flag = R_FAIL;
     check_cuda(cudaMemcpyAsync(st, &zero, sizeof(zero), cudaMemcpyHostToDevice, stream), "status");
-    if (kind == kSchedGrid) {
-        check_cuda(cudaMemsetAsync(sched->level_done, 0, sizeof(unsigned) * std::max(1, sched->host.n_levels), stream), "reset");
-        check_cuda(cudaMemsetAsync(sched->col_arrive, 0, sizeof(unsigned) * std::max(1, J), stream), "reset");
-        check_cuda(cudaMemsetAsync(grid_bar, 0, sizeof(unsigned), stream), "reset");
-    }
+    check_cuda(cudaMemsetAsync(sched->level_done, 0, sizeof(unsigned) * std::max(1, sched->host.n_levels), stream), "reset");
+    check_cuda(cudaMemsetAsync(sched->col_arrive, 0, sizeof(unsigned) * std::max(1, J), stream), "reset");
+    check_cuda(cudaMemsetAsync(grid_bar, 0, sizeof(unsigned), stream), "reset");
     IndepParams P = params();
     P.conv = a.convergence_type;
     P.tol = a.tolerance;
@@ -537,21 +490,14 @@ void Fit::find_mode_once(const ccdb_mode_args& a, double bound, int* flag, int* 
     const char* trace_path = std::getenv("CCDB_TRACE_FILE");
     unsigned long long* d_trace = nullptr;
     const size_t n_seg = sched->host.segs.size();
-    if (trace_path && kind == kSchedCluster) {
-        // the cluster sweep: 4 timestamps per level and CTA of the first sweep
-        const size_t n = 4 * (size_t)sched->host.n_levels * sched->cluster;
-        d_trace = static_cast<unsigned long long*>(ctx->alloc(sizeof(unsigned long long) * n));
-        check_cuda(cudaMemsetAsync(d_trace, 0, sizeof(unsigned long long) * n, stream), "trace");
-        P.trace = d_trace;
-    } else if (trace_path) {
+    if (trace_path) {
         d_trace = static_cast<unsigned long long*>(ctx->alloc(sizeof(unsigned long long) * 5 * n_seg));
         check_cuda(cudaMemsetAsync(d_trace, 0, sizeof(unsigned long long) * 5 * n_seg, stream), "trace");
         P.trace = d_trace;
         P.trace2 = d_trace + 3 * n_seg;
     }
     check_cuda(cudaEventRecord(ctx->fev[0], stream), "event");
-    if (kind == kSchedCluster) check_cuda(launch_cluster_sweep(P, sched->cluster, stream), "sweep launch");
-    else check_cuda(launch_indep_sweep(P, sched->host.n_cta, stream), "sweep launch");
+    check_cuda(launch_indep_sweep(P, sched->host.n_cta, stream), "sweep launch");
     ++launches;
     check_cuda(cudaEventRecord(ctx->fev[1], stream), "event");
     // the host waits for the sweep before it queues the copy back: a device-to-host
@@ -562,23 +508,6 @@ void Fit::find_mode_once(const ccdb_mode_args& a, double bound, int* flag, int* 
     check_cuda(cudaMemcpyAsync(&out, st, sizeof(out), cudaMemcpyDeviceToHost, stream), "status");
     check_cuda(ctx->wait(), "sweep");
     check_cuda(cudaEventElapsedTime(ms, ctx->fev[0], ctx->fev[1]), "elapsed");
-    if (d_trace && kind == kSchedCluster) {
-        const size_t n = 4 * (size_t)sched->host.n_levels * sched->cluster;
-        std::vector<unsigned long long> tr(n);
-        check_cuda(cudaMemcpy(tr.data(), d_trace, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost),
-                   "trace copy");
-        ctx->release(d_trace);
-        d_trace = nullptr;
-        if (FILE* fh = std::fopen(trace_path, "wb")) {
-            // header: levels, CTAs; then the level of every column, the split flags, the stamps
-            const int64_t hdr[2] = {sched->host.n_levels, sched->cluster};
-            std::fwrite(hdr, sizeof(int64_t), 2, fh);
-            std::fwrite(sched->host.level_of.data(), sizeof(int32_t), sched->host.level_of.size(), fh);
-            std::fwrite(sched->host.level_split.data(), 1, sched->host.level_split.size(), fh);
-            std::fwrite(tr.data(), sizeof(unsigned long long), n, fh);
-            std::fclose(fh);
-        }
-    }
     if (d_trace) {
         std::vector<unsigned long long> tr(5 * n_seg);
         check_cuda(cudaMemcpy(tr.data(), d_trace, sizeof(unsigned long long) * 5 * n_seg,
@@ -601,8 +530,7 @@ void Fit::find_mode_once(const ccdb_mode_args& a, double bound, int* flag, int* 
     *flag = out.flag;
     *iters = out.iterations;
     *obj = out.objective;
-    if (kind == kSchedCluster) nz_steps += (int64_t)out.nonzero_steps;
-    else nz_known = false;  // the grid-wide sweep does not count them
+    nz_known = false;  // the grid-wide sweep does not count them
     beta_dirty_host = true;
 }
 
@@ -707,29 +635,70 @@ void Fit::apply_step(int j, double delta) {
 // independent-row models is the on-device cluster sweep.
 bool Fit::use_speculative(const ccdb_mode_args& a) const { return a.strategy == CCDB_SWEEP_SPECULATIVE; }
 
-// The resident sweep serves independent-row fits whose row state fits one
-// CTA's shared memory (chosen by CCDB_SWEEP_AUTO), and in its global form
-// (the row state in device memory) larger fits when asked for
-// (CCDB_SWEEP_RESIDENT).  AUTO leaves larger fits to the cluster sweep: on 43
-// L1 logistic fits of 14,000-96,000 rows the global form took 38 s in all
-// against the cluster sweep's 17.8 s (it won only on some fits of columns
-// below ~250 entries).
-bool Fit::use_resident(const ccdb_mode_args& a) {
-    if (group_engine()) return false;
-    if (a.strategy != CCDB_SWEEP_AUTO && a.strategy != CCDB_SWEEP_RESIDENT) return false;
-    if (ctx->resident_rows < 0) {
-        int64_t r = 0;
-        check_cuda(resident_max_rows(model, &r), "resident capacity");
-        ctx->resident_rows = r;
+// CTAs of the windowed sweep: as many as leave each warp about one entry per
+// lane, and enough of them for the rows.  More CTAs shorten a round's gather and
+// update until a column's share of entries fits one pass of a warp; after that
+// each doubling only adds messages to the exchange.  Milliseconds per L1 fit on
+// 1, 2, 4, 8, 16 CTAs (300 columns of m entries, K rows): K = 1,000, m = 20:
+// 0.149 0.166 0.156 0.159 0.178; K = 3,000, m = 60: 1.09 0.93 0.84 0.85 0.94;
+// K = 10,000, m = 200: 5.3 4.0 3.0 2.62 2.77; K = 30,000, m = 600: 20 12 11 7.8
+// 6.9; K = 100,000, m = 200: 6.6 3.7 2.3 1.51 1.35.
+int Fit::window_ctas() {
+    if (ctx->window_cluster < 0) {
+        int c = 0;
+        check_cuda(window_limits(&c, &ctx->window_smem), "cluster occupancy");
+        ctx->window_cluster = c;
     }
-    return K <= ctx->resident_rows || a.strategy == CCDB_SWEEP_RESIDENT;
+    if (ctx->window_cluster < 1) throw Error(CCDB_ERR_CUDA, "the sweep kernel does not fit on an SM");
+    int64_t total = 0, active = 0;
+    for (int j = 0; j < J; ++j)
+        if (!fixed[j]) {
+            total += m->entries(j);
+            ++active;
+        }
+    const int64_t mean = total / std::max<int64_t>(active, 1);
+    int c = 16;
+    if (K <= 1024 && mean <= 64) c = 1;
+    else if (K <= 4096 && mean <= 128) c = 4;
+    else if (K <= 32768 && mean <= 256) c = 8;
+    c = std::min(c, ctx->window_cluster);
+    while (ctx->max_ctas > 0 && c > ctx->max_ctas && c > 1) c /= 2;
+    return c;
 }
 
-void Fit::find_mode_resident(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms) {
-    std::vector<int32_t> cols;
-    for (int j = 0; j < J; ++j)
-        if (!fixed[j]) cols.push_back(j);
-    if (cols.empty()) {  // an empty cycle: the first check sees conv = 0
+void Fit::release_window() {
+    if (!window) return;
+    for (void* p : {(void*)window->cols, (void*)window->slices, (void*)window->scal,
+                    (void*)window->bh, (void*)window->share})
+        ctx->release(p);
+    window.reset();
+}
+
+void Fit::ensure_window(int ctas) {
+    if (window && window->ctas == ctas && window->fixed == fixed) return;
+    release_window();
+    const WindowPlan plan = build_window_plan(K, J, m->col_start.data(), m->rows_h.data(), m->val_start.data(),
+                                              m->fmt.data(), fixed.data(), ctas);
+    window.reset(new DevWindow());  // owned by the fit from here on, complete or not
+    window->ctas = 0;               // not a plan to reuse until it is complete
+    const size_t n = plan.cols.size();
+    window->cols = upload(ctx, plan.cols.data(), n, stream);
+    window->slices = upload(ctx, plan.slices.data(), plan.slices.size(), stream);
+    window->scal = static_cast<WinScal*>(ctx->alloc(sizeof(WinScal) * n));
+    window->bh = static_cast<double2*>(ctx->alloc(sizeof(double2) * n));
+    for (const WinCol& c : plan.cols) window->any_vals |= (c.flags & 2) != 0;
+    if (!window_share_fits((K + ctas - 1) / ctas, window->any_vals, ctx->window_smem))
+        window->share = static_cast<double*>(ctx->alloc(sizeof(double) * K));
+    check_cuda(ctx->wait(), "sweep plan upload");
+    window->n_active = (int32_t)n;
+    window->fixed = fixed;
+    window->ctas = ctas;
+}
+
+void Fit::find_mode_window(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms) {
+    if (std::find(fixed.begin(), fixed.end(), uint8_t(0)) == fixed.end()) {
+        // every coordinate is fixed: each cycle changes nothing, so the first
+        // convergence check sees conv = 0 (findMode with an empty cycle)
         *obj = objective(a.convergence_type);
         *flag = (*obj != *obj) ? R_ILLCONDITIONED
                 : (a.tolerance > 0 ? R_SUCCESS : (a.max_iterations == 1 ? R_MAX_ITERATIONS : R_SUCCESS));
@@ -737,70 +706,39 @@ void Fit::find_mode_resident(const ccdb_mode_args& a, int* flag, int* iters, dou
         *ms = 0.f;
         return;
     }
-    // the column records in visiting order
-    std::vector<ResCol> recs(cols.size());
-    for (size_t q = 0; q < cols.size(); ++q) {
-        const int j = cols[q];
-        const uint8_t f = m->fmt[j];
-        const bool has_rows = (f == F_SPARSE || f == F_INDICATOR);
-        ResCol& r = recs[q];
-        r.j = j;
-        r.flags = (has_rows ? 1 : 0) | ((f == F_SPARSE || f == F_DENSE) ? 2 : 0) |
-                  ((f == F_INDICATOR || f == F_INTERCEPT) ? 4 : 0);
-        r.n = has_rows ? m->col_start[j + 1] - m->col_start[j] : K;
-        r.cb = m->col_start[j];
-        r.vb = m->val_start[j];
-    }
-    if (d_res_cap < (int32_t)recs.size()) {
-        ctx->release(d_res_recs);
-        d_res_recs = static_cast<ResCol*>(ctx->alloc(sizeof(ResCol) * recs.size()));
-        d_res_cap = (int32_t)recs.size();
-    }
-    check_cuda(cudaMemcpyAsync(d_res_recs, recs.data(), sizeof(ResCol) * recs.size(), cudaMemcpyHostToDevice,
-                               stream), "column records");
+    ensure_window(window_ctas());
     DevStatus zero{};
     zero.flag = R_FAIL;
     check_cuda(cudaMemcpyAsync(st, &zero, sizeof(zero), cudaMemcpyHostToDevice, stream), "status");
-    ResidentParams R{};
+    WindowParams R{};
     R.P = params();
     R.P.conv = a.convergence_type;
     R.P.tol = a.tolerance;
     R.P.max_iter = a.max_iterations;
-    R.recs = d_res_recs;
-    R.n_active = (int32_t)recs.size();
+    R.cols = window->cols;
+    R.slices = window->slices;
+    R.scal = window->scal;
+    R.bh = window->bh;
+    R.share = window->share;
+    R.n_active = window->n_active;
     R.weighted = weighted ? 1 : 0;
-    if (K > ctx->resident_rows) {  // the global form: the row state in a device array
-        if (!d_res_rs) d_res_rs = static_cast<double2*>(ctx->alloc(sizeof(double2) * (size_t)K));
-        R.rs = d_res_rs;
-    }
-    // CCDB_TRACE_FILE=<path>: SM-clock stamps of the first batches (profiling aid; off by default)
-    const char* trace_path = std::getenv("CCDB_TRACE_FILE");
-    const int trace_n = 4096;
-    if (trace_path) {
-        R.trace = static_cast<long long*>(ctx->alloc(sizeof(long long) * kResidentTraceWords * trace_n));
-        check_cuda(cudaMemsetAsync(R.trace, 0, sizeof(long long) * kResidentTraceWords * trace_n, stream), "trace");
-        R.trace_n = trace_n;
-    }
+    R.any_vals = window->any_vals ? 1 : 0;
+    R.cluster = window->ctas;
     check_cuda(cudaEventRecord(ctx->fev[0], stream), "event");
-    check_cuda(launch_resident_sweep(R, stream), "resident sweep launch");
+    check_cuda(launch_window_sweep(R, ctx->window_smem, stream), "sweep launch");
     ++launches;
     check_cuda(cudaEventRecord(ctx->fev[1], stream), "event");
-    check_cuda(ctx->wait(), "resident sweep");  // the sweep is done before a copy is queued behind it
+    // the host waits for the sweep before it queues the copy back: a device-to-host
+    // copy queued behind a long kernel held up the copies of other contexts'
+    // streams, so fits served side by side finished together with the longest one
+    check_cuda(ctx->wait(), "sweep");
     DevStatus out{};
     check_cuda(cudaMemcpyAsync(&out, st, sizeof(out), cudaMemcpyDeviceToHost, stream), "status");
-    check_cuda(ctx->wait(), "resident sweep");
+    check_cuda(ctx->wait(), "sweep");
     check_cuda(cudaEventElapsedTime(ms, ctx->fev[0], ctx->fev[1]), "elapsed");
-    if (R.trace) {
-        std::vector<long long> tr((size_t)kResidentTraceWords * trace_n);
-        check_cuda(cudaMemcpyAsync(tr.data(), R.trace, sizeof(long long) * tr.size(), cudaMemcpyDeviceToHost, stream),
-                   "trace copy");
-        check_cuda(ctx->wait(), "trace copy");
-        ctx->release(R.trace);
-        if (FILE* fh = std::fopen(trace_path, "wb")) {
-            std::fwrite(tr.data(), sizeof(long long), tr.size(), fh);
-            std::fclose(fh);
-        }
-    }
+    if (out.error != E_NONE)
+        throw Error(CCDB_ERR_TIMEOUT, "device wait timed out (code " + std::to_string(out.error) +
+                                          " at " + std::to_string(out.error_where) + ")");
     *flag = out.flag;
     *iters = out.iterations;
     *obj = out.objective;

@@ -16,9 +16,9 @@
 #include "../../include/ccdb.h"
 #include "cox.h"
 #include "indep.h"
-#include "resident.h"
 #include "schedule.h"
 #include "step.h"
+#include "window_sweep.h"
 
 namespace ccdb {
 
@@ -35,8 +35,8 @@ struct Context {
     int device = 0;
     int n_sm = 0;
     int max_ctas = 0;  // persistent sweep grids: at most this many CTAs (0: n_sm)
-    int sweep_cluster = -1;  // largest resident cluster of the cluster sweep (-1: not queried)
-    int64_t resident_rows = -1;  // most rows of a shared-memory resident sweep (-1: not queried)
+    int window_cluster = -1;     // largest resident cluster of the windowed sweep (-1: not queried)
+    int64_t window_smem = 0;     // its shared memory per CTA
     int group_cluster = -1;      // largest resident cluster of the group sweep (-1: not queried)
     size_t budget = 0;
     size_t in_use = 0;
@@ -88,9 +88,6 @@ struct Matrix {
 
 struct DevSchedule {
     std::vector<uint8_t> fixed;
-    int kind = 0;     // kSchedGrid or kSchedCluster
-    int cluster = 0;  // CTAs of the cluster sweep
-    uint8_t* level_split = nullptr;
     Schedule host;
     Seg* segs = nullptr;
     int64_t* cta_seg = nullptr;
@@ -99,6 +96,19 @@ struct DevSchedule {
     unsigned* level_done = nullptr;
     unsigned* col_arrive = nullptr;
     double2* partials = nullptr;
+};
+
+// The plan of a windowed sweep on the device, and its per-position state.
+struct DevWindow {
+    std::vector<uint8_t> fixed;
+    int ctas = 0;
+    int32_t n_active = 0;
+    bool any_vals = false;
+    WinCol* cols = nullptr;
+    WinSlice* slices = nullptr;
+    WinScal* scal = nullptr;
+    double2* bh = nullptr;
+    double* share = nullptr;  // K, where a CTA's rows do not fit its shared memory
 };
 
 // Device tables of the Breslow Cox engine (cox.cu).
@@ -186,12 +196,9 @@ struct Fit {
     ~Fit();
     IndepParams params() const;
     void release_schedule();
-    // kSchedGrid: the grid-wide persistent sweep (one CTA per SM, levels ordered
-    // by global counters); kSchedCluster: one cluster, levels ordered by cluster
-    // barriers
-    static constexpr int kSchedGrid = 0, kSchedCluster = 1;
-    void ensure_schedule(int kind);
-    int sweep_kind(const ccdb_mode_args& a) const;
+    // the schedule of the grid-wide level sweep (one CTA per SM, levels ordered by
+    // global counters)
+    void ensure_schedule();
     void apply_weights();
     void compute_xbeta();
     void compute_xbeta_transpose();  // the MM cycle's product (ModelSpecifics::computeXBeta(beta))
@@ -213,12 +220,12 @@ struct Fit {
     void gh_batch(const int32_t* cols, int n, double2* out);
     void apply_step(int j, double delta);
     bool use_speculative(const ccdb_mode_args& a) const;
-    // the single-CTA sweep with the row state in shared memory (resident.cu)
-    bool use_resident(const ccdb_mode_args& a);
-    void find_mode_resident(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms);
-    ResCol* d_res_recs = nullptr;  // its active columns' records in visiting order
-    int32_t d_res_cap = 0;
-    double2* d_res_rs = nullptr;   // the row state of the global form (K entries)
+    // the windowed sweep (window.cu) on window_ctas() CTAs, and its plan
+    int window_ctas();
+    void ensure_window(int ctas);
+    void release_window();
+    void find_mode_window(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms);
+    std::unique_ptr<DevWindow> window;
     int32_t* d_batch_cols = nullptr;  // independent-row models
     double2* d_batch_out = nullptr;
     bool is_cox() const { return model == M_COX; }

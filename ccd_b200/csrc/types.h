@@ -14,7 +14,7 @@ enum Conv : int32_t { C_GRADIENT = 0, C_LANGE = 1, C_MITTAL = 2 };
 enum Flag : int32_t { R_SUCCESS = 0, R_FAIL = 1, R_MAX_ITERATIONS = 2, R_ILLCONDITIONED = 3 };
 
 // Device error codes written into DevStatus::error.
-enum DevErr : int32_t { E_NONE = 0, E_WAIT_LEVEL = 1, E_WAIT_COLUMN = 2, E_WAIT_GRID = 3 };
+enum DevErr : int32_t { E_NONE = 0, E_WAIT_LEVEL = 1, E_WAIT_COLUMN = 2, E_WAIT_GRID = 3, E_WAIT_CLUSTER = 4 };
 
 // Work unit of a sweep: one column (or one chunk of a long column).
 struct Task {

@@ -13,10 +13,8 @@ server only decides when it starts.
 Each slot's context limits its sweep kernels to its share of the SMs (a
 fast slot one CTA, a general slot an even share of the rest), so the slots'
 kernels can all be resident at once and run side by side.  Every model runs
-a whole findMode attempt in one launch: logistic and Poisson fits whose row
-state fits one CTA's shared memory the resident sweep (one CTA), larger ones
-the cluster sweep over dependency levels (a thread block cluster of at most
-that many CTAs), grouped models (conditional logistic, Cox) the persistent
+a whole findMode attempt in one launch: logistic and Poisson fits the windowed
+sweep (a thread block cluster of at most that many CTAs), grouped models (conditional logistic, Cox) the persistent
 group sweep (a cluster, or a cooperative grid, of at most that many CTAs).
 
 The reference has no serving layer; this loop drives the same C ABI entry
@@ -212,7 +210,7 @@ class Server:
 
         General slots share the SMs the fast slots leave (at most slot_ctas
         each when set); a fast slot's small fits run on fast_ctas CTAs (default
-        one: the resident sweep, or a one-CTA cluster or group sweep), which
+        one: a one-CTA windowed or group sweep), which
         find a free SM beside the general slots' clusters, where a multi-CTA
         cluster may have to wait for a whole GPC."""
         if slot >= self.n_slots:

@@ -6,7 +6,7 @@ neither changes what is computed beyond the order of the per-column sums:
 * the batched engine (ccdb_batch_find_mode, mixed precision): the lockstep
   group size G (instances stepped together by one CTA) and the CTAs per group
   C (a thread-block cluster that splits each column's rows);
-* the plain cluster sweep (ccdb_find_mode): the CTAs of its cluster, set
+* the plain sweep (ccdb_find_mode): the most CTAs of its cluster, set
   through ccdb_context_set_max_ctas (the largest power of two not above it).
 
 The engine's own choice when nothing is passed is a fixed rule (the longest

@@ -190,16 +190,12 @@ typedef struct {
     int32_t max_bound_count;   /* default 5 */
     int32_t per_coordinate;    /* 0: on-device mode finding (default); 1: host loop over
                                   the per-coordinate calls above (the reference's call pattern) */
-    int32_t strategy;          /* sweep strategy.  Logistic/Poisson: CCDB_SWEEP_AUTO runs
-                                  the resident sweep (one CTA, the row state in shared
-                                  memory) when the fit's rows fit it, else the cluster
-                                  sweep; _RESIDENT asks for the resident sweep (beyond
-                                  shared memory its global form, the row state in device
-                                  memory); _LEVELS runs the cluster sweep (one
-                                  launch per findMode over dependency levels),
-                                  _GRID_LEVELS the grid-wide level sweep,
-                                  _SPECULATIVE host-driven batches of gradients that restart
-                                  after each nonzero step.  Cox and conditional models: one
+    int32_t strategy;          /* sweep strategy.  Logistic/Poisson: CCDB_SWEEP_AUTO,
+                                  _LEVELS and _RESIDENT run the windowed sweep (one launch per
+                                  findMode on one thread-block cluster of 1 to 16 CTAs, sixteen
+                                  consecutive columns in flight), _GRID_LEVELS the grid-wide
+                                  level sweep, _SPECULATIVE host-driven batches of gradients
+                                  that restart after each nonzero step.  Cox and conditional models: one
                                   persistent launch per findMode of device-driven speculative
                                   batches -- one thread-block cluster with hardware barriers
                                   for fits a few SMs cover (forced by _LEVELS), else a
@@ -220,10 +216,10 @@ typedef struct {
 #define CCDB_ALGORITHM_MM 1
 
 #define CCDB_SWEEP_AUTO 0
-#define CCDB_SWEEP_LEVELS 1        /* one thread-block cluster, levels ordered by cluster barriers */
+#define CCDB_SWEEP_LEVELS 1        /* one thread-block cluster */
 #define CCDB_SWEEP_SPECULATIVE 2
 #define CCDB_SWEEP_GRID_LEVELS 3   /* one CTA per SM, levels ordered by global counters */
-#define CCDB_SWEEP_RESIDENT 4      /* one CTA, the row state in shared memory (or device memory) */
+#define CCDB_SWEEP_RESIDENT 4      /* logistic and Poisson fits: as CCDB_SWEEP_AUTO */
 
 typedef struct {
     int32_t return_flag;        /* UpdateReturnFlags */
@@ -342,8 +338,9 @@ int ccdb_matrix_validate(int64_t K, int32_t J, const int64_t* col_start, const i
  * per-column sums of the other CTAs of its cluster (default 2 s).  0 restores
  * the defaults.  A wait that runs out ends the call with CCDB_ERR_TIMEOUT and
  * leaves the context usable; the fit's state is then undefined until the next
- * ccdb_set_beta or ccdb_find_mode with starting values.  The cluster sweep
- * (CCDB_SWEEP_LEVELS) has no such wait.  No reference counterpart. */
+ * ccdb_set_beta or ccdb_find_mode with starting values.  The windowed sweep's
+ * wait for the other CTAs of its cluster has a bound of its own (10 s).  No
+ * reference counterpart. */
 int ccdb_fit_set_wait_limit(ccdb_fit* f, int64_t nanoseconds);
 
 /* Device time (CUDA events on the fit's stream) of the kernels of the fit's last
