@@ -48,6 +48,34 @@ CCDB_HD double newton_prior_delta(double g, double h, double beta, int ptype, do
     return newton_prior_delta_l(g, h, beta, ptype, var, ptype == 1 ? sqrt(2.0 / var) : 0.0);
 }
 
+// newton_prior_delta_l as one quotient num / den whose numerator is chosen before
+// the division: for a positive finite h the sign of each of the two Laplace
+// quotients is its numerator's, so only the one that is taken is divided, and a
+// zero step divides nothing.  inv_var = 1 / var and b_var = beta / var are read
+// for a normal prior only.
+CCDB_HD double newton_quotient_step(double g, double h, double beta, int ptype, double var, double lambda,
+                                    double inv_var, double b_var) {
+    double num, den;
+    if (ptype == 1) {
+        if (!(h > 0.0 && h <= 1.7976931348623157e308)) return newton_prior_delta_l(g, h, beta, 1, var, lambda);
+        if (beta == 0.0 && !(fabs(g) > lambda)) return 0.0;
+        num = (beta > 0.0 || (beta == 0.0 && g < 0.0)) ? g + lambda : g - lambda;
+        den = h;
+    } else {
+        if (h < 0.0) g = h = 0.0;
+        num = g;
+        den = h;
+        if (ptype == 2) {
+            num += b_var;
+            den += inv_var;
+        }
+    }
+    double delta = -num / den;
+    // not across zero
+    if (ptype == 1 && beta != 0.0 && (beta > 0.0 ? beta + delta <= 0.0 : !(beta + delta < 0.0))) delta = -beta;
+    return delta;
+}
+
 // applyBounds (CyclicCoordinateDescent.cpp:1503-1520), std::max semantics.
 CCDB_HD double apply_bounds(double delta, double& hd) {
     if (delta < -hd) delta = -hd;

@@ -123,32 +123,6 @@ __device__ __forceinline__ void add_terms(bool ind, bool weighted, double x, dou
     }
 }
 
-// The Laplace step where h > 0 does not hold (an overflowing or empty Hessian).
-__device__ __noinline__ double laplace_step(double g, double h, double b, double var, double lambda) {
-    return newton_prior_delta_l(g, h, b, 1, var, lambda);
-}
-
-// newton_prior_delta_l as one quotient num / den, found without a division:
-// b_var = b / var and inv_var = 1 / var of a normal prior are known before the
-// sums are, and for h > 0 the sign of each of the two Laplace quotients is its
-// numerator's.  A zero step takes no division at all.
-__device__ __forceinline__ double newton_step(double g, double h, double b, const WinScal& s, double b_var) {
-    double num, den;
-    if (s.ptype == 1) {
-        if (!(h > 0.0)) return laplace_step(g, h, b, s.pvar, s.lambda);
-        num = (b > 0.0 || (b == 0.0 && g < 0.0)) ? g + s.lambda : g - s.lambda;
-        if (b == 0.0 && fabs(g) <= s.lambda) return 0.0;
-        den = h;
-    } else {
-        if (h < 0.0) g = h = 0.0;
-        num = g + b_var;
-        den = h + s.inv_var;
-    }
-    double d = -num / den;
-    if (s.ptype == 1 && b != 0.0 && (b > 0.0 ? b + d <= 0.0 : !(b + d < 0.0))) d = -b;  // not across zero
-    return d;
-}
-
 // Sums of g over the warp in lanes 0..15 and of h in lanes 16..31.
 __device__ __forceinline__ double warp_pair_sum(double g, double h) {
     const bool upper = threadIdx.x & 16;
@@ -368,7 +342,6 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
         return (P.conv == C_GRADIENT) ? acc.z : (P.conv == C_MITTAL ? ll : ll + lp);
     };
 
-    // ---- a warp's columns: position, records two ahead, entries one ahead
     // ---- what the helpers copy ahead: records two columns ahead of a warp, entries one
     auto rec_of = [&](int at) -> Rec& { return s_rec[(at / kWindow) & 3][at & (kWindow - 1)]; };
     // lane l8 of the eight that copy a record
@@ -562,7 +535,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                     }
                     if (r.c.n > 0) t.x -= r.s.xjy;
                     else t = make_double2(0.0, 0.0);  // an empty column gives (0, 0) (ModelSpecifics.hpp:720-723)
-                    d = newton_step(t.x, t.y, b0, r.s, b_var);
+                    d = newton_quotient_step(t.x, t.y, b0, r.s.ptype, r.s.pvar, r.s.lambda, r.s.inv_var, b_var);
                     d = (d < -hd) ? -hd : (d > hd ? hd : d);  // apply_bounds; its new bound is not needed yet
                     if (lane == 0) s_moves[wid] = d != 0.0 ? 1 : 0;
                 }

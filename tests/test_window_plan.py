@@ -21,3 +21,16 @@ def test_window_plan_matches_pairwise_comparison(tmp_path):
     r = subprocess.run([exe, "300"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, (r.stdout[-2000:], r.stderr[-4000:])
     assert "identical" in r.stdout
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="no host compiler")
+def test_quotient_step_matches_the_closed_forms(tmp_path):
+    """The windowed sweep's step against newton_prior_delta_l, infinities and
+    not-a-numbers included."""
+    exe = str(tmp_path / "step_check")
+    r = subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I" + os.path.join(ROOT, "ccd_b200", "csrc"),
+                        os.path.join(ROOT, "tests", "native", "step_check.cpp"), "-o", exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-4000:]
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout[-2000:]
+    assert "identical" in r.stdout
