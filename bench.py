@@ -584,7 +584,7 @@ def run_ours(args, world, rank, local, collect=False):
                           "unit": "GB/s", "frac": cox_bytes(d, sweeps, nonzero) / ker_t / 1e9 / peak,
                           "peak_source": peak_kind,
                           "algorithmic_bytes_per_launch": cox_bytes(d, sweeps, nonzero) / attempts,
-                          "kernel": "group_sweep_kernel<COX> (one launch per findMode attempt)",
+                          "kernel": "group_window_kernel<COX> (one launch per findMode attempt)",
                           "bytes": "this engine's O(nnz) gradients plus the O(groups) rebuild per nonzero step "
                                    "(cox_bytes)", "traffic": None}),
             "gpu_launches": int(tot_launch),

@@ -451,7 +451,7 @@ void Fit::find_mode_once(const ccdb_mode_args& a, double bound, int* flag, int* 
         return;
     }
     if (group_engine() && a.strategy != CCDB_SWEEP_SPECULATIVE) {
-        find_mode_group_sweep(a, flag, iters, obj, ms);
+        find_mode_group_window(a, flag, iters, obj, ms);
         return;
     }
     if (!group_engine() && a.strategy != CCDB_SWEEP_SPECULATIVE && a.strategy != CCDB_SWEEP_GRID_LEVELS) {
@@ -669,7 +669,8 @@ int Fit::window_ctas() {
 void Fit::release_window() {
     if (!window) return;
     for (void* p : {(void*)window->cols, (void*)window->slices, (void*)window->scal,
-                    (void*)window->bh, (void*)window->share})
+                    (void*)window->bh, (void*)window->share, (void*)window->cuts, (void*)window->part,
+                    (void*)window->tails, (void*)window->heads})
         ctx->release(p);
     window.reset();
 }

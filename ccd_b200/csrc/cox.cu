@@ -425,7 +425,29 @@ __global__ void __launch_bounds__(kT) grouped_objective_kernel(CoxParams P, doub
     }
 }
 
+// The sums and values of the blocks that the windowed sweep works on.
+__global__ void cox_blocks_kernel(CoxParams P, const int32_t* bgrp, int64_t NB, double* bden, double* bD, double* bS1,
+                                  double* bS2) {
+    for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < NB; b += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t g0 = bgrp[b], g1 = bgrp[b + 1];
+        double v = 0.0;
+        for (int32_t g = g0; g < g1; ++g) v += P.denom[g];
+        bden[b] = v;
+        bD[b] = P.D[g1 - 1];
+        bS1[b] = P.S1[g1 - 1];
+        bS2[b] = P.S2[g1 - 1];
+    }
+}
+
 }  // namespace
+
+cudaError_t launch_cox_blocks(const CoxParams& P, const int32_t* bgrp, int64_t NB, double* bden, double* bD,
+                              double* bS1, double* bS2, cudaStream_t s) {
+    if (NB <= 0) return cudaSuccess;
+    const unsigned nb = (unsigned)((NB + 255) / 256 < 2368 ? (NB + 255) / 256 : 2368);
+    cox_blocks_kernel<<<nb, 256, 0, s>>>(P, bgrp, NB, bden, bD, bS1, bS2);
+    return cudaGetLastError();
+}
 
 // ---------------------------------------------------------------- launchers
 int cox_scan_tiles(int64_t N) { return (int)((N + kTile - 1) / kTile); }

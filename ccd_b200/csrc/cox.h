@@ -50,6 +50,10 @@ cudaError_t launch_cox_remaining(const CoxParams& P, cudaStream_t s);
 // must differ from every earlier call on the same status arrays.
 cudaError_t launch_cox_scans(const CoxParams& P, unsigned* tickets, int* status, void* tails,
                              int epoch, cudaStream_t s);
+// bden[b] = the sum of denom over block b's groups [bgrp[b], bgrp[b + 1]), and D, S1,
+// S2 of its last group (S1 and S2 are the same for all of them).
+cudaError_t launch_cox_blocks(const CoxParams& P, const int32_t* bgrp, int64_t NB, double* bden, double* bD,
+                              double* bS1, double* bS2, cudaStream_t s);
 cudaError_t launch_cox_objective(const CoxParams& P, double2* red, int nblocks, cudaStream_t s);
 
 // Grouped models (conditional logistic / Poisson): grp = stratum, N = strata,

@@ -5,11 +5,12 @@
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "cox.h"
 #include "engine.h"
-#include "group_sweep.h"
+#include "group_window.h"
 
 namespace ccdb {
 
@@ -141,8 +142,9 @@ void Fit::cox_release() {
     for (void* p : {(void*)cox.xbe, (void*)cox.grp, (void*)cox.rstrat, (void*)cox.denom, (void*)cox.D,
                     (void*)cox.S1, (void*)cox.S2, (void*)cox.nEv, (void*)cox.gfirst, (void*)cox.glast,
                     (void*)cox.grow, (void*)cox.tickets, (void*)cox.status, cox.tails,
-                    (void*)cox.batch_cols, (void*)cox.batch_out, (void*)cox.sweep_cols, (void*)cox.dd,
-                    (void*)cox.ddg, cox.agg, (void*)cox.counters, (void*)cox.sweep_gh})
+                    (void*)cox.batch_cols, (void*)cox.batch_out, (void*)cox.counters,
+                    (void*)cox.blk, (void*)cox.bgrp, (void*)cox.bden, (void*)cox.bD, (void*)cox.bS1, (void*)cox.bS2,
+                    (void*)cox.bnev, (void*)cox.bfirst, (void*)cox.blast, (void*)cox.brow})
         ctx->release(p);
 }
 
@@ -197,6 +199,53 @@ void Fit::cox_apply_weights() {
         gl[g] = (g == N - 1 || gstrat[g] != gstrat[g + 1]) ? 1 : 0;
     }
     grow[N] = K;
+    // Blocks: runs of groups up to one with events, or to their stratum's end.  D
+    // counts only where there are events, and S1 and S2 change only there, so the
+    // sweep keeps one denominator, one D and one pair of suffix sums per block.
+    std::vector<int32_t> bgrp, group_block(N);
+    std::vector<int32_t> bstrat;
+    for (int64_t g = 0; g < N; ++g) {
+        if (g == 0 || gf[g] || nev[g - 1] != 0.0) {
+            bgrp.push_back((int32_t)g);
+            bstrat.push_back(gstrat[g]);
+        }
+        group_block[g] = (int32_t)bgrp.size() - 1;
+    }
+    const int64_t NB = (int64_t)bgrp.size();
+    bgrp.push_back((int32_t)N);
+    std::vector<int32_t> blk(K);
+    for (int64_t k = 0; k < K; ++k) blk[k] = grp[k] < N ? group_block[grp[k]] : (int32_t)NB;
+    std::vector<double> bnev(NB + 1, 0.0);
+    std::vector<uint8_t> bf(NB + 1, 0), bl(NB + 1, 0);
+    std::vector<int64_t> brow(NB + 1, K);
+    for (int64_t b = 0; b < NB; ++b) {
+        bnev[b] = nev[bgrp[b + 1] - 1];
+        bf[b] = gf[bgrp[b]];
+        bl[b] = gl[bgrp[b + 1] - 1];
+        brow[b] = grow[bgrp[b]];
+    }
+    for (void* p : {(void*)cox.blk, (void*)cox.bgrp, (void*)cox.bden, (void*)cox.bD, (void*)cox.bS1, (void*)cox.bS2,
+                    (void*)cox.bnev, (void*)cox.bfirst, (void*)cox.blast, (void*)cox.brow})
+        ctx->release(p);
+    cox.blk = nullptr;
+    cox.bgrp = nullptr;
+    cox.bden = cox.bD = cox.bS1 = cox.bS2 = cox.bnev = nullptr;
+    cox.bfirst = cox.blast = nullptr;
+    cox.brow = nullptr;
+    auto put = [&](auto*& d, const auto& h) {
+        d = static_cast<std::remove_reference_t<decltype(d)>>(ctx->alloc(sizeof(h[0]) * h.size()));
+        check_cuda(cudaMemcpyAsync(d, h.data(), sizeof(h[0]) * h.size(), cudaMemcpyHostToDevice, stream), "blocks");
+    };
+    put(cox.blk, blk);
+    put(cox.bgrp, bgrp);
+    put(cox.bnev, bnev);
+    put(cox.bfirst, bf);
+    put(cox.blast, bl);
+    put(cox.brow, brow);
+    for (double** p : {&cox.bden, &cox.bD, &cox.bS1, &cox.bS2})
+        *p = static_cast<double*>(ctx->alloc(sizeof(double) * (NB + 1)));
+    cox.NB = NB;
+    ++cox.grouping;
     check_cuda(cudaMemcpyAsync(w, wh.data(), sizeof(double) * K, cudaMemcpyHostToDevice, stream), "w");
     check_cuda(cudaMemcpyAsync(cox.grp, grp.data(), sizeof(int32_t) * K, cudaMemcpyHostToDevice, stream), "grp");
     check_cuda(cudaMemcpyAsync(cox.nEv, nev.data(), sizeof(double) * (N + 1), cudaMemcpyHostToDevice, stream), "nev");
@@ -216,6 +265,8 @@ void Fit::cox_apply_weights() {
     ++launches;
     ll_fixed = 0.0;
     check_cuda(ctx->wait(), "cox weights");
+    cox_grow_h = std::move(brow);
+    cox_bstrat_h = std::move(bstrat);
     valid_weights = true;
     suff_known = false;
 }
@@ -285,19 +336,115 @@ void Fit::cox_update(int j, double delta) {
     cox_scans();
 }
 
-// findMode (CyclicCoordinateDescent.cpp:909-1216) of the Cox and grouped
-// models as one cooperative launch: speculative gradient batches, the nonzero
-// steps, the denominator updates, the Cox scans and the convergence test all on
-// the device (group_sweep.cu).  The bounds are set by the caller.
-void Fit::find_mode_group_sweep(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms) {
-    std::vector<int32_t> cols;
-    int64_t max_entries = 1;
-    for (int j = 0; j < J; ++j)
-        if (!fixed[j]) {
-            cols.push_back(j);
-            max_entries = std::max<int64_t>(max_entries, m->entries(j));
+// The plan of the group models' windowed sweep on `ctas` CTAs: whole groups, in
+// equal numbers, and what each CTA's strata share with its neighbours'.
+void Fit::ensure_group_window(int ctas, bool cluster) {
+    if (window && window->ctas == ctas && window->cluster == cluster && window->grouping == cox.grouping &&
+        window->fixed == fixed)
+        return;
+    release_window();
+    window.reset(new DevWindow());  // owned by the fit from here on, complete or not
+    std::vector<WinCol> cols;
+    for (int j = 0; j < J; ++j) {
+        if (fixed[j]) continue;
+        const uint8_t f = m->fmt[j];
+        WinCol c{};
+        c.cb = m->col_start[j];
+        c.vb = m->val_start[j];
+        c.j = j;
+        c.n = (int32_t)m->entries(j);
+        c.flags = ((f == F_SPARSE || f == F_INDICATOR) ? 1 : 0) | ((f == F_SPARSE || f == F_DENSE) ? 2 : 0) |
+                  ((f == F_INDICATOR || f == F_INTERCEPT) ? 4 : 0);
+        window->any_vals |= (c.flags & 2) != 0;
+        cols.push_back(c);
+    }
+    // Where a CTA's groups begin.  Cox: at the nearest start of a stratum, when no CTA
+    // then owns a quarter more than its even share, so that no stratum spans CTAs and
+    // a step needs no tail and head sums; else in even shares.
+    std::vector<GroupCut> cuts(ctas + 1);
+    const int64_t N = is_cox() ? cox.NB : cox.N;
+    std::vector<int64_t> first_group(ctas + 1);
+    for (int r = 0; r <= ctas; ++r) first_group[r] = N * r / ctas;
+    if (is_cox() && ctas > 1) {
+        std::vector<int64_t> starts, aligned(first_group);
+        for (int64_t g = 0; g < N; ++g)
+            if (g == 0 || cox_bstrat_h[g] != cox_bstrat_h[g - 1]) starts.push_back(g);
+        starts.push_back(N);
+        int64_t most = 0;
+        for (int r = 1; r < ctas; ++r) {
+            const auto above = std::lower_bound(starts.begin(), starts.end(), first_group[r]);
+            const auto below = above == starts.begin() ? above : above - 1;
+            aligned[r] = *above - first_group[r] < first_group[r] - *below ? *above : *below;
         }
-    if (cols.empty()) {  // an empty cycle: the first check sees conv = 0
+        bool each = true;
+        for (int r = 0; r < ctas; ++r) {
+            most = std::max(most, aligned[r + 1] - aligned[r]);
+            each &= aligned[r + 1] > aligned[r];
+        }
+        if (each && most * ctas * 4 <= N * 5) first_group = aligned;
+    }
+    for (int r = 0; r <= ctas; ++r) {
+        GroupCut& c = cuts[r];
+        const int64_t g0 = first_group[r], g1 = r < ctas ? first_group[r + 1] : N;
+        c.g0 = (int32_t)g0;
+        c.row0 = (int32_t)(r == 0 ? 0 : r == ctas ? K : cox_grow_h[g0]);
+        c.lo = c.hi = r;
+        if (is_cox() && r < ctas && g1 > g0) {
+            c.first = cox_bstrat_h[g0];
+            c.last = cox_bstrat_h[g1 - 1];
+            c.flags = ((g0 > 0 && cox_bstrat_h[g0 - 1] == c.first) ? 1 : 0) | (c.first == c.last ? 2 : 0);
+        } else {
+            c.first = c.last = -1;
+        }
+    }
+    int32_t row = 1;
+    for (int r = 0; r < ctas; ++r) {
+        GroupCut& c = cuts[r];
+        window->most_rows = std::max<int64_t>(window->most_rows, cuts[r + 1].row0 - c.row0);
+        window->most_groups = std::max<int64_t>(window->most_groups, cuts[r + 1].g0 - c.g0);
+        window->meet |= (c.flags & 1) != 0;
+        window->chain = std::max(window->chain, r > 0 && c.flags == 3 ? ++row : (row = 1));
+        if (c.flags & 1) {
+            c.lo = r - 1;
+            while (c.lo > 0 && cuts[c.lo].flags == 3) --c.lo;
+        }
+        if (r + 1 < ctas && (cuts[r + 1].flags & 1)) {
+            c.hi = r + 1;
+            while (c.hi + 1 < ctas && (cuts[c.hi].flags & 2) && (cuts[c.hi + 1].flags & 1)) ++c.hi;
+        }
+    }
+    const size_t n = cols.size();
+    auto upload = [&](const void* h, size_t bytes) {
+        void* d = ctx->alloc(bytes);
+        check_cuda(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, stream), "sweep plan upload");
+        return d;
+    };
+    window->cols = static_cast<WinCol*>(upload(cols.data(), sizeof(WinCol) * n));
+    window->cuts = static_cast<GroupCut*>(upload(cuts.data(), sizeof(GroupCut) * cuts.size()));
+    window->slices = static_cast<WinSlice*>(ctx->alloc(sizeof(WinSlice) * n * ctas));
+    window->scal = static_cast<WinScal*>(ctx->alloc(sizeof(WinScal) * n));
+    window->bh = static_cast<double2*>(ctx->alloc(sizeof(double2) * n));
+    if (!cluster) {
+        window->part = static_cast<double2*>(ctx->alloc(sizeof(double2) * 2 * kWindow * ctas * 3));
+        window->tails = static_cast<double*>(ctx->alloc(sizeof(double) * 2 * ctas));
+        window->heads = static_cast<double2*>(ctx->alloc(sizeof(double2) * 2 * ctas));
+    }
+    check_cuda(launch_window_slices(m->d_rows, window->cols, (int32_t)n, window->cuts, ctas, window->slices, stream),
+               "sweep plan");
+    ++launches;
+    check_cuda(ctx->wait(), "sweep plan");
+    window->n_active = (int32_t)n;
+    window->fixed = fixed;
+    window->grouping = cox.grouping;
+    window->cluster = cluster;
+    window->ctas = ctas;
+}
+
+// findMode (CyclicCoordinateDescent.cpp:909-1216) of the Cox and grouped models
+// in one launch (group_window.cu).  The bounds are set by the caller.
+void Fit::find_mode_group_window(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms) {
+    if (std::find(fixed.begin(), fixed.end(), uint8_t(0)) == fixed.end()) {
+        // an empty cycle: the first check sees conv = 0
         *obj = objective(a.convergence_type);
         *flag = (*obj != *obj) ? R_ILLCONDITIONED
                 : (a.tolerance > 0 ? R_SUCCESS : (a.max_iterations == 1 ? R_MAX_ITERATIONS : R_SUCCESS));
@@ -305,89 +452,98 @@ void Fit::find_mode_group_sweep(const ccdb_mode_args& a, int* flag, int* iters, 
         *ms = 0.f;
         return;
     }
-    int bps = 0;
-    check_cuda(group_sweep_occupancy(&bps), "occupancy");
-    if (bps < 1) throw Error(CCDB_ERR_CUDA, "the group sweep kernel does not fit on an SM");
+    GroupWindowLimits& lim = ctx->group_window;
+    if (lim.cluster < 0) check_cuda(group_window_limits(&lim), "cluster occupancy");
+    bool any_vals = false;
+    for (int j = 0; j < J; ++j) any_vals |= !fixed[j] && (m->fmt[j] == F_SPARSE || m->fmt[j] == F_DENSE);
+    // The cluster form, on the largest cluster of the context's share, when the groups
+    // fit its CTAs' shared memory and a CTA's slice of a column is not over about 128
+    // entries; else the grid form, on 64 CTAs or as many as the groups need: more of
+    // them lengthen every exchange.  CCDB_SWEEP_GRID_LEVELS asks for the grid form,
+    // CCDB_SWEEP_LEVELS for the cluster form.  Milliseconds per fit on a cluster of 4,
+    // 8, 16 and a grid of 32, 64, 148: conditional logistic, 4,000 sets, 512 entries a
+    // column: 4.60 3.27 2.82 3.13 3.41 4.74; 20,000 sets, 2,601 entries: 26.8 14.3 4.78
+    // 4.22 3.84 4.14; Cox, 20,000 rows, 199 entries: 2.75 2.94 2.52 4.47 4.73 6.35;
+    // 200,000 rows, 2,001 entries: 17.7 11.0 7.62 6.68 6.55 7.84.
+    const int64_t N = is_cox() ? cox.NB : cox.N;
+    int64_t total = 0, active = 0;
+    for (int j = 0; j < J; ++j)
+        if (!fixed[j]) {
+            total += m->entries(j);
+            ++active;
+        }
     int n_cta = ctx->n_sm;
     if (ctx->max_ctas > 0) n_cta = std::min(n_cta, ctx->max_ctas);
-    // the cluster form (hardware barriers) when the fit is small enough for a few
-    // SMs or the context's share is a cluster's worth; CCDB_SWEEP_GRID_LEVELS asks
-    // for the grid form, CCDB_SWEEP_LEVELS for the cluster form
-    if (ctx->group_cluster < 0) {
-        int c = 0;
-        check_cuda(group_sweep_max_cluster(&c), "cluster occupancy");
-        ctx->group_cluster = c;
+    int c = lim.cluster;
+    while (c > 1 && (c > n_cta || c > N)) c /= 2;
+    const int64_t smem_grid = lim.smem[0], smem_cluster = lim.smem[is_cox() ? 2 : 1];
+    const bool use_cluster = c >= 1 && a.strategy != CCDB_SWEEP_GRID_LEVELS &&
+                             (a.strategy == CCDB_SWEEP_LEVELS || n_cta <= lim.cluster + lim.cluster / 4 ||
+                              (group_window_fits(is_cox(), N, c, any_vals, smem_cluster) && total / active <= 128 * c));
+    if (use_cluster) {
+        n_cta = c;
+    } else {
+        const int most = (int)std::max<int64_t>(1, std::min<int64_t>({n_cta, N, kGroupWindowCtas}));
+        n_cta = std::min(64, most);
+        while (n_cta < most && !group_window_fits(is_cox(), N, n_cta, any_vals, smem_grid)) ++n_cta;
     }
-    bool use_cluster = false;
-    if (ctx->group_cluster >= 2 && a.strategy != CCDB_SWEEP_GRID_LEVELS) {
-        const int64_t work = cox.N + max_entries;
-        use_cluster = a.strategy == CCDB_SWEEP_LEVELS || n_cta <= ctx->group_cluster + ctx->group_cluster / 4 ||
-                      work <= (int64_t)ctx->group_cluster * kGroupClusterWork;
-        if (use_cluster) {
-            int c = ctx->group_cluster;
-            while (c > 1 && c > n_cta) c /= 2;
-            n_cta = c;
-        }
-    }
-    if (!cox.sweep_cols) {
-        cox.sweep_cols = static_cast<int32_t*>(ctx->alloc(sizeof(int32_t) * std::max(1, J)));
-        cox.agg = ctx->alloc(sizeof(SegAgg) * 2 * ctx->n_sm);
-        cox.counters = static_cast<int64_t*>(ctx->alloc(sizeof(int64_t) * 2));
-    }
-    if (cox.dd_cap < max_entries) {
-        ctx->release(cox.dd);
-        ctx->release(cox.ddg);
-        cox.dd = static_cast<double*>(ctx->alloc(sizeof(double) * max_entries));
-        cox.ddg = static_cast<int32_t*>(ctx->alloc(sizeof(int32_t) * max_entries));
-        cox.dd_cap = max_entries;
-    }
-    check_cuda(cudaMemcpyAsync(cox.sweep_cols, cols.data(), sizeof(int32_t) * cols.size(), cudaMemcpyHostToDevice,
-                               stream), "columns");
-    if (!cox.sweep_gh) cox.sweep_gh = static_cast<double2*>(ctx->alloc(sizeof(double2) * 2 * kGroupBatchMax));
+    ensure_group_window(n_cta, use_cluster);
+    if (!cox.counters) cox.counters = static_cast<int64_t*>(ctx->alloc(sizeof(int64_t) * 2));
     if (!beta_dirty_host) upload_beta();
     DevStatus zero{};
     zero.flag = R_FAIL;
     check_cuda(cudaMemcpyAsync(st, &zero, sizeof(zero), cudaMemcpyHostToDevice, stream), "status");
     check_cuda(cudaMemsetAsync(grid_bar, 0, sizeof(unsigned), stream), "barrier");
     check_cuda(cudaMemsetAsync(cox.counters, 0, sizeof(int64_t) * 2, stream), "counters");
-    GroupSweepParams Q{};
+    GroupWindowParams Q{};
     Q.P = cox_params();
     Q.cox = is_cox() ? 1 : 0;
-    Q.n_active = (int32_t)cols.size();
-    Q.cols = cox.sweep_cols;
+    if (is_cox()) {
+        check_cuda(launch_cox_blocks(Q.P, cox.bgrp, cox.NB, cox.bden, cox.bD, cox.bS1, cox.bS2, stream), "blocks");
+        ++launches;
+        Q.P.N = cox.NB;
+        Q.P.grp = cox.blk;
+        Q.P.denom = cox.bden;
+        Q.P.D = cox.bD;
+        Q.P.S1 = cox.bS1;
+        Q.P.S2 = cox.bS2;
+        Q.P.nEv = cox.bnev;
+        Q.P.gfirst = cox.bfirst;
+        Q.P.glast = cox.blast;
+        Q.P.grow = cox.brow;
+    }
+    Q.n_active = window->n_active;
+    Q.cols = window->cols;
+    Q.slices = window->slices;
+    Q.scal = window->scal;
+    Q.bh = window->bh;
+    Q.cuts = window->cuts;
     Q.beta = beta;
     Q.hdelta = hdelta;
     Q.ptype = ptype;
     Q.pvar = pvar;
+    Q.J = J;
     Q.conv = a.convergence_type;
     Q.max_iter = a.max_iterations;
     Q.tol = a.tolerance;
+    Q.ctas = window->ctas;
     Q.ll_fixed = ll_fixed;
-    Q.batch_max = std::min(kBatchMax, kGroupBatchMax);
-    Q.J = J;
-    Q.gh = cox.sweep_gh;
-    Q.dd = cox.dd;
-    Q.ddg = cox.ddg;
-    Q.red = red;
-    Q.agg = static_cast<SegAgg*>(cox.agg);
-    Q.grid_bar = grid_bar;
+    Q.any_vals = window->any_vals ? 1 : 0;
+    Q.meet = window->meet ? 1 : 0;
+    Q.chain = window->chain;
     Q.st = st;
+    Q.part = window->part;
+    Q.tails = window->tails;
+    Q.heads = window->heads;
+    Q.red = red;
+    Q.grid_bar = grid_bar;
     Q.wait_limit_ns = wait_limit_ns;
     Q.counters = cox.counters;
-    // CCDB_TRACE_FILE=<path>: timestamps of the first 4,096 nonzero steps (profiling aid; off by default)
-    const char* trace_path = std::getenv("CCDB_TRACE_FILE");
-    unsigned long long* d_trace = nullptr;
-    const int trace_steps = 4096;
-    if (trace_path) {
-        d_trace = static_cast<unsigned long long*>(ctx->alloc(sizeof(unsigned long long) * kTraceStamps * trace_steps));
-        check_cuda(cudaMemsetAsync(d_trace, 0, sizeof(unsigned long long) * kTraceStamps * trace_steps, stream), "trace");
-        Q.trace = d_trace;
-        Q.trace_steps = trace_steps;
-    }
     check_cuda(cudaEventRecord(ctx->fev[0], stream), "event");
-    check_cuda(launch_group_sweep(Q, n_cta, use_cluster, stream), "group sweep launch");
+    check_cuda(launch_group_window(Q, use_cluster, window->most_rows, window->most_groups, stream), "group sweep launch");
     ++launches;
     check_cuda(cudaEventRecord(ctx->fev[1], stream), "event");
+    if (is_cox()) cox_remaining();  // the groups' own denominators and sums, for the calls that follow
     check_cuda(ctx->wait(), "group sweep");  // the sweep is done before a copy is queued behind it
     DevStatus out{};
     int64_t cnt[2] = {0, 0};
@@ -395,21 +551,9 @@ void Fit::find_mode_group_sweep(const ccdb_mode_args& a, int* flag, int* iters, 
     check_cuda(cudaMemcpyAsync(cnt, cox.counters, sizeof(cnt), cudaMemcpyDeviceToHost, stream), "counters");
     check_cuda(ctx->wait(), "group sweep");
     check_cuda(cudaEventElapsedTime(ms, ctx->fev[0], ctx->fev[1]), "elapsed");
-    if (d_trace) {
-        std::vector<unsigned long long> tr(kTraceStamps * (size_t)trace_steps);
-        check_cuda(cudaMemcpy(tr.data(), d_trace, sizeof(unsigned long long) * tr.size(), cudaMemcpyDeviceToHost),
-                   "trace copy");
-        ctx->release(d_trace);
-        if (FILE* fh = std::fopen(trace_path, "wb")) {
-            std::fwrite(tr.data(), sizeof(unsigned long long), tr.size(), fh);
-            std::fclose(fh);
-        }
-    }
     if (out.error != E_NONE)
         throw Error(CCDB_ERR_TIMEOUT, "device wait timed out (code " + std::to_string(out.error) + " at " +
                                           std::to_string(out.error_where) + ")");
-    cox.last_updates = cnt[0];
-    cox.last_batches = cnt[1];
     nz_steps += cnt[0];
     *flag = out.flag;
     *iters = out.iterations;

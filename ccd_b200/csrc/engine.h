@@ -15,6 +15,7 @@
 
 #include "../../include/ccdb.h"
 #include "cox.h"
+#include "group_window.h"
 #include "indep.h"
 #include "schedule.h"
 #include "step.h"
@@ -37,7 +38,7 @@ struct Context {
     int max_ctas = 0;  // persistent sweep grids: at most this many CTAs (0: n_sm)
     int window_cluster = -1;     // largest resident cluster of the windowed sweep (-1: not queried)
     int64_t window_smem = 0;     // its shared memory per CTA
-    int group_cluster = -1;      // largest resident cluster of the group sweep (-1: not queried)
+    GroupWindowLimits group_window{-1, {0, 0, 0}};  // of the group models' sweep (cluster -1: not queried)
     size_t budget = 0;
     size_t in_use = 0;
     cudaStream_t stream = nullptr;
@@ -109,6 +110,17 @@ struct DevWindow {
     WinScal* scal = nullptr;
     double2* bh = nullptr;
     double* share = nullptr;  // K, where a CTA's rows do not fit its shared memory
+    // group models: the CTAs' cuts, of the grouping that was current, and the grid
+    // form's exchange buffers
+    bool cluster = false;
+    int64_t grouping = -1;
+    int64_t most_rows = 0, most_groups = 0;
+    bool meet = false;  // a stratum spans CTAs
+    int32_t chain = 1;
+    GroupCut* cuts = nullptr;
+    double2* part = nullptr;
+    double* tails = nullptr;
+    double2* heads = nullptr;
 };
 
 // Device tables of the Breslow Cox engine (cox.cu).
@@ -126,16 +138,15 @@ struct CoxDev {
     void* tails = nullptr;
     int32_t* batch_cols = nullptr;
     double2* batch_out = nullptr;
-    // the persistent sweep (group_sweep.cu): active columns, the updated
-    // column's per-entry changes, scan aggregates, counters
-    int32_t* sweep_cols = nullptr;
-    double2* sweep_gh = nullptr;
-    double* dd = nullptr;
-    int32_t* ddg = nullptr;
-    int64_t dd_cap = 0;
-    void* agg = nullptr;
-    int64_t* counters = nullptr;
-    int64_t last_updates = 0, last_batches = 0;  // of the last persistent findMode
+    int64_t grouping = 0;  // changes when the rows are regrouped
+    // Cox: runs of groups that end with events or with their stratum, the grouping
+    // that the windowed sweep works on (block_rows); NB of them
+    int64_t NB = 0;
+    int32_t *blk = nullptr, *bgrp = nullptr;  // block of each row, first group of each block
+    double *bden = nullptr, *bD = nullptr, *bS1 = nullptr, *bS2 = nullptr, *bnev = nullptr;
+    uint8_t *bfirst = nullptr, *blast = nullptr;
+    int64_t* brow = nullptr;
+    int64_t* counters = nullptr;  // nonzero steps and rounds of the windowed sweep
 };
 
 int64_t cox_group_rows(const std::vector<int32_t>& pid0, const std::vector<double>& time,
@@ -185,7 +196,8 @@ struct Fit {
     std::vector<double> y_h, w_h, beta_h, pvar_h, time_h;
     std::vector<int64_t> stratum_h;
     std::vector<int32_t> pid0_h;
-    std::vector<int64_t> cox_grow_h;
+    std::vector<int64_t> cox_grow_h;    // first row of each stratum (grouped) or block (Cox), then K
+    std::vector<int32_t> cox_bstrat_h;  // Cox: stratum of each block
     std::vector<int32_t> ptype_h;
     std::vector<uint8_t> fixed;
     bool weighted = false;
@@ -242,8 +254,9 @@ struct Fit {
     void cox_objective_terms(double* out4);
     void cox_gh_batch(const int32_t* cols, int n, double2* out);
     void cox_update(int j, double delta);
-    // one findMode of the group engine in one persistent launch (group_sweep.cu)
-    void find_mode_group_sweep(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms);
+    // one findMode of the group engine in one launch (group_window.cu), and its plan
+    void ensure_group_window(int ctas, bool cluster);
+    void find_mode_group_window(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms);
     // mode-finding variants (modes_host.cu): the MM cycle, the KKT swindle, and
     // the MM all-coordinate (g, h) into out[J] (fixed may be nullptr)
     void find_mode_mm(const ccdb_mode_args& a, int* flag, int* iters, double* obj);

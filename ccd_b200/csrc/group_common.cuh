@@ -1,5 +1,5 @@
 // group_common.cuh -- device pieces shared by the group engine's per-call
-// kernels (cox.cu) and its persistent sweep (group_sweep.cu): the segmented
+// kernels (cox.cu): the segmented
 // block scan, and the gradient/Hessian of one column for the Breslow Cox and
 // the grouped (conditional logistic / Poisson) models, computed by one CTA.
 #pragma once

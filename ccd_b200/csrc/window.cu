@@ -50,63 +50,17 @@
 #include <algorithm>
 #include <cstdint>
 
-#include "common.cuh"
-#include "window_sweep.h"
+#include "window_device.cuh"
 
 namespace ccdb {
 
 namespace {
 
-constexpr int kHelpers = 4;                         // warps that look ahead for the others, one per scheduler
-constexpr int kWorkers = kWindow * 32;              // threads that hold columns
-constexpr int kT = kWorkers + 32 * kHelpers;
-constexpr int kWarps = kT / 32;
-constexpr int kE = 4;             // staged entries per lane
-constexpr int kStage = 32 * kE;   // a warp's column: its first entries, copied ahead
-constexpr unsigned kFull = 0xffffffffu;
-constexpr unsigned long long kWaitNs = 10ull * 1000 * 1000 * 1000;
+using namespace win;
 
 // What shared memory holds of a row: everything; the share alone; nothing; or, on
 // one CTA, xBeta and the denominator, from which a gather works the share out
 enum Where : int { kAllShared = 0, kShareShared = 1, kGlobal = 2, kPairShared = 3 };
-
-// The record of one position, copied ahead of its use.
-struct __align__(16) Rec {
-    WinCol c;
-    WinScal s;
-    double2 bh;
-    WinSlice e;
-    int64_t pad;
-};
-static_assert(kHelpers * 4 == kWindow, "eight lanes of a helper copy for a slot");
-static_assert(sizeof(WinScal) == 48 && sizeof(Rec) == 112, "copied in 16-byte pieces");
-
-// What the helpers decide between two rounds.
-struct __align__(16) Turn {
-    int base;      // the first position in flight
-    int limit;     // positions below it are in flight
-    int alone;     // base's column is the only one
-    int stop;      // the wait for the other CTAs ran out
-};
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned peer_u32(const void* p, int rank) {
-    unsigned a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-    return a;
-}
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // One entry's gradient and Hessian terms from its row's share
 // (ModelSpecifics.h:541-568 logistic, ModelSpecifics.h:1509-1530 Poisson).
@@ -237,9 +191,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
         s_abort = 0;
         if (CL) {
             for (int i = 0; i < 2 * kWindow * kWindowCluster; ++i) (&s_pair[0][0][0])[i] = make_double2(0.0, 0.0);
-            for (int i = 0; i < 2; ++i)
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_bar[i])) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            init_bars(s_bar, 2);
         }
     }
     if (CL) cluster_barrier();
@@ -257,39 +209,13 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
     auto send_pair = [&](double v) {
         const double h = __shfl_xor_sync(kFull, v, 16);
         const unsigned par = n_xch & 1;
-        if (lane < C)
-            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(
-                             to_pair + par * (unsigned)sizeof(s_pair[0])),
-                         "d"(v), "d"(h), "r"(to_bar + par * (unsigned)sizeof(s_bar[0]))
-                         : "memory");
+        if (lane < C) send16(to_pair + par * (unsigned)sizeof(s_pair[0]), to_bar + par * (unsigned)sizeof(s_bar[0]), v, h);
     };
     auto expect_pairs = [&](int columns) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&s_bar[n_xch & 1])),
-                     "r"((unsigned)(columns * C * 2 * sizeof(double)))
-                     : "memory");
-    };
-    auto arrived = [&](int bar, unsigned parity) {
-        unsigned done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-            " selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(smem_u32(&s_bar[bar])), "r"(parity)
-            : "memory");
-        return done != 0;
+        expect_bytes(&s_bar[n_xch & 1], (unsigned)(columns * C * 2 * sizeof(double)));
     };
     auto wait_pairs = [&]() {
-        const unsigned parity = (n_xch >> 1) & 1;
-        unsigned long long t0 = 0;
-        for (unsigned n = 0; !arrived(n_xch & 1, parity); ++n)  // an attempt sleeps in hardware for a while
-            if ((n & 15u) == 15u) {
-                const unsigned long long t = global_ns();
-                if (t0 == 0) t0 = t;
-                if (t - t0 > kWaitNs) {
-                    s_abort = 1;
-                    return;
-                }
-            }
+        if (!wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1)) s_abort = 1;
     };
     // the column's sums over the CTAs, the same bits in every lane and CTA (the
     // pairs of CTAs that there are not stay zero)
@@ -344,37 +270,9 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
 
     // ---- what the helpers copy ahead: records two columns ahead of a warp, entries one
     auto rec_of = [&](int at) -> Rec& { return s_rec[(at / kWindow) & 3][at & (kWindow - 1)]; };
-    // lane l8 of the eight that copy a record
-    auto fetch = [&](int at, Rec& r, int l8) {
-        if (at >= n_active) return;
-        const char* from = reinterpret_cast<const char*>(l8 < 2   ? (const void*)(R.cols + at)
-                                                         : l8 < 5 ? (const void*)(R.scal + at)
-                                                                  : (const void*)(R.bh + at));
-        if (l8 < 6) cp_async16(reinterpret_cast<char*>(&r) + 16 * l8, from + 16 * (l8 < 2 ? l8 : l8 < 5 ? l8 - 2 : 0));
-        else if (l8 == 6) cp_async8(&r.e, slices + at);
-    };
-    auto fetched = [&]() {
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncwarp();
-    };
-    // the first kStage entries of the column at a position
-    auto buffer_of = [&](int at) { return (((at / kWindow) & 1) * kWindow + (at & (kWindow - 1))) * kStage; };
-    auto stage = [&](int at, int l8) {
-        if (at >= n_active) return;
-        const Rec& r = rec_of(at);
-        if (r.c.flags & 8) return;
-        const int n = min(r.e.hi - r.e.lo, kStage);
-        const int32_t* from = P.rows + r.c.cb + r.e.lo;
-        const double* vfrom = P.vals + r.c.vb + r.e.lo;
-        int32_t* to = s_rows + buffer_of(at);
-        double* vto = s_vals + buffer_of(at);
-#pragma unroll 2
-        for (int p = l8; p < n; p += 8) {
-            if (r.c.flags & 1) cp_async4(to + p, from + p);
-            else to[p] = r.e.lo + p;
-            if (r.c.flags & 2) cp_async8(vto + p, vfrom + p);
-        }
-    };
+    const Ahead ahead{R.cols, R.scal, R.bh, slices, P.rows, P.vals, n_active};
+    auto fetch = [&](int at, int l8) { ahead.record(at, rec_of(at), l8); };
+    auto stage = [&](int at, int l8) { ahead.entries(at, rec_of(at), s_rows + stage_at(at), s_vals + stage_at(at), l8); };
 
     double last = 0.0;
     unsigned long long moved = 0;
@@ -404,11 +302,11 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
             const int me = wid - kWindow;
             int q = lane < kWindow ? lane : 0x7fffffff;  // the slot's position
             const int l8 = lane & 7, mine = me + kHelpers * (lane >> 3);  // eight lanes a slot
-            for (int i = 0; i < 3; ++i) fetch(mine + i * kWindow, rec_of(mine + i * kWindow), l8);
-            fetched();
+            for (int i = 0; i < 3; ++i) fetch(mine + i * kWindow, l8);
+            ahead.done();
             stage(mine, l8);
             stage(mine + kWindow, l8);
-            fetched();
+            ahead.done();
             unsigned moved_on = 0;  // the slots that took up a new column in the last round
             Turn t{0, 0, 0, 0};
             // what is in flight next: a column runs alone when it is long, or medium and
@@ -454,7 +352,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 const int at = __shfl_sync(kFull, q, mine);
                 if (moved_on >> mine & 1u) {
                     stage(at + kWindow, l8);
-                    fetch(at + 2 * kWindow, rec_of(at + 2 * kWindow), l8);
+                    fetch(at + 2 * kWindow, l8);
                 }
                 if (CL) ++n_xch;
                 __syncthreads();
@@ -469,7 +367,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 moved_on = taken;
                 t.stop = CL ? s_abort : 0;
                 next_turn();
-                fetched();
+                ahead.done();
                 __syncthreads();
             }
         } else {
@@ -486,8 +384,8 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 const Rec& r = rec_of(alone ? now.base : pos);
                 const int n = r.e.hi - r.e.lo, flags = r.c.flags;
                 const bool ind = flags & 4, has_vals = flags & 2;
-                const int32_t* const kr = s_rows + buffer_of(pos);
-                const double* const xr = s_vals + buffer_of(pos);
+                const int32_t* const kr = s_rows + stage_at(pos);
+                const double* const xr = s_vals + stage_at(pos);
                 // entry e of the slice, from global memory: local row and value
                 auto entry_row = [&](int e) { return ((flags & 1) ? __ldg(P.rows + r.c.cb + r.e.lo + e) : r.e.lo + e) - (int)r0; };
                 auto entry_val = [&](int e) { return has_vals ? __ldg(P.vals + r.c.vb + r.e.lo + e) : 1.0; };
@@ -517,7 +415,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                     double v = warp_pair_sum(g, h);
                     if (alone) {
                         if ((lane & 15) == 0) s_red[wid][lane >> 4] = v;
-                        asm volatile("bar.sync 1, %0;" ::"n"(kWorkers) : "memory");
+                        workers_barrier();
                         v = s_red[lane & 15][lane >> 4];
 #pragma unroll
                         for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
@@ -576,9 +474,8 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
         if (failed && tid == 0 && atomicCAS(&P.st->error, 0, E_WAIT_CLUSTER) == 0) P.st->error_where = rank;
         cluster_barrier();  // no CTA leaves while another may still send to it
         if (failed) {  // pairs already sent to this CTA land before it leaves
-            const unsigned long long t0 = global_ns();
             const unsigned m = n_xch - 1;  // the exchange that gave up
-            while (!arrived(m & 1, (m >> 1) & 1) && global_ns() - t0 < 1000000000ull) __nanosleep(200);
+            drain(&s_bar[m & 1], (m >> 1) & 1);
             return;
         }
     }

@@ -11,12 +11,6 @@ breakdown by segment kind.
 engine: CTA 0's SM clock at six points of every column of one sweep
 (``CCDB_BATCH_TRACE_SWEEP``, default 1).  ``python -m ccd_b200.trace --batch
 <path> [sm_mhz]`` prints the per-phase breakdown.
-
-The group sweep writes its own format to the same ``CCDB_TRACE_FILE`` (the
-last findMode of the process wins):
-
-* ``--group <path>``: the group sweep (Cox), CTA 0's global timer at eight
-  points of each of the first 4,096 nonzero steps.
 """
 from __future__ import annotations
 
@@ -97,23 +91,8 @@ def summarise_batch(path: str, sm_mhz: float = 1965.0) -> str:
     return "\n".join(out)
 
 
-def summarise_group(path: str) -> str:
-    """Per-stage timing of the group sweep's nonzero steps (Cox)."""
-    t = np.fromfile(path, dtype=np.uint64).reshape(-1, 8).astype(np.int64)
-    t = t[t[:, 0] > 0]
-    d = np.diff(t, axis=1) / 1e3
-    names = ["gradients of the batch + barrier", "rows + barrier", "denominators + barrier",
-             "rebuild phase 1 + barrier", "rebuild phase 2 + barrier", "rebuild phase 3 + barrier"]
-    lines = [f"nonzero steps traced {len(t)}"]
-    lines += [f"{n}: median {np.median(d[:, i]):.2f} us" for i, n in enumerate(names)]
-    lines.append(f"one nonzero step: median {np.median(np.diff(t[:, 0])) / 1e3:.2f} us")
-    return "\n".join(lines)
-
-
 if __name__ == "__main__":
     if sys.argv[1] == "--batch":
         print(summarise_batch(sys.argv[2], *(float(a) for a in sys.argv[3:4])))
-    elif sys.argv[1] == "--group":
-        print(summarise_group(sys.argv[2]))
     else:
         print(summarise(sys.argv[1]))

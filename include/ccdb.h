@@ -195,11 +195,11 @@ typedef struct {
                                   findMode on one thread-block cluster of 1 to 16 CTAs, sixteen
                                   consecutive columns in flight), _GRID_LEVELS the grid-wide
                                   level sweep, _SPECULATIVE host-driven batches of gradients
-                                  that restart after each nonzero step.  Cox and conditional models: one
-                                  persistent launch per findMode of device-driven speculative
-                                  batches -- one thread-block cluster with hardware barriers
-                                  for fits a few SMs cover (forced by _LEVELS), else a
-                                  cooperative grid (forced by _GRID_LEVELS) -- or with
+                                  that restart after each nonzero step.  Cox and conditional models:
+                                  the windowed sweep of the group engine, one launch per findMode
+                                  on one thread-block cluster (forced by _LEVELS) or, for fits
+                                  that its shared memory does not hold or whose columns are long,
+                                  a cooperative grid (forced by _GRID_LEVELS) -- or with
                                   _SPECULATIVE the host-driven batches */
     int32_t algorithm;         /* AlgorithmType (Types.h:149-153): CCDB_ALGORITHM_CCD (0,
                                   default) or CCDB_ALGORITHM_MM (findMode's MM cycle,
