@@ -925,7 +925,11 @@ def run_cv(args, world, rank, local, collect=False):
     byts = cv_bytes(d, res_all)
     achieved = byts / (t / args.steps) / 1e9
     sweeps = [r["iterations"] for r in res_all]
-    kernel = "batch_mixed_kernel<LOGISTIC>" if mixed else "batch_sweep_kernel<LOGISTIC>"
+    lens = np.sort(np.diff(d.col_start))[:-1]
+    if mixed and group or lens.mean() > 640:  # the engine's rule for columns too long to step side by side
+        kernel = "batch_mixed_kernel<LOGISTIC>" if mixed else "batch_sweep_kernel<LOGISTIC>"
+    else:
+        kernel = "batch_window_kernel<LOGISTIC>"
     line = {
         "metric": "converged fits/s", "value": fits / t, "unit": "fits/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * t / args.steps,

@@ -21,6 +21,7 @@
 
 #include "../../include/ccdb.h"
 #include "batch.h"
+#include "batch_window.h"
 #include "csr_device.h"
 #include "csr_host.h"
 #include "engine.h"
@@ -90,6 +91,15 @@ int64_t Matrix::entries(int j) const {
     return col_start[j + 1] - col_start[j];
 }
 
+int64_t Matrix::mean_entries() const {
+    int64_t sum = 0, longest = 0;
+    for (int j = 0; j < J; ++j) {
+        sum += entries(j);
+        longest = std::max(longest, entries(j));
+    }
+    return J > 1 ? (sum - longest) / (J - 1) : longest;
+}
+
 Matrix::~Matrix() {
     for (void* p : {(void*)d_col_ptr, (void*)d_rows, (void*)d_val_ptr, (void*)d_vals, (void*)d_fmt,
                     (void*)d_row_ptr, (void*)d_csr_col, (void*)d_csr_val})
@@ -140,6 +150,7 @@ Fit::~Fit() {
         ctx->release(p);
     release_schedule();
     release_window();
+    release_batch_window();
     if (group_engine()) cox_release();
 }
 
@@ -694,6 +705,43 @@ void Fit::ensure_window(int ctas) {
     window->n_active = (int32_t)n;
     window->fixed = fixed;
     window->ctas = ctas;
+}
+
+// The batched fits' plan: every column but an offset one, whole on one CTA.
+void Fit::ensure_batch_window() {
+    if (batch_window) return;
+    const BatchTeam t = batch_team(m->mean_entries());
+    std::vector<uint8_t> skip(J, 0);
+    if (offset_col0) skip[0] = 1;
+    const WindowPlan plan = build_window_plan(K, J, m->col_start.data(), m->rows_h.data(), m->val_start.data(),
+                                              m->fmt.data(), skip.data(), 1, t.short_entries, t.long_entries);
+    std::vector<int32_t> longs;
+    std::unique_ptr<DevWindow> w(new DevWindow());
+    for (size_t q = 0; q < plan.cols.size(); ++q) {
+        const WinCol& c = plan.cols[q];
+        if (c.flags & 8) longs.push_back((int32_t)q);
+        w->any_vals |= (c.flags & 2) != 0;
+        w->entries += c.n;
+    }
+    w->n_active = (int32_t)plan.cols.size();
+    w->n_long = (int32_t)longs.size();
+    w->team = t.warps;
+    release_batch_window();
+    batch_window = std::move(w);  // owned by the fit from here on
+    try {
+        batch_window->cols = upload(ctx, plan.cols.data(), plan.cols.size(), stream);
+        batch_window->slices = upload(ctx, plan.slices.data(), plan.slices.size(), stream);
+        batch_window->longs = upload(ctx, longs.data(), longs.size(), stream);
+    } catch (...) {
+        release_batch_window();
+        throw;
+    }
+}
+
+void Fit::release_batch_window() {
+    if (!batch_window) return;
+    for (void* p : {(void*)batch_window->cols, (void*)batch_window->slices, (void*)batch_window->longs}) ctx->release(p);
+    batch_window.reset();
 }
 
 void Fit::find_mode_window(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms) {
@@ -1429,6 +1477,17 @@ static int batch_cluster_size(const Matrix* m, int64_t K, int n_groups, int n_sm
     return 8;
 }
 
+// Whether the windowed engine serves a batch whose caller names no launch shape:
+// short columns, and a workspace within the context's memory budget.
+static bool batch_windowed(Context* ctx, const Matrix* m, int64_t K, int n, int ctas, bool mixed, int spill) {
+    if (m->mean_entries() > kBatchWindowMean) return false;
+    const size_t J = m->J, state = (spill & 1 ? 8 : 0) + (spill & 2 ? (mixed ? 4 : 8) : 0);
+    const size_t bytes = ctas * ((sizeof(WinScal) + sizeof(double2)) * J + state * K) + sizeof(double) * J * n +
+                         (sizeof(WinCol) + sizeof(WinSlice) + sizeof(int32_t)) * J + 4096;
+    std::lock_guard<std::mutex> g(ctx->mu);
+    return !ctx->budget || ctx->in_use + bytes <= ctx->budget;
+}
+
 int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_args* a, double* beta_out,
                          ccdb_batch_result* results, double* device_seconds) {
     return guard([&] {
@@ -1504,17 +1563,49 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
         P.order = (const int32_t*)keep(upload(ctx, order.data(), (size_t)n, s));
         P.results = (BatchResult*)keep(ctx->alloc(sizeof(BatchResult) * n));
         int G = 1, n_groups = n;
-        if (mixed) {
+        // CCDB_BATCH_TRACE_FILE: per-column phase clocks of CTA 0 in one sweep
+        // (CCDB_BATCH_TRACE_SWEEP, default 1) of the mixed lockstep engine, written as int64 [J][6]
+        const char* trace_path = mixed ? std::getenv("CCDB_BATCH_TRACE_FILE") : nullptr;
+        if (mixed && K > kKeyRowMask)
+            throw Error(CCDB_ERR_UNSUPPORTED, "mixed batched fits: at most 16,777,215 rows");
+        for (int i = 0; mixed && i < n; ++i)
+            if (hold[i] >= kKeyNoFold)
+                throw Error(CCDB_ERR_UNSUPPORTED, "mixed batched fits: held-out fold ids below 127");
+        BatchWindowParams W{};
+        bool any_vals = false;
+        for (int j = f->offset_col0 ? 1 : 0; j < J; ++j) any_vals |= m->fmt[j] == F_SPARSE || m->fmt[j] == F_DENSE;
+        const int ctas = std::min(n, ctx->n_sm);
+        int spill = 0;
+        check_cuda(batch_window_spill(K, mixed, any_vals, &spill), "batch sweep");
+        const bool shaped = mixed && (b->group || b->cluster || trace_path);  // asks for the lockstep engine
+        const bool windowed = !shaped && batch_windowed(ctx, m, K, n, ctas, mixed, spill);
+        if (windowed) {
+            f->ensure_batch_window();
+            const DevWindow& w = *f->batch_window;
+            W.cols = w.cols;
+            W.slices = w.slices;
+            W.longs = w.longs;
+            W.n_active = w.n_active;
+            W.n_long = w.n_long;
+            W.entries = w.entries;
+            W.any_vals = w.any_vals ? 1 : 0;
+            W.mixed = mixed ? 1 : 0;
+            W.team = w.team;
+            W.ctas = ctas;
+            const size_t cols = (size_t)W.ctas * std::max(W.n_active, 1);
+            W.scal = (WinScal*)keep(ctx->alloc(sizeof(WinScal) * cols));
+            W.bh = (double2*)keep(ctx->alloc(sizeof(double2) * cols));
+            if (spill & 1) W.xbeta = (double*)keep(ctx->alloc(sizeof(double) * (size_t)K * W.ctas));
+            if (spill & 2) W.share = (double*)keep(ctx->alloc((mixed ? 4 : 8) * (size_t)K * W.ctas));
+            P.queue = (int32_t*)keep(ctx->alloc(sizeof(int32_t)));
+            check_cuda(cudaMemsetAsync(P.queue, 0, sizeof(int32_t), s), "batch queue");
+            W.beta_out = P.beta = (double*)keep(ctx->alloc(sizeof(double) * (size_t)J * n));
+        } else if (mixed) {
             G = b->group ? b->group : batch_group_size(m, n, ctx->n_sm);
             if (G != 1 && G != 2 && G != 4) throw Error(CCDB_ERR_INVALID, "batch group must be 1, 2 or 4");
             n_groups = (n + G - 1) / G;
             P.group = G;
-            // the mixed engine reads each entry's fold with its row id (row | fold << 24)
-            if (K > kKeyRowMask)
-                throw Error(CCDB_ERR_UNSUPPORTED, "mixed batched fits: at most 16,777,215 rows");
-            for (int i = 0; i < n; ++i)
-                if (hold[i] >= kKeyNoFold)
-                    throw Error(CCDB_ERR_UNSUPPORTED, "mixed batched fits: held-out fold ids below 127");
+            // the lockstep engine reads each entry's fold with its row id (row | fold << 24)
             const int64_t nnz = m->col_start.back();
             int32_t* keys = (int32_t*)keep(ctx->alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(nnz, 1)));
             check_cuda(launch_batch_keys(m->d_rows, nnz, P.row_fold, keys, s), "batch keys");
@@ -1554,9 +1645,6 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
             P.hdelta = (double*)keep(ctx->alloc(sizeof(double) * (size_t)J * n));
             P.xjy = (double*)keep(ctx->alloc(sizeof(double) * (size_t)J * n));
         }
-        // CCDB_BATCH_TRACE_FILE: per-column phase clocks of CTA 0 in one sweep
-        // (CCDB_BATCH_TRACE_SWEEP, default 1) of the mixed engine, written as int64 [J][6]
-        const char* trace_path = mixed ? std::getenv("CCDB_BATCH_TRACE_FILE") : nullptr;
         if (trace_path) {
             const char* sw = std::getenv("CCDB_BATCH_TRACE_SWEEP");
             P.trace_sweep = sw ? std::atoi(sw) : 1;
@@ -1567,8 +1655,10 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
         check_cuda(cudaEventCreate(&e0), "event");
         check_cuda(cudaEventCreate(&e1), "event");
         check_cuda(cudaEventRecord(e0, s), "event");
-        if (mixed) check_cuda(launch_batch_mixed(P, s), "batch sweep (mixed)");
-        else check_cuda(launch_batch_sweep(P, s), "batch sweep");
+        W.P = P;
+        if (windowed) check_cuda(launch_batch_window(W, s), "batch sweep");
+        else if (mixed) check_cuda(launch_batch_mixed(P, s), "batch sweep (lockstep)");
+        else check_cuda(launch_batch_sweep(P, s), "batch sweep (one column at a time)");
         check_cuda(cudaEventRecord(e1, s), "event");
         check_cuda(f->ctx->wait(), "batch sync");  // the sweep is done before a copy is queued behind it
         std::vector<BatchResult> res(n);
@@ -1578,7 +1668,7 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
         if (P.abort)
             check_cuda(cudaMemcpyAsync(&aborted, P.abort, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "abort word");
         std::vector<double> bg;
-        if (beta_out && mixed) {
+        if (beta_out && P.beta_g) {
             bg.resize((size_t)J * G * n_groups);
             check_cuda(cudaMemcpyAsync(bg.data(), P.beta_g, sizeof(double) * bg.size(), cudaMemcpyDeviceToHost, s),
                        "beta");
@@ -1596,7 +1686,7 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
                 std::fclose(fh);
             }
         }
-        if (beta_out && mixed)  // [group][J][G] -> [instance][J]
+        if (beta_out && P.beta_g)  // [group][J][G] -> [instance][J]
             for (int q = 0; q < n; ++q) {
                 const int grp = q / G, gi = q % G, inst = order[q];
                 for (int j = 0; j < J; ++j) beta_out[(size_t)inst * J + j] = bg[((size_t)grp * J + j) * G + gi];

@@ -83,6 +83,7 @@ struct Matrix {
     double* d_csr_val = nullptr;
 
     int64_t entries(int j) const;
+    int64_t mean_entries() const;  // of the columns but the longest
     void ensure_csr(cudaStream_t s);
     ~Matrix();
 };
@@ -105,6 +106,10 @@ struct DevWindow {
     int ctas = 0;
     int32_t n_active = 0;
     bool any_vals = false;
+    // batched fits: the long columns' positions, the entries of all
+    int32_t n_long = 0, team = 1;
+    int64_t entries = 0;
+    int32_t* longs = nullptr;
     WinCol* cols = nullptr;
     WinSlice* slices = nullptr;
     WinScal* scal = nullptr;
@@ -236,8 +241,11 @@ struct Fit {
     int window_ctas();
     void ensure_window(int ctas);
     void release_window();
+    void ensure_batch_window();
+    void release_batch_window();
     void find_mode_window(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms);
     std::unique_ptr<DevWindow> window;
+    std::unique_ptr<DevWindow> batch_window;
     int32_t* d_batch_cols = nullptr;  // independent-row models
     double2* d_batch_out = nullptr;
     bool is_cox() const { return model == M_COX; }

@@ -6,8 +6,10 @@
 
 #ifdef __CUDACC__
 #define CCDB_HD __host__ __device__ __forceinline__
+#define CCDB_HD_COLD static __host__ __device__ __noinline__
 #else
 #define CCDB_HD inline
+#define CCDB_HD_COLD inline
 #endif
 
 namespace ccdb {
@@ -48,6 +50,12 @@ CCDB_HD double newton_prior_delta(double g, double h, double beta, int ptype, do
     return newton_prior_delta_l(g, h, beta, ptype, var, ptype == 1 ? sqrt(2.0 / var) : 0.0);
 }
 
+// The Laplace step where the Hessian is not positive and finite, out of the way
+// of the kernels that step through millions of ordinary ones.
+CCDB_HD_COLD double laplace_delta_cold(double g, double h, double beta, double lambda) {
+    return newton_prior_delta_l(g, h, beta, 1, 0.0, lambda);
+}
+
 // newton_prior_delta_l as one quotient num / den whose numerator is chosen before
 // the division: for a positive finite h the sign of each of the two Laplace
 // quotients is its numerator's, so only the one that is taken is divided, and a
@@ -57,7 +65,7 @@ CCDB_HD double newton_quotient_step(double g, double h, double beta, int ptype, 
                                     double inv_var, double b_var) {
     double num, den;
     if (ptype == 1) {
-        if (!(h > 0.0 && h <= 1.7976931348623157e308)) return newton_prior_delta_l(g, h, beta, 1, var, lambda);
+        if (!(h > 0.0 && h <= 1.7976931348623157e308)) return laplace_delta_cold(g, h, beta, lambda);
         if (beta == 0.0 && !(fabs(g) > lambda)) return 0.0;
         num = (beta > 0.0 || (beta == 0.0 && g < 0.0)) ? g + lambda : g - lambda;
         den = h;

@@ -44,6 +44,7 @@ struct WindowPlan {
 constexpr int64_t window_row(int64_t K, int r, int C) { return K * r / C; }
 
 WindowPlan build_window_plan(int64_t K, int32_t J, const int64_t* col_start, const int32_t* rows,
-                             const int64_t* val_start, const uint8_t* fmt, const uint8_t* fixed, int C);
+                             const int64_t* val_start, const uint8_t* fmt, const uint8_t* fixed, int C,
+                             int64_t short_entries = kWindowShort, int64_t long_entries = kWindowLong);
 
 }  // namespace ccdb

@@ -98,6 +98,13 @@ __device__ __forceinline__ void init_bars(uint64_t* bars, int n) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bars + i)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
+// A copy of `bytes` (a multiple of 16, from and to 16-byte boundaries) to this CTA's
+// shared memory by the copy engine, counted by `bar`.
+__device__ __forceinline__ void bulk_copy(void* to, const void* from, unsigned bytes, const uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(to)),
+                 "l"(from), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
 // What was sent to a CTA that gave up an exchange lands before it leaves (bounded).
 __device__ __forceinline__ void drain(const uint64_t* bar, unsigned parity) {
     const unsigned long long t0 = global_ns();
@@ -123,14 +130,15 @@ struct Ahead {
         if (l8 < 6) cp_async16(reinterpret_cast<char*>(&r) + 16 * l8, from + 16 * (l8 < 2 ? l8 : l8 < 5 ? l8 - 2 : 0));
         else if (l8 == 6) cp_async8(&r.e, slices + at);
     }
-    // its first kStage entries
+    // its first STAGE entries, by LANES lanes
+    template <int STAGE = kStage, int LANES = 8>
     __device__ __forceinline__ void entries(int at, const Rec& r, int32_t* to, double* vto, int l8) const {
         if (at >= n_active || (r.c.flags & 8)) return;
-        const int n = min(r.e.hi - r.e.lo, kStage);
+        const int n = min(r.e.hi - r.e.lo, STAGE);
         const int32_t* from = rows + r.c.cb + r.e.lo;
         const double* vfrom = vals + r.c.vb + r.e.lo;
 #pragma unroll 2
-        for (int p = l8; p < n; p += 8) {
+        for (int p = l8; p < n; p += LANES) {
             if (r.c.flags & 1) cp_async4(to + p, from + p);
             else to[p] = r.e.lo + p;
             if (r.c.flags & 2) cp_async8(vto + p, vfrom + p);
@@ -144,7 +152,8 @@ struct Ahead {
 };
 
 // where the staged entries of a position lie
-__device__ __forceinline__ int stage_at(int pos) { return (((pos / kWindow) & 1) * kWindow + (pos & (kWindow - 1))) * kStage; }
+template <int STAGE = kStage, int WINDOW = kWindow>
+__device__ __forceinline__ int stage_at(int pos) { return (((pos / WINDOW) & 1) * WINDOW + (pos & (WINDOW - 1))) * STAGE; }
 
 }  // namespace win
 }  // namespace ccdb

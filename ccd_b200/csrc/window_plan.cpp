@@ -32,7 +32,8 @@ uint16_t by_position(uint32_t distances) {
 }  // namespace
 
 WindowPlan build_window_plan(int64_t K, int32_t J, const int64_t* col_start, const int32_t* rows,
-                             const int64_t* val_start, const uint8_t* fmt, const uint8_t* fixed, int C) {
+                             const int64_t* val_start, const uint8_t* fmt, const uint8_t* fixed, int C,
+                             int64_t short_entries, int64_t long_entries) {
     WindowPlan w;
     int32_t n_active = 0;
     for (int32_t j = 0; j < J; ++j) n_active += (fixed && fixed[j]) ? 0 : 1;
@@ -71,8 +72,8 @@ WindowPlan build_window_plan(int64_t K, int32_t J, const int64_t* col_start, con
         }
         uint32_t dist = n > 0 ? all_rows : 0;
         bool holds_all = false;
-        if (longest > kWindowShort) c.flags |= 16;
-        if (longest > kWindowLong) {
+        if (longest > short_entries) c.flags |= 16;
+        if (longest > long_entries) {
             c.flags |= 8;  // never in flight beside another column: its conflicts are not needed
         } else if (!has_rows) {
             dist = any_row;

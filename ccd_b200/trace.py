@@ -7,8 +7,8 @@ the warp phase, arrival.  ``python -m ccd_b200.trace <path>`` prints where the
 time of a sweep goes: level-to-level detection, per-level span, and the phase
 breakdown by segment kind.
 
-``CCDB_BATCH_TRACE_FILE=<path>`` does the same for the mixed-precision batched
-engine: CTA 0's SM clock at six points of every column of one sweep
+``CCDB_BATCH_TRACE_FILE=<path>`` does the same for mixed-precision batched fits,
+which then run the lockstep engine: CTA 0's SM clock at six points of every column of one sweep
 (``CCDB_BATCH_TRACE_SWEEP``, default 1).  ``python -m ccd_b200.trace --batch
 <path> [sm_mhz]`` prints the per-phase breakdown.
 """

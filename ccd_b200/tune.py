@@ -85,7 +85,7 @@ def filling(candidates, n_instances: int, n_sm: int):
 
 
 def tune_batch(fit, variance, holdout, row_fold, args=None, candidates=None) -> BatchChoice:
-    """The (group, cluster) of the mixed-precision batched engine that runs one
+    """The (group, cluster) of the mixed-precision lockstep engine that runs one
     sweep of this grid fastest among the shapes that occupy every SM.  `fit` is a
     native.Fit (or anything with its batch_find_mode and ctx.sm_count); the grid
     is the one about to be fitted."""

@@ -284,9 +284,10 @@ typedef struct {
  * uses args->prior_type per column with variance[i], and starts from beta = 0.
  * Each instance runs the sequential sweep of a standalone fit; instances do not
  * interact.  Logistic and Poisson models.  beta_out: n_instances x J.
- * A CCDB_PRECISION_MIXED fit runs the mixed-precision engine, whose instances
- * step through the columns in lockstep groups of batch->group (at most
- * 16,777,215 rows; held-out fold ids below 127). */
+ * Fits with short columns run the windowed sweep, one CTA an instance.  A
+ * CCDB_PRECISION_MIXED fit with long columns, or whose caller gives a group or a
+ * cluster, steps lockstep groups of batch->group instances through the columns
+ * (mixed fits: at most 16,777,215 rows; held-out fold ids below 127). */
 int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* batch, const ccdb_mode_args* args,
                          double* beta_out, ccdb_batch_result* results, double* device_seconds);
 
