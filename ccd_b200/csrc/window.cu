@@ -37,13 +37,15 @@
 // A round is a chain of latencies (gather, warp sum, exchange, FP64 division,
 // exp): nothing in it is bound by bandwidth, so what counts is how many dependent
 // instructions it has and how many columns it takes.  Measured on a B200 at
-// 1,965 MHz, a round is about 3,500 SM clocks (gather and warp sum 900, exchange
-// 500, sums and step 750, update 750, two barriers and skew the rest) and takes
-// 5.7 columns of the 10,000 x 1,001 L1 logistic fit: 4.5 ms a fit, where
+// 1,965 MHz, a round is about 3,200 SM clocks (gather and warp sum 900, exchange
+// 500, sums and step 550, update 750, two barriers and skew the rest) and takes
+// 5.7 columns of the 10,000 x 1,001 L1 logistic fit: 4.2 ms a fit, where
 // speculative batches on one CTA that recomputed exp and divided for every
-// gathered entry took 9.3 ms.  60,000 x 2,501 L1 logistic: 51 ms; Poisson, 50,000
-// x 4,002, every step nonzero: 138 ms; both ran one cluster barrier per
-// dependency level before, at 217 and 398 ms.
+// gathered entry took 9.3 ms.  60,000 x 2,501 L1 logistic: 45 ms; Poisson, 50,000
+// x 4,002, every step nonzero: 136 ms; both ran one cluster barrier per
+// dependency level before, at 217 and 398 ms.  Short straight code counts: with
+// the CTAs' pairs added four at a time in every lane, bounds settled by the warps
+// with columns and the gather unrolled, these took 4.5, 53 and 154 ms.
 //
 // The wait for the other CTAs' pairs is bounded (kWaitNs): a wait that runs out
 // records an error and the CTA leaves through the closing cluster barrier.
@@ -145,7 +147,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
     __shared__ double s_red[kWindow][2];
     __shared__ double4 s_red4[kWarps];
     __shared__ double4 s_obj[kWindowCluster];
-    __shared__ int s_moves[kWindow];        // the column's step is nonzero
+    __shared__ double s_delta[2][kWindow];  // by round parity: the column's step
     __shared__ unsigned s_holders[kWindow];  // the slots that hold the column back if they move
     __shared__ Turn s_turn;
     __shared__ uint64_t s_bar[2];
@@ -218,17 +220,14 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
         if (!wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1)) s_abort = 1;
     };
     // the column's sums over the CTAs, the same bits in every lane and CTA (the
-    // pairs of CTAs that there are not stay zero)
+    // pairs of CTAs that there are not stay zero): lane l takes CTA l & 15, its g
+    // below lane 16 and its h above
     auto pair_sum = [&](int c) {
-        const double2* from = s_pair[n_xch & 1][c];
-        double2 t = make_double2(0.0, 0.0);
-#pragma unroll 1
-        for (int i = 0; i < C; i += 4) {
-            const double2 a = from[i], b = from[i + 1], e = from[i + 2], f = from[i + 3];
-            t.x += (a.x + b.x) + (e.x + f.x);
-            t.y += (a.y + b.y) + (e.y + f.y);
-        }
-        return t;
+        const double* from = &s_pair[n_xch & 1][c][lane & 15].x;
+        double v = from[lane >> 4];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+        return v;
     };
 
     // ---- the objective terms {LL numerator, LL denominator, gradient objective,
@@ -308,6 +307,21 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
             stage(mine + kWindow, l8);
             ahead.done();
             unsigned moved_on = 0;  // the slots that took up a new column in the last round
+            int par = 0;
+            // the bound of a column whose step was taken in the last round, and its
+            // coefficient where the step moved it (lane l: slot l), off the warps' path
+            auto settle = [&]() {
+                if (rank != 0 || me != kHelpers - 1 || !(moved_on >> lane & 1u)) return;
+                const Rec& r = rec_of(q - kWindow);
+                const double d = s_delta[par ^ 1][lane];
+                double2 bh = r.bh;
+                apply_bounds(d, bh.y);
+                if (d != 0.0) {
+                    bh.x += d;
+                    P.beta[r.c.j] = bh.x;
+                }
+                R.bh[q - kWindow] = bh;
+            };
             Turn t{0, 0, 0, 0};
             // what is in flight next: a column runs alone when it is long, or medium and
             // expected to move (nothing holds it at zero, or a warp has found its step)
@@ -354,10 +368,11 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                     stage(at + kWindow, l8);
                     fetch(at + 2 * kWindow, l8);
                 }
+                settle();
                 if (CL) ++n_xch;
                 __syncthreads();
                 // ---- which steps stand, and what is in flight next
-                const unsigned moves = __ballot_sync(kFull, flying && s_moves[lane & (kWindow - 1)]);
+                const unsigned moves = __ballot_sync(kFull, flying && s_delta[par][lane & (kWindow - 1)] != 0.0);
                 bool stands = flying && (s_holders[lane & (kWindow - 1)] & moves) == 0;
                 found = stands && !t.alone && (moves >> lane & 1u) && (rec_of(q).c.flags & 16);
                 stands = stands && !found;
@@ -365,15 +380,18 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 if (me == 0 && lane == 0) moved += __popc(taken & moves);
                 if (taken >> lane & 1u) q += kWindow;
                 moved_on = taken;
+                par ^= 1;
                 t.stop = CL ? s_abort : 0;
                 next_turn();
                 ahead.done();
                 __syncthreads();
             }
+            settle();
         } else {
             // ================ a warp with a column
             int pos = wid;
             bool fresh = true;  // the column's first round
+            int par = 0;
             __syncthreads();
             __syncthreads();
             for (;;) {
@@ -390,20 +408,16 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 auto entry_row = [&](int e) { return ((flags & 1) ? __ldg(P.rows + r.c.cb + r.e.lo + e) : r.e.lo + e) - (int)r0; };
                 auto entry_val = [&](int e) { return has_vals ? __ldg(P.vals + r.c.vb + r.e.lo + e) : 1.0; };
                 const int first = alone ? tid : lane + kStage, stride = alone ? kWorkers : 32;
-                double d = 0.0, hd = 0.0, b0 = 0.0;
+                double d = 0.0;
                 if (mine) {
                     double g = 0.0, h = 0.0;
                     if (!alone) {
-#pragma unroll
-                        for (int i = 0; i < kE; ++i)
-                            if (32 * i < n) {
-                                const int e = lane + 32 * i;
-                                if (e < n) {
-                                    const int k = kr[e] - (int)r0;
-                                    add_terms<MODEL>(ind, WT, has_vals ? xr[e] : 1.0, rows.p(k), rows.weight(k), g, h);
-                                    if (fresh) rows.expect(k);
-                                }
-                            }
+#pragma unroll 1
+                        for (int e = lane; e < min(n, kStage); e += 32) {
+                            const int k = kr[e] - (int)r0;
+                            add_terms<MODEL>(ind, WT, has_vals ? xr[e] : 1.0, rows.p(k), rows.weight(k), g, h);
+                            if (fresh) rows.expect(k);
+                        }
                     }
                     if (alone || n > kStage) {
 #pragma unroll 4
@@ -421,26 +435,24 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                         for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
                     }
                     if (CL && (!alone || wid == slot)) send_pair(v);
-                    b0 = r.bh.x;
-                    hd = r.bh.y;
+                    const double b0 = r.bh.x, hd = r.bh.y;
                     const double b_var = r.s.ptype == 2 ? b0 / r.s.pvar : 0.0;
-                    double2 t;
                     if (CL) {
                         wait_pairs();
-                        t = pair_sum(slot);
-                    } else {
-                        t = make_double2(__shfl_sync(kFull, v, 0), __shfl_sync(kFull, v, 16));
+                        v = pair_sum(slot);
                     }
+                    double2 t = make_double2(__shfl_sync(kFull, v, 0), __shfl_sync(kFull, v, 16));
                     if (r.c.n > 0) t.x -= r.s.xjy;
                     else t = make_double2(0.0, 0.0);  // an empty column gives (0, 0) (ModelSpecifics.hpp:720-723)
                     d = newton_quotient_step(t.x, t.y, b0, r.s.ptype, r.s.pvar, r.s.lambda, r.s.inv_var, b_var);
                     d = (d < -hd) ? -hd : (d > hd ? hd : d);  // apply_bounds; its new bound is not needed yet
-                    if (lane == 0) s_moves[wid] = d != 0.0 ? 1 : 0;
+                    if (lane == 0) s_delta[par][wid] = d;
                 }
                 fresh = false;
                 if (CL) ++n_xch;
                 __syncthreads();
-                const unsigned moves = __ballot_sync(kFull, s_moves[lane & (kWindow - 1)]);
+                const unsigned moves = __ballot_sync(kFull, s_delta[par][lane & (kWindow - 1)] != 0.0);
+                par ^= 1;
                 // does the step stand (a medium column's waits until it runs alone)
                 if (mine && (alone || ((s_holders[wid] & moves) == 0 && !((flags & 16) && d != 0.0)))) {
                     if (d != 0.0) {
@@ -453,11 +465,6 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                         }
                     }
                     if (wid == slot) {  // pos is the position of this column
-                        if (rank == 0 && lane == 0) {  // the bound, and the coefficient where the step moved it
-                            apply_bounds(d, hd);
-                            R.bh[pos] = make_double2(d != 0.0 ? b0 + d : b0, hd);
-                            if (d != 0.0) P.beta[r.c.j] = b0 + d;
-                        }
                         pos += kWindow;
                         fresh = true;
                     }
@@ -465,6 +472,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 __syncthreads();
             }
         }
+        __syncthreads();  // the last round's bounds and coefficients
         if (CL && s_abort) {
             failed = true;
             break;
