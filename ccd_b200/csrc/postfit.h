@@ -43,7 +43,11 @@ struct FisherParams {
     double* out;
 };
 
-// Slots t < n_slots take columns idx[p0 + t]; U (and C) must be zero on entry.
+// Whether a column's row vector (and the sums of its groups) fit in a CTA's shared
+// memory; the whole result in one launch then (U and C are not used).
+cudaError_t fisher_in_shared(const FisherParams& P, bool* fits);
+cudaError_t launch_fisher(const FisherParams& P, cudaStream_t s);
+// Otherwise, pass by pass: slots t < n_slots take columns idx[p0 + t]; U (and C) must be zero on entry.
 cudaError_t launch_fisher_scatter(const FisherParams& P, int p0, int n_slots, int64_t max_entries,
                                   cudaStream_t s);
 // Entries (p0 + t, q) and (q, p0 + t) of `out` for every q >= p0 + t.

@@ -52,17 +52,25 @@ void Fit::fisher_information(const int32_t* idx, int n, double* out) {
         P.gden = cox.denom;
         P.N = cox.N;
     }
+    bool shared = false;
+    check_cuda(fisher_in_shared(P, &shared), "fisher layout");
     const size_t u_bytes = sizeof(double) * (size_t)K * kFisherSlots;
     const size_t c_bytes = grouped ? sizeof(double) * (size_t)(cox.N + 1) * kFisherSlots : 0;
-    P.U = s.get<double>((size_t)K * kFisherSlots);
-    P.C = grouped ? s.get<double>((size_t)(cox.N + 1) * kFisherSlots) : nullptr;
+    if (!shared) {
+        P.U = s.get<double>((size_t)K * kFisherSlots);
+        P.C = grouped ? s.get<double>((size_t)(cox.N + 1) * kFisherSlots) : nullptr;
+    }
     int32_t* d_idx = s.get<int32_t>(n);
     check_cuda(cudaMemcpyAsync(d_idx, idx, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream), "fisher idx");
     P.idx = d_idx;
     P.n = n;
     P.out = s.get<double>((size_t)n * n);
     check_cuda(cudaEventRecord(ctx->fev[2], stream), "event");
-    for (int p0 = 0; p0 < n; p0 += kFisherSlots) {
+    if (shared) {
+        check_cuda(launch_fisher(P, stream), "fisher");
+        ++launches;
+    }
+    for (int p0 = 0; !shared && p0 < n; p0 += kFisherSlots) {
         const int ns = std::min(kFisherSlots, n - p0);
         int64_t most = 0;
         for (int t = 0; t < ns; ++t) most = std::max(most, m->entries(idx[p0 + t]));
