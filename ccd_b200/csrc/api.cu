@@ -1294,13 +1294,7 @@ int ccdb_get_xbeta(ccdb_fit* f, double* out) {
         require(f && out, "NULL argument");
         require_fp64(f);
         f->check_lazy();
-        const int stride = f->group_engine() ? 1 : 2;
-        const double2* src = f->group_engine() ? f->cox.xbe : f->row;
-        std::vector<double2> r(stride * f->K);
-        check_cuda(cudaMemcpyAsync(r.data(), src, sizeof(double2) * stride * f->K, cudaMemcpyDeviceToHost,
-                                   f->stream), "xbeta copy");
-        check_cuda(f->ctx->wait(), "sync");
-        for (int64_t k = 0; k < f->K; ++k) out[k] = r[stride * k].x;
+        f->copy_xbeta(out);
     });
 }
 
@@ -1355,10 +1349,14 @@ int ccdb_get_predictive_estimates(ccdb_fit* f, const double* weights, double* y)
     return guard([&] {
         require(f && y, "NULL argument");
         require_fp64(f);
+        if (!weights) {
+            f->predictive_estimates(y);
+            return;
+        }
         std::vector<double> p(f->K);
         f->predictive_estimates(p.data());
         for (int64_t k = 0; k < f->K; ++k)
-            if (!weights || weights[k] != 0.0) y[k] = p[k];
+            if (weights[k] != 0.0) y[k] = p[k];
     });
 }
 

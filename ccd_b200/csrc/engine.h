@@ -275,6 +275,8 @@ struct Fit {
     double predictive_log_likelihood(const double* weights);
     double predictive_sum(const double* weights);
     void predictive_estimates(double* out);
+    void copy_xbeta(double* out);
+    void rows_to_host(struct PredictParams P, double* out);
 };
 
 }  // namespace ccdb

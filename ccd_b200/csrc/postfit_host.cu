@@ -161,11 +161,33 @@ double Fit::predictive_sum(const double* weights) {
 // predictEstimate of every row's xBeta into out (K entries).
 void Fit::predictive_estimates(double* out) {
     check_lazy();
+    PredictParams P{};
+    P.model = model;
+    rows_to_host(P, out);
+}
+
+// xBeta of every row.
+void Fit::copy_xbeta(double* out) {
+    PredictParams P{};
+    P.model = M_CLR;  // a model whose prediction is xBeta
+    try {
+        rows_to_host(P, out);
+    } catch (const Error& e) {
+        if (e.code != CCDB_ERR_BUDGET) throw;
+        // no room for the column of results: the row words themselves
+        const int words = group_engine() ? 1 : 2;
+        std::vector<double2> r((size_t)words * K);
+        check_cuda(cudaMemcpyAsync(r.data(), group_engine() ? cox.xbe : row, sizeof(double2) * r.size(),
+                                   cudaMemcpyDeviceToHost, stream), "xbeta copy");
+        check_cuda(ctx->wait(), "xbeta sync");
+        for (int64_t k = 0; k < K; ++k) out[k] = r[words * k].x;
+    }
+}
+
+void Fit::rows_to_host(PredictParams P, double* out) {
     Scratch s(ctx);
     double* d_out = s.get<double>(K);
-    PredictParams P{};
     P.K = K;
-    P.model = model;
     P.grouped = group_engine() ? 1 : 0;
     P.row = row;
     P.xbe = group_engine() ? cox.xbe : nullptr;
