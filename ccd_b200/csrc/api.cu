@@ -117,10 +117,11 @@ void Matrix::ensure_csr(cudaStream_t s) {
     CsrDeviceArgs a{K, J, d_col_ptr, d_rows, d_val_ptr, d_vals, d_fmt};
     auto* counts = static_cast<int32_t*>(ctx->alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(K, 1)));
     auto* cursor = static_cast<int64_t*>(ctx->alloc(sizeof(int64_t) * (size_t)std::max<int64_t>(K, 1)));
+    auto* tiles = static_cast<int64_t*>(ctx->alloc(sizeof(int64_t) * (size_t)std::max<int64_t>(csr_device_tiles(K), 1)));
     auto* d_max = static_cast<int32_t*>(ctx->alloc(sizeof(int32_t)));
     d_row_ptr = static_cast<int64_t*>(ctx->alloc(sizeof(int64_t) * (size_t)(K + 1)));
     int32_t longest = 0;
-    check_cuda(csr_device_count(a, counts, d_row_ptr, cursor, d_max, s), "row counts");
+    check_cuda(csr_device_count(a, counts, tiles, d_row_ptr, cursor, d_max, s), "row counts");
     check_cuda(cudaMemcpyAsync(&longest, d_max, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "longest row");
     check_cuda(ctx->wait(), "row counts");
     if (longest <= kCsrDeviceMaxRow) {
@@ -137,6 +138,7 @@ void Matrix::ensure_csr(cudaStream_t s) {
     }
     ctx->release(counts);
     ctx->release(cursor);
+    ctx->release(tiles);
     ctx->release(d_max);
     check_cuda(ctx->wait(), "row-major copy");
 }

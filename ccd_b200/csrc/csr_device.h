@@ -21,12 +21,13 @@ struct CsrDeviceArgs {
     const uint8_t* fmt;
 };
 
-// Pass 1: per-row entry counts (`counts`, K int32, zeroed here), their
-// exclusive sum into `row_ptr` (K + 1) and `cursor` (K), and the longest row
-// into `*max_row` (device).  The caller reads max_row and, when it is at most
+// Pass 1: per-row entry counts (`counts`, K int32, zeroed here), their sums by
+// tile of rows (`tile_sum`, csr_device_tiles), their exclusive sum into `row_ptr`
+// (K + 1) and `cursor` (K), and the longest row into `*max_row` (device).  The caller reads max_row and, when it is at most
 // kCsrDeviceMaxRow, runs pass 2.
-cudaError_t csr_device_count(const CsrDeviceArgs& a, int32_t* counts, int64_t* row_ptr, int64_t* cursor,
-                             int32_t* max_row, cudaStream_t s);
+int64_t csr_device_tiles(int64_t K);
+cudaError_t csr_device_count(const CsrDeviceArgs& a, int32_t* counts, int64_t* tile_sum, int64_t* row_ptr,
+                             int64_t* cursor, int32_t* max_row, cudaStream_t s);
 // Pass 2: every entry placed in its row (`col`, `val`), then each row sorted
 // by column: per row the columns in increasing order, dense-like columns
 // (DENSE, INTERCEPT) at every row -- the layout of build_csr (csr_host.h).

@@ -23,6 +23,7 @@ struct MMParams {
     const int32_t* grp;
     const double* nEv;
     const double* denom;
+    double* share;         // K, scratch: events x offsExpXBeta / denominator of each row
     const double* xjy;
     const uint8_t* fixed;  // J flags (nullptr: none)
     // per column
@@ -32,7 +33,7 @@ struct MMParams {
     double2* gh;           // J outputs {gradient, Hessian bound}
 };
 
-// One CTA per column: the MM (gradient, Hessian bound), and with P.step the
+// The rows' shares, then one CTA per column: the MM (gradient, Hessian bound), and with P.step the
 // prior's step added to beta (no trust-region bound, as the reference's MM).
 cudaError_t launch_mm_gradient_hessian(const MMParams& P, cudaStream_t s);
 
