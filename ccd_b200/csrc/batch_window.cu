@@ -1,16 +1,16 @@
 // batch_window.cu -- many fits over one matrix in one launch (the
 // cross-validation grid: folds x prior variances), each fit on one CTA with the
-// next kWindow columns in flight.
+// next four or sixteen columns in flight.
 //
 // An instance has its own row weights (0 on its held-out fold, as
 // CrossValidationSelector::getWeights sets them, drivers/CrossValidationSelector.cpp:72-130),
 // prior variance, coefficients and bounds.  CTAs take instances from a queue,
 // weakest priors first, and never wait for one another.  The sweep is the one of
 // window.cu on one CTA: sixteen warps, in teams of one or four with a column
-// each, gather gradients against the same state, and in visiting order a step stands unless an earlier
-// column in flight that shares a row with it moves or is itself held back; four
-// helper warps copy ahead and decide what is in flight next.  The instance
-// therefore takes exactly the steps of the sequential cycle
+// each, gather gradients against the same state, and in visiting order a step
+// stands unless an earlier column in flight that shares a row with it moves or is
+// itself held back; four helper warps copy ahead and decide what is in flight
+// next.  The instance therefore takes exactly the steps of the sequential cycle
 // (CyclicCoordinateDescent.cpp:1008-1021).  After convergence it reports the
 // predictive log-likelihood of its held-out rows (ModelSpecifics.hpp:652-690).
 //
@@ -28,11 +28,11 @@
 // cycles.  What shortens it: no exp and no division in a gather; the two entries
 // that a thread of a team has stay in registers from the gather to the update;
 // xBeta, when it is in global memory, is loaded with the gather where the step is
-// going to stand; the bounds are settled by a helper.  One warp a column,
-// seven entries a lane, takes 53 ms where teams of four take 27.  Measured on a B200: 200 mixed fits of 40,000 x 1,001 in 22.8
-// ms, in lockstep groups with a cluster exchange a column 81.9; 100 FP64 fits of
-// 8,000 x 301 in 3.4 ms, one column at a time with exp and division in the gather
-// 12.1.
+// going to stand; the bounds are settled by a helper.  With one warp a column,
+// seven entries a lane, the mixed grid below takes 53 ms where teams of four took
+// 27.  Measured on a B200: 200 mixed fits of 40,000 x 1,001 in 22 ms, in lockstep
+// groups with a cluster exchange a column 82; 100 FP64 fits of 8,000 x 301 in 3.5
+// ms, one column at a time with exp and division in the gather 12.1.
 //
 // The helpers' copies go through the copy engine and are awaited with a bound; a
 // wait that runs out is reported as a timeout of the instance.
@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(kT, 1) batch_window_kernel(BatchWindowParams R
     auto staged_all = [&](unsigned& phase) {
         if (phase < 2) return true;
         const bool ok = wait_bytes(&s_bar[wid - kWindow], phase & 1);
+        if (!ok) drain(&s_bar[wid - kWindow], phase & 1);  // what is under way lands before the CTA leaves
         phase = (phase & 1) ^ 1;
         return ok;
     };
@@ -376,7 +377,7 @@ __global__ void __launch_bounds__(kT, 1) batch_window_kernel(BatchWindowParams R
                 __syncthreads();  // every helper's records
                 next_turn();
                 __syncthreads();
-                while (t.base < n_active) {
+                while (t.base < n_active && !s_failed) {
                     const bool flying = q < t.limit;
                     const unsigned slots = __ballot_sync(kFull, flying);
                     const int turn = t.base & (W - 1);
@@ -415,7 +416,6 @@ __global__ void __launch_bounds__(kT, 1) batch_window_kernel(BatchWindowParams R
                     ahead.done();
                     if (!staged_all(phase)) s_failed = 1;
                     __syncthreads();
-                    if (s_failed) break;
                 }
                 settle();
                 if (moved) {
