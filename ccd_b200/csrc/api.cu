@@ -73,6 +73,29 @@ void Context::release(void* p) {
     }
 }
 
+void Context::make_results() {
+    if (cudaHostAlloc(reinterpret_cast<void**>(&results), sizeof(double2) * kResults, cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        results = nullptr;  // fits copy their results back instead
+        return;
+    }
+    for (int i = kResults - 1; i >= 0; --i) free_results.push_back(i);
+}
+
+int Context::take_result() {
+    std::lock_guard<std::mutex> g(mu);
+    if (free_results.empty()) return -1;
+    const int slot = free_results.back();
+    free_results.pop_back();
+    return slot;
+}
+
+void Context::give_result(int slot) {
+    if (slot < 0) return;
+    std::lock_guard<std::mutex> g(mu);
+    free_results.push_back(slot);
+}
+
 cudaError_t Context::wait() {
     if (!blocking_wait) return cudaStreamSynchronize(stream);
     cudaError_t e = cudaEventRecord(ev_wait, stream);
@@ -150,6 +173,7 @@ Fit::~Fit() {
                     (void*)pvar, (void*)st, (void*)grid_bar, (void*)red, (void*)xb_tmp, (void*)w,
                     (void*)gh_parts, (void*)gh_out, (void*)d_batch_cols, (void*)d_batch_out})
         ctx->release(p);
+    ctx->give_result(result_slot);
     release_schedule();
     release_window();
     release_batch_window();
@@ -375,11 +399,15 @@ void Fit::gradient_hessian(int j, double* g, double* h) {
         return;
     }
     IndepParams P = params();
-    check_cuda(launch_indep_gh(P, j, m->entries(j), gh_parts, kGhParts, gh_out, stream), "gh");
-    launches += 2;
+    int launched = 0;
+    // into the fit's word of pinned memory, where it has one: no copy back
+    double2* const slot = ctx->result(result_slot);
+    check_cuda(launch_indep_gh(P, j, m->entries(j), gh_parts, kGhParts, slot ? slot : gh_out, &launched, stream), "gh");
+    launches += launched;
     double2 r;
-    check_cuda(cudaMemcpyAsync(&r, gh_out, sizeof(double2), cudaMemcpyDeviceToHost, stream), "gh copy");
+    if (!slot) check_cuda(cudaMemcpyAsync(&r, gh_out, sizeof(double2), cudaMemcpyDeviceToHost, stream), "gh copy");
     check_cuda(ctx->wait(), "gh sync");
+    if (slot) r = *slot;
     *g = r.x;
     *h = r.y;
 }
@@ -387,15 +415,16 @@ void Fit::gradient_hessian(int j, double* g, double* h) {
 void Fit::update_xbeta(int j, double delta) {
     check_lazy();
     beta_h[j] += delta;
-    check_cuda(cudaMemcpyAsync(beta + j, &beta_h[j], sizeof(double), cudaMemcpyHostToDevice, stream),
-               "beta j");
+    if (group_engine() || m->entries(j) == 0)  // else the update's kernel writes it
+        check_cuda(cudaMemcpyAsync(beta + j, &beta_h[j], sizeof(double), cudaMemcpyHostToDevice, stream),
+                   "beta j");
     if (group_engine()) {
         cox_update(j, delta);
         check_cuda(ctx->wait(), "update sync");
         return;
     }
     IndepParams P = params();
-    check_cuda(launch_indep_update(P, j, m->fmt[j], m->entries(j), delta, stream), "update");
+    check_cuda(launch_indep_update(P, j, m->fmt[j], m->entries(j), delta, beta_h[j], stream), "update");
     launches += m->entries(j) > 0 ? 1 : 0;
     check_cuda(ctx->wait(), "update sync");
 }
@@ -639,13 +668,13 @@ void Fit::apply_step(int j, double delta) {
         return;
     }
     IndepParams P = params();
-    check_cuda(launch_indep_update(P, j, m->fmt[j], m->entries(j), delta, stream), "update");
+    check_cuda(launch_indep_update(P, j, m->fmt[j], m->entries(j), delta, beta_h[j], stream), "update");
     launches += m->entries(j) > 0 ? 1 : 0;
 }
 
 // The host-driven speculative batches (one round trip per batch of gradients
 // and per nonzero step) run only when asked for; every default path of the
-// independent-row models is the on-device cluster sweep.
+// independent-row models is the windowed sweep.
 bool Fit::use_speculative(const ccdb_mode_args& a) const { return a.strategy == CCDB_SWEEP_SPECULATIVE; }
 
 // CTAs of the windowed sweep: as many as leave each warp about one entry per
@@ -950,6 +979,7 @@ int ccdb_context_create(int device, size_t hbm_budget_bytes, ccdb_context** out)
         check_cuda(cudaEventCreate(&c->ev_a), "event");
         check_cuda(cudaEventCreate(&c->ev_b), "event");
         for (cudaEvent_t& e : c->fev) check_cuda(cudaEventCreate(&e), "event");
+        c->make_results();
         *out = c;
     });
 }
@@ -963,6 +993,7 @@ int ccdb_context_destroy(ccdb_context* ctx) {
         cudaEventDestroy(ctx->ev_b);
         for (cudaEvent_t e : ctx->fev) cudaEventDestroy(e);
         if (ctx->ev_wait) cudaEventDestroy(ctx->ev_wait);
+        if (ctx->results) cudaFreeHost(ctx->results);
         cudaStreamDestroy(ctx->stream);
         if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
         delete ctx;
@@ -1189,6 +1220,7 @@ int ccdb_fit_create(ccdb_context* ctx, const ccdb_matrix* m, const ccdb_fit_desc
         f->w = static_cast<double*>(ctx->alloc(sizeof(double) * K));
         f->gh_parts = static_cast<double2*>(ctx->alloc(sizeof(double2) * Fit::kGhParts));
         f->gh_out = static_cast<double2*>(ctx->alloc(sizeof(double2)));
+        f->result_slot = ctx->take_result();
         // CyclicCoordinateDescent::init (.cpp:200-239)
         f->beta_h.assign(J, 0.0);
         f->fixed.assign(J, 0);

@@ -56,6 +56,15 @@ struct Context {
     bool blocking_wait = false;
     cudaEvent_t ev_wait = nullptr;
 
+    // pinned words that kernels write a fit's per-call results to; a fit holds one
+    static constexpr int kResults = 1024;
+    double2* results = nullptr;
+    std::vector<int> free_results;
+    void make_results();
+    int take_result();  // -1: none left
+    void give_result(int slot);
+    double2* result(int slot) const { return slot < 0 ? nullptr : results + slot; }
+
     void* alloc(size_t bytes);
     void release(void* p);
     // wait for everything queued on the context's stream
@@ -189,6 +198,7 @@ struct Fit {
     double* w = nullptr;
     double2* gh_parts = nullptr;
     double2* gh_out = nullptr;
+    int result_slot = -1;
     int64_t launches = 0;                        // engine kernels launched so far
     double last_call_seconds = 0.0;              // device time of the last fisher_information passes
     int last_iterations = 0;                     // getIterationCount: the last findMode's cycles

@@ -654,6 +654,9 @@ __global__ void __launch_bounds__(kThreads, 1) indep_sweep_kernel(IndepParams P)
 
 // ---------------------------------------------------------------- per-coordinate kernels
 
+// One block takes the whole of a column up to 8,192 entries and finishes it: a call
+// is a launch, a wait and no more, so a second kernel for the last sum cost it a
+// fifth.
 template <int MODEL>
 __global__ void __launch_bounds__(256) gh_column_kernel(IndepParams P, int j, int64_t entries,
                                                         int64_t per_block, double2* out) {
@@ -663,7 +666,9 @@ __global__ void __launch_bounds__(256) gh_column_kernel(IndepParams P, int j, in
     double g = 0.0, h = 0.0;
     if (p0 < p1) gh_dispatch<MODEL>(P, j, P.fmt[j], p0, p1, threadIdx.x, blockDim.x, g, h);
     const double2 s = block_sum2<8>(make_double2(g, h), s_red2);
-    if (threadIdx.x == 0) out[blockIdx.x] = s;
+    if (threadIdx.x != 0) return;
+    if (gridDim.x > 1) out[blockIdx.x] = s;
+    else *out = entries > 0 ? make_double2(s.x - P.xjy[j], s.y) : make_double2(0.0, 0.0);
 }
 
 // (g, h) of a list of columns, one CTA per column (speculative batches).
@@ -699,7 +704,8 @@ __global__ void gh_finish_kernel(const double2* parts, int n, const double* xjy,
 
 // Each thread handles entries p = tid, tid + nthr, ... of column j.
 template <int FMT>
-__global__ void update_column_grid(IndepParams P, int j, int64_t entries, double delta) {
+__global__ void update_column_grid(IndepParams P, int j, int64_t entries, double delta, double beta) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) P.beta[j] = beta;
     const int64_t cb = P.col_ptr[j], vb = P.val_ptr[j];
     const int64_t nthr = (int64_t)gridDim.x * blockDim.x;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < entries; p += nthr) {
@@ -823,7 +829,7 @@ cudaError_t launch_indep_sweep(const IndepParams& P, int n_cta, cudaStream_t str
 }
 
 cudaError_t launch_indep_gh(const IndepParams& P, int j, int64_t entries, double2* parts,
-                            int max_parts, double2* out, cudaStream_t stream) {
+                            int max_parts, double2* out, int* launched, cudaStream_t stream) {
     int64_t per_block = 8192;
     int nb = (int)((entries + per_block - 1) / per_block);
     if (nb < 1) nb = 1;
@@ -831,11 +837,16 @@ cudaError_t launch_indep_gh(const IndepParams& P, int j, int64_t entries, double
         nb = max_parts;
         per_block = (entries + nb - 1) / nb;
     }
+    double2* const to = nb > 1 ? parts : out;
     if (P.model == M_LOGISTIC)
-        gh_column_kernel<M_LOGISTIC><<<nb, 256, 0, stream>>>(P, j, entries, per_block, parts);
+        gh_column_kernel<M_LOGISTIC><<<nb, 256, 0, stream>>>(P, j, entries, per_block, to);
     else
-        gh_column_kernel<M_POISSON><<<nb, 256, 0, stream>>>(P, j, entries, per_block, parts);
-    gh_finish_kernel<<<1, 32, 0, stream>>>(parts, nb, P.xjy, j, entries, out);
+        gh_column_kernel<M_POISSON><<<nb, 256, 0, stream>>>(P, j, entries, per_block, to);
+    *launched = 1;
+    if (nb > 1) {
+        gh_finish_kernel<<<1, 32, 0, stream>>>(parts, nb, P.xjy, j, entries, out);
+        *launched = 2;
+    }
     return cudaGetLastError();
 }
 
@@ -848,15 +859,15 @@ cudaError_t launch_indep_gh_batch(const IndepParams& P, const int32_t* cols, int
 }
 
 cudaError_t launch_indep_update(const IndepParams& P, int j, uint8_t fmt, int64_t entries,
-                                double delta, cudaStream_t stream) {
+                                double delta, double beta, cudaStream_t stream) {
     if (entries <= 0) return cudaSuccess;
     int nb = (int)((entries + 255) / 256);
     if (nb > 4096) nb = 4096;
     switch (fmt) {
-    case F_INDICATOR: update_column_grid<F_INDICATOR><<<nb, 256, 0, stream>>>(P, j, entries, delta); break;
-    case F_SPARSE: update_column_grid<F_SPARSE><<<nb, 256, 0, stream>>>(P, j, entries, delta); break;
-    case F_DENSE: update_column_grid<F_DENSE><<<nb, 256, 0, stream>>>(P, j, entries, delta); break;
-    default: update_column_grid<F_INTERCEPT><<<nb, 256, 0, stream>>>(P, j, entries, delta); break;
+    case F_INDICATOR: update_column_grid<F_INDICATOR><<<nb, 256, 0, stream>>>(P, j, entries, delta, beta); break;
+    case F_SPARSE: update_column_grid<F_SPARSE><<<nb, 256, 0, stream>>>(P, j, entries, delta, beta); break;
+    case F_DENSE: update_column_grid<F_DENSE><<<nb, 256, 0, stream>>>(P, j, entries, delta, beta); break;
+    default: update_column_grid<F_INTERCEPT><<<nb, 256, 0, stream>>>(P, j, entries, delta, beta); break;
     }
     return cudaGetLastError();
 }

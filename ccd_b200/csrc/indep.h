@@ -58,11 +58,13 @@ int indep_max_split();
 cudaError_t indep_sweep_occupancy(int model, int* blocks_per_sm);
 cudaError_t launch_indep_sweep(const IndepParams& P, int n_cta, cudaStream_t stream);
 cudaError_t launch_indep_gh(const IndepParams& P, int j, int64_t entries, double2* parts,
-                            int max_parts, double2* out, cudaStream_t stream);
+                            int max_parts, double2* out, int* launched, cudaStream_t stream);
 cudaError_t launch_indep_gh_batch(const IndepParams& P, const int32_t* cols, int ncols, double2* out,
                                   cudaStream_t stream);
+// xBeta += delta x_j and what follows from it; `beta` into P.beta[j] (nothing for
+// a column without entries)
 cudaError_t launch_indep_update(const IndepParams& P, int j, uint8_t fmt, int64_t entries,
-                                double delta, cudaStream_t stream);
+                                double delta, double beta, cudaStream_t stream);
 cudaError_t launch_remaining_stats(double2* row, const double* xb, const double* w, int64_t K,
                                    double null_denom, cudaStream_t stream);
 // one pass of the objective reduction into P.red[0 .. n_blocks) (buffer 0)
