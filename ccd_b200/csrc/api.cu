@@ -74,7 +74,7 @@ void Context::release(void* p) {
 }
 
 void Context::make_results() {
-    if (cudaHostAlloc(reinterpret_cast<void**>(&results), sizeof(double2) * kResults, cudaHostAllocMapped) != cudaSuccess) {
+    if (cudaHostAlloc(reinterpret_cast<void**>(&results), 2 * sizeof(double2) * kResults, cudaHostAllocMapped) != cudaSuccess) {
         cudaGetLastError();
         results = nullptr;  // fits copy their results back instead
         return;

@@ -317,15 +317,19 @@ void Fit::cox_objective_terms(double* out4) {
 }
 
 void Fit::cox_gh_batch(const int32_t* cols, int n, double2* out) {
-    check_cuda(cudaMemcpyAsync(cox.batch_cols, cols, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream),
-               "batch cols");
+    // one column: its index and its result in the fit's pinned words, no copies
+    double2* const slot = n == 1 ? ctx->result(result_slot) : nullptr;
+    int32_t* const which = slot ? reinterpret_cast<int32_t*>(slot + 1) : cox.batch_cols;
+    if (slot) *which = cols[0];
+    else check_cuda(cudaMemcpyAsync(which, cols, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream), "batch cols");
+    double2* const to = slot ? slot : cox.batch_out;
     CoxParams P = cox_params();
-    if (is_cox()) check_cuda(launch_cox_gh(P, cox.batch_cols, n, cox.batch_out, stream), "cox gh");
-    else check_cuda(launch_grouped_gh(P, cox.batch_cols, n, cox.batch_out, stream), "grouped gh");
+    if (is_cox()) check_cuda(launch_cox_gh(P, which, n, to, stream), "cox gh");
+    else check_cuda(launch_grouped_gh(P, which, n, to, stream), "grouped gh");
     ++launches;
-    check_cuda(cudaMemcpyAsync(out, cox.batch_out, sizeof(double2) * n, cudaMemcpyDeviceToHost, stream),
-               "gh copy");
+    if (!slot) check_cuda(cudaMemcpyAsync(out, to, sizeof(double2) * n, cudaMemcpyDeviceToHost, stream), "gh copy");
     check_cuda(ctx->wait(), "gh sync");
+    if (slot) *out = *slot;
 }
 
 void Fit::cox_update(int j, double delta) {

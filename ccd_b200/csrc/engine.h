@@ -56,14 +56,15 @@ struct Context {
     bool blocking_wait = false;
     cudaEvent_t ev_wait = nullptr;
 
-    // pinned words that kernels write a fit's per-call results to; a fit holds one
+    // pinned words that kernels write a fit's per-call results to, with room behind
+    // each for the call's column; a fit holds one
     static constexpr int kResults = 1024;
     double2* results = nullptr;
     std::vector<int> free_results;
     void make_results();
     int take_result();  // -1: none left
     void give_result(int slot);
-    double2* result(int slot) const { return slot < 0 ? nullptr : results + slot; }
+    double2* result(int slot) const { return slot < 0 ? nullptr : results + 2 * slot; }
 
     void* alloc(size_t bytes);
     void release(void* p);

@@ -4,8 +4,8 @@ context's pinned result words; an update's coefficient reaches the device."""
 import numpy as np
 import pytest
 
-from ccd_b200 import native
-from ccd_b200.data import MODEL_LOGISTIC, MODEL_POISSON, PRIOR_NORMAL
+from ccd_b200 import native, synthetic
+from ccd_b200.data import MODEL_CONDITIONAL_LOGISTIC, MODEL_COX, MODEL_LOGISTIC, MODEL_POISSON, PRIOR_NORMAL
 from oracle import checker
 
 from .test_gpu_window import problem
@@ -38,18 +38,21 @@ def test_gradients_at_the_block_limit(gpu_ctx, model):
     agree([f.get_log_likelihood()], [e.loglik()])
 
 
-def test_more_fits_than_result_words():
+@pytest.mark.parametrize("model", [MODEL_LOGISTIC, MODEL_CONDITIONAL_LOGISTIC, MODEL_COX])
+def test_more_fits_than_result_words(model):
     ctx = native.Context(0)
-    d = problem(MODEL_LOGISTIC, 200, [20, 30], seed=5)
+    d = synthetic.small(model, seed=5, K=200, P=4)
     m = native.Matrix(ctx, d)
     fits = [native.Fit(ctx, m, d) for _ in range(1026)]
-    want = fits[0].compute_gradient_and_hessian(1)
-    for f in (fits[1023], fits[1024], fits[1025]):
-        assert f.compute_gradient_and_hessian(1) == want
+    for j in range(d.J):
+        want = fits[0].compute_gradient_and_hessian(j)
+        agree(want, checker.RestatementEngine(d).grad_hess(j))
+        for f in (fits[1023], fits[1024], fits[1025]):  # the last word and none
+            assert f.compute_gradient_and_hessian(j) == want
     for f in fits:
         f.close()
     again = native.Fit(ctx, m, d)
-    assert again.compute_gradient_and_hessian(1) == want
+    agree(again.compute_gradient_and_hessian(1), checker.RestatementEngine(d).grad_hess(1))
     again.close()
     m.close()
     ctx.close()
