@@ -137,7 +137,7 @@ void Matrix::ensure_csr(cudaStream_t s) {
     if (d_row_ptr) return;
     int64_t total = 0;
     for (int j = 0; j < J; ++j) total += entries(j);
-    CsrDeviceArgs a{K, J, d_col_ptr, d_rows, d_val_ptr, d_vals, d_fmt};
+    CsrDeviceArgs a{K, J, d_col_ptr, d_rows, d_val_ptr, d_vals, d_fmt, val_start.back() > 0};
     auto* counts = static_cast<int32_t*>(ctx->alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(K, 1)));
     auto* cursor = static_cast<int64_t*>(ctx->alloc(sizeof(int64_t) * (size_t)std::max<int64_t>(K, 1)));
     auto* tiles = static_cast<int64_t*>(ctx->alloc(sizeof(int64_t) * (size_t)std::max<int64_t>(csr_device_tiles(K), 1)));
@@ -277,7 +277,7 @@ void Fit::compute_xbeta() {
         ++launches;
     } else {
         const_cast<Matrix*>(m)->ensure_csr(stream);
-        check_cuda(launch_xbeta_csr(m->d_row_ptr, m->d_csr_col, m->d_csr_val, beta, K, xb_tmp, stream),
+        check_cuda(launch_xbeta_csr(m->d_row_ptr, m->d_csr_col, m->csr_values(), beta, K, xb_tmp, stream),
                    "xbeta");
         ++launches;
     }

@@ -108,10 +108,12 @@ __global__ void __launch_bounds__(kT) cox_update_kernel(CoxParams P, int j, doub
 
 // computeRemainingStatisticsImpl, Cox branch (ModelSpecifics.hpp:1594-1603):
 // e = exp(xBeta) per row; denom[g] = 0 + sum of w*e over the group's rows in row order.
-__global__ void cox_exp_kernel(CoxParams P) {
+// xBeta from a fresh product, where there is one (a strided device copy of 130,000
+// words of eight bytes into xbe took some 25 us a cycle).
+__global__ void cox_exp_kernel(CoxParams P, const double* fresh) {
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < P.K;
          k += (int64_t)gridDim.x * blockDim.x) {
-        const double xb = P.xbe[k].x;
+        const double xb = fresh ? fresh[k] : P.xbe[k].x;
         P.xbe[k] = make_double2(xb, row_exp(xb, P.mixed));
     }
 }
@@ -464,8 +466,8 @@ cudaError_t launch_cox_update(const CoxParams& P, int j, double delta, cudaStrea
     return cudaGetLastError();
 }
 
-cudaError_t launch_cox_remaining(const CoxParams& P, cudaStream_t s) {
-    cox_exp_kernel<<<1184, 256, 0, s>>>(P);
+cudaError_t launch_cox_remaining(const CoxParams& P, const double* fresh, cudaStream_t s) {
+    cox_exp_kernel<<<1184, 256, 0, s>>>(P, fresh);
     cox_denom_kernel<<<1184, 256, 0, s>>>(P);
     return cudaGetLastError();
 }
@@ -496,8 +498,8 @@ cudaError_t launch_grouped_update(const CoxParams& P, int j, double delta, cudaS
     return cudaGetLastError();
 }
 
-cudaError_t launch_grouped_remaining(const CoxParams& P, cudaStream_t s) {
-    cox_exp_kernel<<<1184, 256, 0, s>>>(P);
+cudaError_t launch_grouped_remaining(const CoxParams& P, const double* fresh, cudaStream_t s) {
+    cox_exp_kernel<<<1184, 256, 0, s>>>(P, fresh);
     grouped_denom_kernel<<<1184, 256, 0, s>>>(P);
     return cudaGetLastError();
 }

@@ -281,15 +281,11 @@ void Fit::cox_scans() {
 
 // computeRemainingStatistics (ModelSpecifics.hpp:1588-1617) + the accumulated scans.
 void Fit::cox_remaining() {
-    if (xb_pending) {  // xBeta computed into xb_tmp: place it into {xBeta, e}
-        check_cuda(cudaMemcpy2DAsync(cox.xbe, sizeof(double2), xb_tmp, sizeof(double), sizeof(double), K,
-                                     cudaMemcpyDeviceToDevice, stream),
-                   "xb place");
-        xb_pending = false;
-    }
+    const double* const fresh = xb_pending ? xb_tmp : nullptr;  // xBeta computed into xb_tmp
+    xb_pending = false;
     CoxParams P = cox_params();
-    if (is_cox()) check_cuda(launch_cox_remaining(P, stream), "cox remaining");
-    else check_cuda(launch_grouped_remaining(P, stream), "grouped remaining");
+    if (is_cox()) check_cuda(launch_cox_remaining(P, fresh, stream), "cox remaining");
+    else check_cuda(launch_grouped_remaining(P, fresh, stream), "grouped remaining");
     launches += 2;
     cox_scans();
     suff_known = true;

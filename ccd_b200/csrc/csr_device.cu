@@ -138,21 +138,24 @@ __global__ void __launch_bounds__(kCT) csr_place_kernel(CsrDeviceArgs a, int64_t
 
 // One thread per row: insertion sort of the row's (column, value) pairs by
 // column (columns are distinct within a row).
+// Without values every one is 1, and only the columns move (2.6 million entries: 54
+// us, 112 with the values).
+template <bool VALUES>
 __global__ void __launch_bounds__(kCT) csr_sort_kernel(const int64_t* row_ptr, int64_t K, int32_t* col,
                                                         double* val) {
     for (int64_t k = (int64_t)blockIdx.x * kCT + threadIdx.x; k < K; k += (int64_t)gridDim.x * kCT) {
         const int64_t lo = row_ptr[k], hi = row_ptr[k + 1];
         for (int64_t i = lo + 1; i < hi; ++i) {
             const int32_t cj = col[i];
-            const double vj = val[i];
+            const double vj = VALUES ? val[i] : 1.0;
             int64_t q = i - 1;
             while (q >= lo && col[q] > cj) {
                 col[q + 1] = col[q];
-                val[q + 1] = val[q];
+                if (VALUES) val[q + 1] = val[q];
                 --q;
             }
             col[q + 1] = cj;
-            val[q + 1] = vj;
+            if (VALUES) val[q + 1] = vj;
         }
     }
 }
@@ -179,8 +182,9 @@ cudaError_t csr_device_fill(const CsrDeviceArgs& a, const int64_t* row_ptr, int6
                             double* val, cudaStream_t s) {
     csr_place_kernel<<<col_grid(a.J), kCT, 0, s>>>(a, cursor, col, val);
     const int64_t blocks = (a.K + kCT - 1) / kCT;
-    csr_sort_kernel<<<(unsigned)(blocks < 4096 ? (blocks > 0 ? blocks : 1) : 4096), kCT, 0, s>>>(row_ptr, a.K, col,
-                                                                                                  val);
+    const unsigned grid = (unsigned)(blocks < 4096 ? (blocks > 0 ? blocks : 1) : 4096);
+    if (a.has_values) csr_sort_kernel<true><<<grid, kCT, 0, s>>>(row_ptr, a.K, col, val);
+    else csr_sort_kernel<false><<<grid, kCT, 0, s>>>(row_ptr, a.K, col, val);
     return cudaGetLastError();
 }
 

@@ -19,6 +19,7 @@ struct CsrDeviceArgs {
     const int64_t* val_ptr;  // J + 1 value offsets (sparse, dense columns)
     const double* vals;
     const uint8_t* fmt;
+    bool has_values;         // some column has values of its own
 };
 
 // Pass 1: per-row entry counts (`counts`, K int32, zeroed here), their sums by

@@ -93,6 +93,8 @@ struct Matrix {
     double* d_csr_val = nullptr;
 
     int64_t entries(int j) const;
+    // values of the row-major copy; NULL where every one is 1
+    const double* csr_values() const { return val_start.back() > 0 ? d_csr_val : nullptr; }
     int64_t mean_entries() const;  // of the columns but the longest
     void ensure_csr(cudaStream_t s);
     ~Matrix();

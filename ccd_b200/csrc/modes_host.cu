@@ -78,7 +78,7 @@ void Fit::compute_xbeta_transpose() {
         any_dense |= m->fmt[j] == F_DENSE;
     }
     const_cast<Matrix*>(m)->ensure_csr(stream);
-    check_cuda(launch_xbeta_csr(m->d_row_ptr, m->d_csr_col, m->d_csr_val, beta, K, xb_tmp, stream,
+    check_cuda(launch_xbeta_csr(m->d_row_ptr, m->d_csr_col, m->csr_values(), beta, K, xb_tmp, stream,
                                 any_indicator && !any_dense),
                "xbeta (transpose)");
     ++launches;
