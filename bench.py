@@ -1470,7 +1470,7 @@ def run_variant(args, world, rank, local):
             ach = b * args.steps / dev_t / 1e9
             roofline = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                         "peak_source": peak_kind, "algorithmic_bytes_per_launch": b / (2 * ((len(cols) + 7) // 8)),
-                        "kernel": "fisher_scatter + fisher_gather passes (one call)", "traffic": None}
+                        "kernel": "fisher_dense_kernel (one launch a call)", "traffic": None}
         elif name == "mm_clr":
             b = mm_cycle_bytes(d) * cycles
             ach = b / dev_t / 1e9
