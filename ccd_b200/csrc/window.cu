@@ -47,8 +47,9 @@
 // the CTAs' pairs added four at a time in every lane, bounds settled by the warps
 // with columns and the gather unrolled, these took 4.5, 53 and 154 ms.
 //
-// The wait for the other CTAs' pairs is bounded (kWaitNs): a wait that runs out
-// records an error and the CTA leaves through the closing cluster barrier.
+// The wait for the other CTAs' pairs is bounded (kWaitNs).  A CTA whose wait runs out
+// steps and sends no more; at the end of the cycle the CTAs learn of it from one
+// another and all leave, each once what was sent to it has landed (sweep_exit.h).
 #include <algorithm>
 #include <cstdint>
 
@@ -146,7 +147,10 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
     __shared__ double2 s_pair[2][kWindow][kWindowCluster];  // (g, h) by round parity, column and CTA
     __shared__ double s_red[kWindow][2];
     __shared__ double4 s_red4[kWarps];
-    __shared__ double4 s_obj[kWindowCluster];
+    // by cycle parity and CTA: a CTA that gave up may be a cycle ahead of one that reads them
+    __shared__ double4 s_obj[CL ? 2 : 1][kWindowCluster];
+    __shared__ CycleReport s_report[CL ? 2 : 1][kWindowCluster];
+    __shared__ unsigned s_sent[2];  // bytes to each CTA, by exchange parity
     __shared__ double s_delta[2][kWindow];  // by round parity: the column's step
     __shared__ unsigned s_holders[kWindow];  // the slots that hold the column back if they move
     __shared__ Turn s_turn;
@@ -231,8 +235,9 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
     };
 
     // ---- the objective terms {LL numerator, LL denominator, gradient objective,
-    // log prior} (ModelSpecifics.hpp:103-120, 605-650; JointPrior.h:121-128)
-    auto objective = [&](double& ll, double& lp) {
+    // log prior} (ModelSpecifics.hpp:103-120, 605-650; JointPrior.h:121-128); false
+    // when a CTA gave up in this cycle
+    auto objective = [&](int cycle, bool gave_up, double& obj, double& ll, double& lp) {
         double4 acc = make_double4(0.0, 0.0, 0.0, 0.0);
 #pragma unroll 1
         for (int k = tid; k < n_rows; k += kT) {
@@ -248,23 +253,29 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
         acc = block_sum4<kWarps>(acc, s_red4);
         if (CL) {
             if (tid < C) {
-                const unsigned a = peer_u32(&s_obj[rank], tid);
+                const unsigned a = peer_u32(&s_obj[cycle & 1][rank], tid);
                 asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(acc.x), "d"(acc.y) : "memory");
                 asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a + 16), "d"(acc.z), "d"(acc.w) : "memory");
+                tell(&s_report[cycle & 1][rank], tid, CycleReport{gave_up ? 1u : 0u, n_xch, {s_sent[0], s_sent[1]}});
             }
             cluster_barrier();  // also: rank 0's coefficients and bounds are seen by the next cycle
             acc = make_double4(0.0, 0.0, 0.0, 0.0);
+            unsigned any = 0;
 #pragma unroll 1
             for (int c = 0; c < C; ++c) {
-                acc.x += s_obj[c].x;
-                acc.y += s_obj[c].y;
-                acc.z += s_obj[c].z;
-                acc.w += s_obj[c].w;
+                const double4 o = s_obj[cycle & 1][c];
+                acc.x += o.x;
+                acc.y += o.y;
+                acc.z += o.z;
+                acc.w += o.w;
+                any |= s_report[cycle & 1][c].gave_up;
             }
+            if (any) return false;
         }
         ll = (acc.x - acc.y) + P.ll_fixed;
         lp = acc.w;
-        return (P.conv == C_GRADIENT) ? acc.z : (P.conv == C_MITTAL ? ll : ll + lp);
+        obj = (P.conv == C_GRADIENT) ? acc.z : (P.conv == C_MITTAL ? ll : ll + lp);
+        return true;
     };
 
     // ---- what the helpers copy ahead: records two columns ahead of a warp, entries one
@@ -275,12 +286,18 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
 
     double last = 0.0;
     unsigned long long moved = 0;
-    bool failed = false;
+    bool gave_up = false;  // a wait of this CTA ran out
 
     for (int iteration = 0;; ++iteration) {
         // ---- a cycle is complete: convergence (findMode, CyclicCoordinateDescent.cpp:1023-1056)
-        double ll, lp;
-        const double cur = objective(ll, lp);
+        double cur, ll, lp;
+        if (!objective(iteration, gave_up, cur, ll, lp)) {  // every CTA leaves
+            if (gave_up && tid == 0) {
+                if (atomicCAS(&P.st->error, 0, E_WAIT_CLUSTER) == 0) P.st->error_where = rank;
+                land_all(s_bar, s_report[iteration & 1], C, rank);
+            }
+            return;
+        }
         if (iteration > 0) {
             const bool ill = cur != cur;
             const double conv = ill ? 0.0 : fabs(cur - last) / (fabs(cur) + 1.0);
@@ -347,7 +364,10 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 const unsigned slots = __ballot_sync(kFull, flying);
                 const int turn = t.base & (kWindow - 1);
                 if (me == 0) {
-                    if (CL && lane == 0) expect_pairs(__popc(slots));
+                    if (CL && lane == 0) {
+                        expect_pairs(__popc(slots));
+                        s_sent[n_xch & 1] = (unsigned)(__popc(slots) * 2 * sizeof(double));
+                    }
                     // the earlier columns in flight that hold a column back if they move: those
                     // it shares a row with, and those that may hold one of these back
                     unsigned holders = 0;
@@ -473,20 +493,9 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
             }
         }
         __syncthreads();  // the last round's bounds and coefficients
-        if (CL && s_abort) {
-            failed = true;
-            break;
-        }
+        gave_up = CL && s_abort;
     }
-    if (CL) {
-        if (failed && tid == 0 && atomicCAS(&P.st->error, 0, E_WAIT_CLUSTER) == 0) P.st->error_where = rank;
-        cluster_barrier();  // no CTA leaves while another may still send to it
-        if (failed) {  // pairs already sent to this CTA land before it leaves
-            const unsigned m = n_xch - 1;  // the exchange that gave up
-            drain(&s_bar[m & 1], (m >> 1) & 1);
-            return;
-        }
-    }
+    if (CL) cluster_barrier();  // no CTA leaves while another may still send to it
     // the state back to where the other calls read it
     if (rows.kPair)
 #pragma unroll 1

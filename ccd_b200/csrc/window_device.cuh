@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "common.cuh"
+#include "sweep_exit.h"
 #include "window_sweep.h"
 
 namespace ccdb {
@@ -109,6 +110,26 @@ __device__ __forceinline__ void bulk_copy(void* to, const void* from, unsigned b
 __device__ __forceinline__ void drain(const uint64_t* bar, unsigned parity) {
     const unsigned long long t0 = global_ns();
     while (!arrived(bar, parity) && global_ns() - t0 < 1000000000ull) __nanosleep(200);
+}
+// `bytes` that were announced to this CTA's `bar` and that nobody sends.
+__device__ __forceinline__ void forgo_bytes(const uint64_t* bar, unsigned bytes) {
+    asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// A CTA's report of the cycle into `to` (by CTA) of CTA `peer`.
+__device__ __forceinline__ void tell(const CycleReport* to, int peer, const CycleReport& r) {
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(peer_u32(to, peer)), "r"(r.gave_up), "r"(r.sent),
+                 "r"(r.bytes[0]), "r"(r.bytes[1])
+                 : "memory");
+}
+// One thread of a CTA that gave up, once all reports are here: every byte that was
+// sent to this CTA has landed (sweep_exit.h).
+__device__ __forceinline__ void land_all(const uint64_t* bars, const CycleReport* all, int C, int me) {
+    const OnTheWay w = on_the_way(all, C, me);
+    const unsigned e = all[me].sent - 1, n = e + 1;  // the last announced exchange, and the one after it
+    if (w.missing) forgo_bytes(&bars[e & 1], w.missing);
+    if (w.ahead) expect_bytes(&bars[n & 1], w.ahead);
+    drain(&bars[e & 1], (e >> 1) & 1);
+    if (w.ahead) drain(&bars[n & 1], (n >> 1) & 1);
 }
 
 // Copies made ahead of use by eight lanes (l8) of a helper.
