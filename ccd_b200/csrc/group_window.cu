@@ -48,8 +48,12 @@
 // global memory and the rebuild over every group that it replaces took 27, 38, 60
 // and 11 us.
 //
-// The waits of both forms are bounded; one that runs out records an error and
-// every CTA leaves.
+// The waits of both forms are bounded.  In the grid form one that runs out raises
+// the launch's abort word and every CTA leaves at its next wait.  In a cluster the
+// CTA steps and sends no more, and all leave together at the end of the cycle, each
+// once what was sent to it has landed (sweep_exit.h).  Within a CTA the warps pass
+// the same barriers: a wait marks the half of the round that it lies in, and every
+// warp reads the mark in the other half.
 #include <algorithm>
 #include <cstdint>
 
@@ -183,10 +187,14 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     __shared__ Rec s_rec[4][kWindow];  // by position: (position / kWindow) & 3, slot
     // cluster form, by exchange parity, column and CTA: Cox {G, HQ}, {B, T}, {H2, 0}, else {g, h}
     __shared__ double2 s_part[CL ? 2 : 1][CL ? kWindow : 1][COX ? 3 : 1][CL ? kWindowCluster : 1];
-    __shared__ double s_tail[CL ? 2 : 1][kWindowCluster];
-    __shared__ double2 s_head[CL ? 2 : 1][kWindowCluster];
+    constexpr int kSumBuffers = CL && COX ? 2 : 1, kSumCtas = CL && COX ? kWindowCluster : 1;
+    __shared__ double s_tail[kSumBuffers][kSumCtas];
+    __shared__ double2 s_head[kSumBuffers][kSumCtas];
     __shared__ double4 s_red4[kWarps];
-    __shared__ double4 s_obj[kWindowCluster];
+    // by cycle parity and CTA: a CTA that gave up may be a cycle ahead of one that reads them
+    __shared__ double4 s_obj[CL ? 2 : 1][kWindowCluster];
+    __shared__ CycleReport s_report[CL ? 2 : 1][kWindowCluster];
+    __shared__ unsigned s_sent[2];  // bytes to each CTA, by exchange parity
     __shared__ double s_dd[kWorkers];    // an update's changes of exp, by entry
     __shared__ int32_t s_dg[kWorkers];   // and their groups
     __shared__ double s_run[kWindow];    // the worker warps' prefix sums
@@ -195,7 +203,9 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     __shared__ double s_delta[kWindow];  // the steps of the columns in flight
     __shared__ Turn s_turn;
     __shared__ uint64_t s_bar[2];
-    __shared__ int s_abort;
+    // a wait ran out: of the gradients, before the round's first barrier, read behind it;
+    // of an update, before the second, read behind that
+    __shared__ int s_quit, s_quit_update;
     __shared__ int32_t s_fail;
     __shared__ uint8_t s_flags[kGroupWindowCtas];  // GroupCut::flags of every CTA
     extern __shared__ __align__(16) unsigned char s_dyn[];
@@ -262,13 +272,13 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     }
     for (int c = tid; c < C; c += kT) s_flags[c] = (uint8_t)Q.cuts[c].flags;
     if (tid == 0) {
-        s_abort = 0;
+        s_quit = s_quit_update = 0;
         if (CL) init_bars(s_bar, 2);
     }
     // sums of CTAs that there are not stay zero
-    if (CL && tid < 2 * kWindowCluster) {
-        s_tail[tid / kWindowCluster][tid % kWindowCluster] = 0.0;
-        s_head[tid / kWindowCluster][tid % kWindowCluster] = make_double2(0.0, 0.0);
+    if (CL && COX && tid < 2 * kWindowCluster) {
+        (&s_tail[0][0])[tid] = 0.0;
+        (&s_head[0][0])[tid] = make_double2(0.0, 0.0);
     }
     for (int i = tid; CL && i < (int)(sizeof(s_part) / sizeof(double2)); i += kT)
         (&s_part[0][0][0][0])[i] = make_double2(0.0, 0.0);
@@ -281,8 +291,8 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     // cluster form: the base of each peer's shared variables, lane l for CTA l
     unsigned to_part = 0, to_bar = 0, to_tail = 0, to_head = 0;
     if (CL && lane < C) {
-        to_tail = peer_u32(&s_tail[0][rank], lane);
-        to_head = peer_u32(&s_head[0][rank], lane);
+        to_tail = peer_u32(&s_tail[0][COX ? rank : 0], lane);
+        to_head = peer_u32(&s_head[0][COX ? rank : 0], lane);
         to_part = peer_u32(&s_part[0][0][0][0], lane);
         to_bar = peer_u32(&s_bar[0], lane);
     }
@@ -290,24 +300,31 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     // bytes that a column's partial sums of one CTA take in an exchange
     auto pair_bytes = [&](int pos, const Rec& r) { return COX ? ((r.c.flags & 4) ? 32u : 48u) : 16u; };
     // workers, grid form: everything written before is seen by every CTA after it
-    auto grid_wait = [&]() {
+    auto grid_wait = [&](int& quit) {
         workers_barrier();
         if (tid == 0) {
             ++epoch;
             red_release_gpu_add(Q.grid_bar, 1u);
-            if (!wait_geq(Q.grid_bar, epoch * (unsigned)C, Q.wait_limit_ns, Q.st, E_WAIT_GRID, -1)) s_abort = 1;
+            if (!wait_geq(Q.grid_bar, epoch * (unsigned)C, Q.wait_limit_ns, Q.st, E_WAIT_GRID, -1)) quit = 1;
         }
         workers_barrier();
     };
-    // this exchange's bytes have come (cluster form)
-    auto wait_sums = [&]() {
-        if (!wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1)) s_abort = 1;
+    // this exchange's bytes have come, all of them to the whole warp (cluster form)
+    auto wait_sums = [&](int& quit) {
+        const bool ok = __all_sync(kFull, wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1));
+        if (!ok) quit = 1;
+        return ok;
+    };
+    // announce an exchange in which every CTA sends `bytes` to every other (cluster form)
+    auto expect_sums = [&](unsigned bytes) {
+        expect_bytes(&s_bar[n_xch & 1], bytes * (unsigned)C);
+        s_sent[n_xch & 1] = bytes;
     };
 
     // ---- the objective terms {LL numerator, LL denominator, gradient objective,
     // log prior} (ModelSpecifics.hpp:103-120, 605-650; JointPrior.h:121-128); false
-    // when a wait ran out
-    auto objective = [&](double& obj, double& ll, double& lp) {
+    // when a wait ran out, of any CTA of a cluster
+    auto objective = [&](int cycle, bool gave_up, double& obj, double& ll, double& lp) {
         double4 acc = make_double4(0.0, 0.0, 0.0, 0.0);
 #pragma unroll 1
         for (int k = tid; k < own.n_rows; k += kT) {
@@ -326,18 +343,23 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
         double4 t = make_double4(0.0, 0.0, 0.0, 0.0);
         if (CL) {
             if (tid < C) {
-                const unsigned a = peer_u32(&s_obj[rank], tid);
+                const unsigned a = peer_u32(&s_obj[cycle & 1][rank], tid);
                 asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(acc.x), "d"(acc.y) : "memory");
                 asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a + 16), "d"(acc.z), "d"(acc.w) : "memory");
+                tell(&s_report[cycle & 1][rank], tid, CycleReport{gave_up ? 1u : 0u, n_xch, {s_sent[0], s_sent[1]}});
             }
             cluster_barrier();  // also: rank 0's coefficients and bounds are seen by the next cycle
+            unsigned any = 0;
 #pragma unroll 1
             for (int c = 0; c < C; ++c) {
-                t.x += s_obj[c].x;
-                t.y += s_obj[c].y;
-                t.z += s_obj[c].z;
-                t.w += s_obj[c].w;
+                const double4 o = s_obj[cycle & 1][c];
+                t.x += o.x;
+                t.y += o.y;
+                t.z += o.z;
+                t.w += o.w;
+                any |= s_report[cycle & 1][c].gave_up;
             }
+            if (any) return false;
         } else {
             if (tid == 0) {
                 __stcg(Q.red + 2 * rank, make_double2(acc.x, acc.y));
@@ -406,12 +428,18 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
 
     double last = 0.0;
     long long moved = 0, rounds = 0;
-    bool failed = false;
+    bool gave_up = false;  // a wait of this CTA ran out
 
     for (int iteration = 0;; ++iteration) {
         // ---- a cycle is complete: convergence (findMode, CyclicCoordinateDescent.cpp:1023-1056)
         double cur, ll, lp;
-        if (!objective(cur, ll, lp)) return;  // the grid form's wait ran out: every CTA leaves
+        if (!objective(iteration, gave_up, cur, ll, lp)) {  // every CTA leaves
+            if (CL && gave_up && tid == 0) {
+                if (atomicCAS(&Q.st->error, 0, E_WAIT_CLUSTER) == 0) Q.st->error_where = rank;
+                land_all(s_bar, s_report[iteration & 1], C, rank);
+            }
+            return;
+        }
         if (iteration > 0) {
             const bool ill = cur != cur;
             const double conv = ill ? 0.0 : fabs(cur - last) / (fabs(cur) + 1.0);
@@ -443,11 +471,11 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
             if (me == 0 && lane == 0) s_turn = t;
             __syncthreads();
             for (;;) {
-                if (t.base >= n_active || t.stop) break;
+                if (t.base >= n_active) break;
                 const bool flying = q < t.limit;
                 if (CL && me == 0) {
                     const unsigned bytes = __reduce_add_sync(kFull, flying ? pair_bytes(q, rec_of(q)) : 0u);
-                    if (lane == 0) expect_bytes(&s_bar[n_xch & 1], bytes * (unsigned)C);
+                    if (lane == 0) expect_sums(bytes);
                 }
                 const int at = __shfl_sync(kFull, q, mine);
                 if (moved_on >> mine & 1u) {
@@ -456,6 +484,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 }
                 ++n_xch;
                 __syncthreads();
+                if (s_quit) break;
                 // ---- every column up to the first that moves is behind us
                 const unsigned to = __reduce_min_sync(kFull, flying && s_delta[lane & (kWindow - 1)] != 0.0 ? (unsigned)q : 0xffffffffu);
                 const bool moves = to != 0xffffffffu;
@@ -466,13 +495,14 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 if (COX && moves && Q.meet) n_xch += 2;
                 moved += moves;
                 ++rounds;
-                t.stop = s_abort;
                 t.base = __reduce_min_sync(kFull, q);
                 t.limit = min(t.base + width, n_active);
                 if (me == 0 && lane == 0) s_turn = t;
                 ahead.done();
                 __syncthreads();
+                if (s_quit_update) break;
             }
+            ahead.done();
         } else {
             // ================ a warp with a column
             int pos = wid;
@@ -483,7 +513,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
             __syncthreads();
             for (;;) {
                 const Turn now = s_turn;
-                if (now.base >= n_active || now.stop) break;
+                if (now.base >= n_active) break;
                 const bool mine = pos < now.limit;
                 const Rec& r = rec_of(pos);
                 double d = 0.0, hd = 0.0, b0 = 0.0, g = 0.0, h = 0.0;
@@ -662,11 +692,11 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                     }
                 }
                 // ---- the column's sums over the CTAs, the same bits in every one, and its step
-                if (!CL) grid_wait();
+                if (!CL) grid_wait(s_quit);
                 if (mine) {
                     const bool ind = r.c.flags & 4;
                     const double b_var = r.s.ptype == 2 ? b0 / r.s.pvar : 0.0;
-                    if (CL) wait_sums();
+                    if (CL) wait_sums(s_quit);
                     g = 0.0;
                     h = 0.0;
                     if (CL) {  // lane l: CTA l
@@ -732,6 +762,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 }
                 ++n_xch;
                 __syncthreads();
+                if (s_quit) break;
                 // ---- every step up to the first that is not zero stands
                 int to;
                 {
@@ -823,18 +854,19 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                         const double below = __shfl_sync(kFull, all, wid ? wid - 1 : 0);
                         if (lane == 0) pre = 0.0;
                         if (lane_open && wid > 0) pre += below;
+                        bool tails = true;  // they have come
                         if (Q.meet) {  // a stratum spans CTAs: the tail sums of the CTAs before
                             double carry = 0.0;
                             const double total = __shfl_sync(kFull, all, kWindow - 1);
                             if (CL) {
                                 if (wid == 0 && lane < C)
                                     send8(to_tail + (n_xch & 1) * (unsigned)sizeof(s_tail[0]), to_bar + (n_xch & 1) * 8u, total);
-                                if (tid == 0) expect_bytes(&s_bar[n_xch & 1], (unsigned)C * 8u);
-                                wait_sums();
-                                carry = (lane >= cut.lo && lane < rank) ? s_tail[n_xch & 1][lane & (kWindowCluster - 1)] : 0.0;
+                                if (tid == 0) expect_sums(8);
+                                tails = wait_sums(s_quit_update);
+                                carry = (lane >= cut.lo && lane < rank) ? s_tail[n_xch & (kSumBuffers - 1)][lane & (kSumCtas - 1)] : 0.0;
                             } else {
                                 if (tid == 0) __stcg(Q.tails + (n_xch & 1) * C + rank, total);
-                                grid_wait();
+                                grid_wait(s_quit_update);
                                 for (int c = cut.lo + lane; c < rank; c += 32) carry += __ldcg(Q.tails + (n_xch & 1) * C + c);
                             }
 #pragma unroll
@@ -871,23 +903,23 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                             nxt.x += ax;
                             nxt.y += ay;
                         }
-                        if (Q.meet) {  // the head sums of the CTAs after
+                        if (Q.meet && tails) {  // the head sums of the CTAs after
                             double c1 = 0.0, c2 = 0.0;
                             if (CL) {
                                 if (wid == 0 && lane < C) {
                                     const double hx = __shfl_sync(kFull >> (32 - C), all2.x, 0), hy = __shfl_sync(kFull >> (32 - C), all2.y, 0);
                                     send16(to_head + (n_xch & 1) * (unsigned)sizeof(s_head[0]), to_bar + (n_xch & 1) * 8u, hx, hy);
                                 }
-                                if (tid == 0) expect_bytes(&s_bar[n_xch & 1], (unsigned)C * 16u);
-                                wait_sums();
+                                if (tid == 0) expect_sums(16);
+                                wait_sums(s_quit_update);
                                 if (lane > rank && lane <= cut.hi) {
-                                    const double2 v = s_head[n_xch & 1][lane & (kWindowCluster - 1)];
+                                    const double2 v = s_head[n_xch & (kSumBuffers - 1)][lane & (kSumCtas - 1)];
                                     c1 = v.x;
                                     c2 = v.y;
                                 }
                             } else {
                                 if (tid == 0) __stcg(Q.heads + (n_xch & 1) * C + rank, all2);
-                                grid_wait();
+                                grid_wait(s_quit_update);
                                 for (int c = rank + 1 + lane; c <= cut.hi; c += 32) {
                                     const double2 v = __ldcg(Q.heads + (n_xch & 1) * C + c);
                                     c1 += v.x;
@@ -916,24 +948,14 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                     }
                 }
                 __syncthreads();
+                if (s_quit_update) break;
             }
         }
-        if (s_turn.stop) {
-            failed = true;
-            break;
-        }
+        __syncthreads();  // every warp is out of the rounds
+        gave_up = s_quit || s_quit_update;
+        if (!CL && gave_up) return;
     }
-    if (failed && !CL) return;
-    if (CL) {
-        if (failed && tid == 0 && atomicCAS(&Q.st->error, 0, E_WAIT_CLUSTER) == 0) Q.st->error_where = rank;
-        cluster_barrier();  // no CTA leaves while another may still send to it
-        if (failed) {
-            const unsigned m = n_xch - 1;  // the last two exchanges' bytes
-            drain(&s_bar[m & 1], (m >> 1) & 1);
-            if (m > 0) drain(&s_bar[(m - 1) & 1], ((m - 1) >> 1) & 1);
-            return;
-        }
-    }
+    if (CL) cluster_barrier();  // no CTA leaves while another may still send to it
     // the state back to where the other calls read it
 #pragma unroll 1
     for (int k = tid; WHERE == kRowsShared && k < own.n_rows; k += kT) P.xbe[own.row0 + k] = make_double2(own.xb(k), own.ex(k));
