@@ -1556,6 +1556,7 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
         P.max_iter = a->max_iterations;
         P.tol = a->tolerance;
         P.initial_bound = a->initial_bound;
+        P.xch_wait_ns = f->xch_wait_ns;
         P.y = f->y;
         if (b->row_fold) P.row_fold = (const int32_t*)keep(upload(ctx, b->row_fold, (size_t)K, s));
         std::vector<int32_t> hold(n, -1);
@@ -1665,7 +1666,6 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
             P.stage_cap = max_slice <= 1024 ? 1024 : 3072;
             P.queue = (int32_t*)keep(ctx->alloc(sizeof(int32_t) * 2));
             P.abort = P.queue + 1;
-            P.xch_wait_ns = f->xch_wait_ns;
             check_cuda(cudaMemsetAsync(P.queue, 0, sizeof(int32_t) * 2, s), "batch queue");
             P.xg = (double*)keep(ctx->alloc(sizeof(double) * (size_t)K * G * n_groups));
             P.beta_g = (double*)keep(ctx->alloc(sizeof(double) * (size_t)J * G * n_groups));
@@ -1731,7 +1731,8 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
         bool timed_out = aborted != 0;
         for (int i = 0; i < n; ++i) timed_out |= (res[i].flag == kBatchTimeoutFlag);
         if (timed_out)
-            throw Error(CCDB_ERR_TIMEOUT, "batched fits: a bounded wait for the other CTAs of a cluster ran out");
+            throw Error(CCDB_ERR_TIMEOUT, windowed ? "batched fits: a bounded wait for a copy ran out"
+                                                   : "batched fits: a bounded wait for the other CTAs of a cluster ran out");
         if (results)
             for (int i = 0; i < n; ++i) {
                 results[i].return_flag = res[i].flag;

@@ -77,7 +77,7 @@ struct BatchParams {
     // mixed, clusters: raised (set to 1) by a CTA whose wait for the other CTAs'
     // column sums ran out; zeroed before the launch
     int32_t* abort;
-    long long xch_wait_ns;     // mixed, clusters: bound on one exchange wait before abort
+    long long xch_wait_ns;     // bound on one wait: for a cluster's exchange (mixed), for a copy (windowed)
 };
 
 constexpr int kKeyRowBits = 24;

@@ -180,7 +180,8 @@ struct Fit {
     bool offset_col0 = false;
     cudaStream_t stream = nullptr;
     // bounds on device-side waits (ccdb_fit_set_wait_limit): the grid sweep's level,
-    // column and grid waits, and the mixed batch engine's cluster exchange
+    // column and grid waits and the windowed sweeps' exchanges; the batch engines'
+    // cluster exchange and copies
     static constexpr long long kDefaultWaitNs = 20LL * 1000 * 1000 * 1000;
     static constexpr long long kDefaultXchWaitNs = 2LL * 1000 * 1000 * 1000;
     long long wait_limit_ns = kDefaultWaitNs;

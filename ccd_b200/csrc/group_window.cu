@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     };
     // this exchange's bytes have come, all of them to the whole warp (cluster form)
     auto wait_sums = [&](int& quit) {
-        const bool ok = __all_sync(kFull, wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1));
+        const bool ok = __all_sync(kFull, wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1, Q.wait_limit_ns));
         if (!ok) quit = 1;
         return ok;
     };

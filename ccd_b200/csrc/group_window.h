@@ -53,7 +53,7 @@ struct GroupWindowParams {
     double2* heads;  // 2 x ctas
     double2* red;    // 2 x ctas: objective partials
     unsigned* grid_bar;
-    long long wait_limit_ns;
+    long long wait_limit_ns;  // bound on any single wait for the other CTAs
     int64_t* counters;  // [0]: nonzero steps, [1]: rounds
 };
 

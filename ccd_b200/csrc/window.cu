@@ -47,7 +47,7 @@
 // the CTAs' pairs added four at a time in every lane, bounds settled by the warps
 // with columns and the gather unrolled, these took 4.5, 53 and 154 ms.
 //
-// The wait for the other CTAs' pairs is bounded (kWaitNs).  A CTA whose wait runs out
+// The wait for the other CTAs' pairs is bounded (the fit's limit).  A CTA whose wait runs out
 // steps and sends no more; at the end of the cycle the CTAs learn of it from one
 // another and all leave, each once what was sent to it has landed (sweep_exit.h).
 #include <algorithm>
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
         expect_bytes(&s_bar[n_xch & 1], (unsigned)(columns * C * 2 * sizeof(double)));
     };
     auto wait_pairs = [&]() {
-        if (!wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1)) s_abort = 1;
+        if (!wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1, P.wait_limit_ns)) s_abort = 1;
     };
     // the column's sums over the CTAs, the same bits in every lane and CTA (the
     // pairs of CTAs that there are not stay zero): lane l takes CTA l & 15, its g

@@ -19,7 +19,7 @@ constexpr int kWarps = kT / 32;
 constexpr int kE = 4;            // staged entries per lane
 constexpr int kStage = 32 * kE;  // a warp's column: its first entries, copied ahead
 constexpr unsigned kFull = 0xffffffffu;
-constexpr unsigned long long kWaitNs = 10ull * 1000 * 1000 * 1000;
+constexpr long long kLookNs = 1000 * 1000;  // an attempt to wait sleeps in hardware for less
 static_assert(kHelpers * 4 == kWindow, "eight lanes of a helper copy for a slot");
 
 // The record of one position, copied ahead of its use.
@@ -73,6 +73,17 @@ __device__ __forceinline__ void send16(unsigned at, unsigned bar, double a, doub
 __device__ __forceinline__ void expect_bytes(const uint64_t* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+// whether the bytes have come: a look, then one that sleeps in hardware for a while
+__device__ __forceinline__ bool landed(const uint64_t* bar, unsigned parity) {
+    unsigned done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return done != 0;
+}
 __device__ __forceinline__ bool arrived(const uint64_t* bar, unsigned parity) {
     unsigned done;
     asm volatile(
@@ -83,14 +94,15 @@ __device__ __forceinline__ bool arrived(const uint64_t* bar, unsigned parity) {
         : "memory");
     return done != 0;
 }
-// false when the bytes have not all come within kWaitNs
-__device__ __forceinline__ bool wait_bytes(const uint64_t* bar, unsigned parity) {
-    unsigned long long t0 = 0;
-    for (unsigned n = 0; !arrived(bar, parity); ++n)  // an attempt sleeps in hardware for a while
-        if ((n & 15u) == 15u) {
+// false when the bytes have not all come within limit_ns
+__device__ __forceinline__ bool wait_bytes(const uint64_t* bar, unsigned parity, long long limit_ns) {
+    const bool brief = limit_ns < kLookNs;  // a bound below one sleep is kept by looks alone
+    unsigned long long t0 = brief ? global_ns() : 0;
+    for (unsigned n = 0; !(brief ? landed(bar, parity) : arrived(bar, parity)); ++n)
+        if (brief || (n & 15u) == 15u) {
             const unsigned long long t = global_ns();
             if (t0 == 0) t0 = t;
-            if (t - t0 > kWaitNs) return false;
+            if ((long long)(t - t0) > limit_ns) return false;
         }
     return true;
 }

@@ -364,7 +364,7 @@ class Fit:
 
     def set_wait_limit(self, nanoseconds: int) -> None:
         """Bound on every single device-side wait of later launches (0: the
-        defaults, 20 s for the grid sweep, 2 s for the batch exchange)."""
+        defaults, 20 s for a sweep's waits, 2 s for the batch engines')."""
         _check(lib().ccdb_fit_set_wait_limit(self.h, int(nanoseconds)))
 
     def last_call_seconds(self) -> float:

@@ -335,13 +335,13 @@ int ccdb_matrix_validate(int64_t K, int32_t J, const int64_t* col_start, const i
 
 /* Bound, in nanoseconds, on every single device-side wait of this fit's later
  * launches: the grid-wide level sweep's waits for a level, a split column and
- * the grid barrier (default 20 s), and the mixed batch engine's wait for the
- * per-column sums of the other CTAs of its cluster (default 2 s).  0 restores
+ * the grid barrier and the windowed sweeps' waits for the sums of the other CTAs
+ * (default 20 s), the mixed batch engine's wait for the per-column sums of the
+ * other CTAs of its cluster and the windowed one's for a copy (default 2 s).  0 restores
  * the defaults.  A wait that runs out ends the call with CCDB_ERR_TIMEOUT and
  * leaves the context usable; the fit's state is then undefined until the next
- * ccdb_set_beta or ccdb_find_mode with starting values.  The windowed sweep's
- * wait for the other CTAs of its cluster has a bound of its own (10 s).  No
- * reference counterpart. */
+ * ccdb_set_beta or ccdb_find_mode with starting values.  No reference
+ * counterpart. */
 int ccdb_fit_set_wait_limit(ccdb_fit* f, int64_t nanoseconds);
 
 /* Device time (CUDA events on the fit's stream) of the kernels of the fit's last
