@@ -200,12 +200,12 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     __shared__ double s_run[kWindow];    // the worker warps' prefix sums
     __shared__ double2 s_run2[kWindow];  // and suffix sums
     __shared__ int s_first[kWindow], s_last[kWindow];  // a stratum begins, ends among a worker warp's groups
-    __shared__ double s_delta[kWindow];  // the steps of the columns in flight
+    // the steps of the columns in flight; behind them, not zero: a wait for their sums ran
+    // out (before the round's first barrier, and read behind it; one of an update is in
+    // s_turn.stop, before the second barrier and read behind that)
+    __shared__ double s_delta[kWindow + 1];
     __shared__ Turn s_turn;
     __shared__ uint64_t s_bar[2];
-    // a wait ran out: of the gradients, before the round's first barrier, read behind it;
-    // of an update, before the second, read behind that
-    __shared__ int s_quit, s_quit_update;
     __shared__ int32_t s_fail;
     __shared__ uint8_t s_flags[kGroupWindowCtas];  // GroupCut::flags of every CTA
     extern __shared__ __align__(16) unsigned char s_dyn[];
@@ -272,7 +272,8 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     }
     for (int c = tid; c < C; c += kT) s_flags[c] = (uint8_t)Q.cuts[c].flags;
     if (tid == 0) {
-        s_quit = s_quit_update = 0;
+        s_delta[kWindow] = 0.0;
+        s_turn.stop = 0;
         if (CL) init_bars(s_bar, 2);
     }
     // sums of CTAs that there are not stay zero
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     // bytes that a column's partial sums of one CTA take in an exchange
     auto pair_bytes = [&](int pos, const Rec& r) { return COX ? ((r.c.flags & 4) ? 32u : 48u) : 16u; };
     // workers, grid form: everything written before is seen by every CTA after it
-    auto grid_wait = [&](int& quit) {
+    auto grid_wait = [&](auto& quit) {
         workers_barrier();
         if (tid == 0) {
             ++epoch;
@@ -309,9 +310,9 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
         }
         workers_barrier();
     };
-    // this exchange's bytes have come, all of them to the whole warp (cluster form)
-    auto wait_sums = [&](int& quit) {
-        const bool ok = __all_sync(kFull, wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1, Q.wait_limit_ns));
+    // this exchange's bytes have come to this thread (cluster form)
+    auto wait_sums = [&](auto& quit) {
+        const bool ok = wait_bytes(&s_bar[n_xch & 1], (n_xch >> 1) & 1, Q.wait_limit_ns);
         if (!ok) quit = 1;
         return ok;
     };
@@ -468,7 +469,12 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
             unsigned moved_on = 0;  // the slots that took up a new column in the last round
             int width = kNarrow;
             Turn t{0, min(width, n_active), 0, 0};
-            if (me == 0 && lane == 0) s_turn = t;
+            auto show_turn = [&]() {
+                if (me != 0 || lane != 0) return;
+                s_turn.base = t.base;
+                s_turn.limit = t.limit;
+            };
+            show_turn();
             __syncthreads();
             for (;;) {
                 if (t.base >= n_active) break;
@@ -484,7 +490,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 }
                 ++n_xch;
                 __syncthreads();
-                if (s_quit) break;
+                if (s_delta[kWindow] != 0.0) break;
                 // ---- every column up to the first that moves is behind us
                 const unsigned to = __reduce_min_sync(kFull, flying && s_delta[lane & (kWindow - 1)] != 0.0 ? (unsigned)q : 0xffffffffu);
                 const bool moves = to != 0xffffffffu;
@@ -497,10 +503,10 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 ++rounds;
                 t.base = __reduce_min_sync(kFull, q);
                 t.limit = min(t.base + width, n_active);
-                if (me == 0 && lane == 0) s_turn = t;
+                show_turn();
                 ahead.done();
                 __syncthreads();
-                if (s_quit_update) break;
+                if (s_turn.stop) break;
             }
             ahead.done();
         } else {
@@ -513,7 +519,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
             __syncthreads();
             for (;;) {
                 const Turn now = s_turn;
-                if (now.base >= n_active) break;
+                if (now.stop || now.base >= n_active) break;
                 const bool mine = pos < now.limit;
                 const Rec& r = rec_of(pos);
                 double d = 0.0, hd = 0.0, b0 = 0.0, g = 0.0, h = 0.0;
@@ -692,11 +698,11 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                     }
                 }
                 // ---- the column's sums over the CTAs, the same bits in every one, and its step
-                if (!CL) grid_wait(s_quit);
+                if (!CL) grid_wait(s_delta[kWindow]);
                 if (mine) {
                     const bool ind = r.c.flags & 4;
                     const double b_var = r.s.ptype == 2 ? b0 / r.s.pvar : 0.0;
-                    if (CL) wait_sums(s_quit);
+                    if (CL) wait_sums(s_delta[kWindow]);
                     g = 0.0;
                     h = 0.0;
                     if (CL) {  // lane l: CTA l
@@ -762,12 +768,13 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 }
                 ++n_xch;
                 __syncthreads();
-                if (s_quit) break;
                 // ---- every step up to the first that is not zero stands
                 int to;
                 {
-                    const int slot = (now.base + lane) & (kWindow - 1);
-                    const unsigned nz = __ballot_sync(kFull, now.base + lane < now.limit && lane < kWindow && s_delta[slot] != 0.0);
+                    const int slot = lane < kWindow ? (now.base + lane) & (kWindow - 1) : kWindow;
+                    const bool here = lane < kWindow ? now.base + lane < now.limit : lane == kWindow;
+                    const unsigned nz = __ballot_sync(kFull, here & (s_delta[slot] != 0.0));
+                    if (nz >> kWindow) break;
                     to = nz ? now.base + __ffs(nz) - 1 : 0x7fffffff;
                 }
                 if (mine && pos <= to) {
@@ -862,11 +869,11 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                                 if (wid == 0 && lane < C)
                                     send8(to_tail + (n_xch & 1) * (unsigned)sizeof(s_tail[0]), to_bar + (n_xch & 1) * 8u, total);
                                 if (tid == 0) expect_sums(8);
-                                tails = wait_sums(s_quit_update);
+                                tails = __all_sync(kFull, wait_sums(s_turn.stop));
                                 carry = (lane >= cut.lo && lane < rank) ? s_tail[n_xch & (kSumBuffers - 1)][lane & (kSumCtas - 1)] : 0.0;
                             } else {
                                 if (tid == 0) __stcg(Q.tails + (n_xch & 1) * C + rank, total);
-                                grid_wait(s_quit_update);
+                                grid_wait(s_turn.stop);
                                 for (int c = cut.lo + lane; c < rank; c += 32) carry += __ldcg(Q.tails + (n_xch & 1) * C + c);
                             }
 #pragma unroll
@@ -911,7 +918,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                                     send16(to_head + (n_xch & 1) * (unsigned)sizeof(s_head[0]), to_bar + (n_xch & 1) * 8u, hx, hy);
                                 }
                                 if (tid == 0) expect_sums(16);
-                                wait_sums(s_quit_update);
+                                wait_sums(s_turn.stop);
                                 if (lane > rank && lane <= cut.hi) {
                                     const double2 v = s_head[n_xch & (kSumBuffers - 1)][lane & (kSumCtas - 1)];
                                     c1 = v.x;
@@ -919,7 +926,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                                 }
                             } else {
                                 if (tid == 0) __stcg(Q.heads + (n_xch & 1) * C + rank, all2);
-                                grid_wait(s_quit_update);
+                                grid_wait(s_turn.stop);
                                 for (int c = rank + 1 + lane; c <= cut.hi; c += 32) {
                                     const double2 v = __ldcg(Q.heads + (n_xch & 1) * C + c);
                                     c1 += v.x;
@@ -948,11 +955,9 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                     }
                 }
                 __syncthreads();
-                if (s_quit_update) break;
             }
         }
-        __syncthreads();  // every warp is out of the rounds
-        gave_up = s_quit || s_quit_update;
+        gave_up = s_delta[kWindow] != 0.0 || s_turn.stop;
         if (!CL && gave_up) return;
     }
     if (CL) cluster_barrier();  // no CTA leaves while another may still send to it
