@@ -114,15 +114,6 @@ int64_t Matrix::entries(int j) const {
     return col_start[j + 1] - col_start[j];
 }
 
-int64_t Matrix::mean_entries() const {
-    int64_t sum = 0, longest = 0;
-    for (int j = 0; j < J; ++j) {
-        sum += entries(j);
-        longest = std::max(longest, entries(j));
-    }
-    return J > 1 ? (sum - longest) / (J - 1) : longest;
-}
-
 Matrix::~Matrix() {
     for (void* p : {(void*)d_col_ptr, (void*)d_rows, (void*)d_val_ptr, (void*)d_vals, (void*)d_fmt,
                     (void*)d_row_ptr, (void*)d_csr_col, (void*)d_csr_val})
@@ -738,10 +729,14 @@ void Fit::ensure_window(int ctas) {
     window->ctas = ctas;
 }
 
+int64_t Fit::batch_mean() const {
+    return batch_mean_entries(J, offset_col0, [&](int j) { return m->entries(j); });
+}
+
 // The batched fits' plan: every column but an offset one, whole on one CTA.
 void Fit::ensure_batch_window() {
     if (batch_window) return;
-    const BatchTeam t = batch_team(m->mean_entries());
+    const BatchTeam t = batch_team(batch_mean());
     std::vector<uint8_t> skip(J, 0);
     if (offset_col0) skip[0] = 1;
     const WindowPlan plan = build_window_plan(K, J, m->col_start.data(), m->rows_h.data(), m->val_start.data(),
@@ -1511,9 +1506,9 @@ static int batch_cluster_size(const Matrix* m, int64_t K, int n_groups, int n_sm
 
 // Whether the windowed engine serves a batch whose caller names no launch shape:
 // short columns, and a workspace within the context's memory budget.
-static bool batch_windowed(Context* ctx, const Matrix* m, int64_t K, int n, int ctas, bool mixed, int spill) {
-    if (m->mean_entries() > kBatchWindowMean) return false;
-    const size_t J = m->J, state = (spill & 1 ? 8 : 0) + (spill & 2 ? (mixed ? 4 : 8) : 0);
+static bool batch_windowed(Context* ctx, const Fit* f, int n, int ctas, bool mixed, int spill) {
+    if (f->batch_mean() > kBatchWindowMean) return false;
+    const size_t J = f->J, K = f->K, state = (spill & 1 ? 8 : 0) + (spill & 2 ? (mixed ? 4 : 8) : 0);
     const size_t bytes = ctas * ((sizeof(WinScal) + sizeof(double2)) * J + state * K) + sizeof(double) * J * n +
                          (sizeof(WinCol) + sizeof(WinSlice) + sizeof(int32_t)) * J + 4096;
     std::lock_guard<std::mutex> g(ctx->mu);
@@ -1611,7 +1606,7 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
         int spill = 0;
         check_cuda(batch_window_spill(K, mixed, any_vals, &spill), "batch sweep");
         const bool shaped = mixed && (b->group || b->cluster || trace_path);  // asks for the lockstep engine
-        const bool windowed = !shaped && batch_windowed(ctx, m, K, n, ctas, mixed, spill);
+        const bool windowed = !shaped && batch_windowed(ctx, f, n, ctas, mixed, spill);
         if (windowed) {
             f->ensure_batch_window();
             const DevWindow& w = *f->batch_window;

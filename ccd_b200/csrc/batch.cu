@@ -1,7 +1,7 @@
 // batch.cu -- many fits over one shared CompressedDataMatrix in one launch
 // (the cross-validation grid: folds x prior variances), in FP64 and one column
 // at a time: the engine of fits with long columns (kBatchWindowMean,
-// batch_window.h).
+// batch_route.h).
 //
 // Each CTA owns one instance: its row weights (0 on the held-out fold, as
 // CrossValidationSelector::getWeights sets them, drivers/CrossValidationSelector.cpp:72-130),

@@ -1,6 +1,6 @@
 // batch_mixed.cu -- the cross-validation grid in mixed precision, with the
 // instances of a CTA stepping through the columns in lockstep: the engine of fits
-// with long columns (kBatchWindowMean, batch_window.h) and of calls that name a
+// with long columns (kBatchWindowMean, batch_route.h) and of calls that name a
 // group or cluster.
 //
 // A CTA runs a group of G instances (G = 1, 2 or 4; consecutive in the launch

@@ -95,7 +95,6 @@ struct Matrix {
     int64_t entries(int j) const;
     // values of the row-major copy; NULL where every one is 1
     const double* csr_values() const { return val_start.back() > 0 ? d_csr_val : nullptr; }
-    int64_t mean_entries() const;  // of the columns but the longest
     void ensure_csr(cudaStream_t s);
     ~Matrix();
 };
@@ -255,6 +254,7 @@ struct Fit {
     int window_ctas();
     void ensure_window(int ctas);
     void release_window();
+    int64_t batch_mean() const;  // entries of the columns that a batch steps (batch_route.h)
     void ensure_batch_window();
     void release_batch_window();
     void find_mode_window(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms);
