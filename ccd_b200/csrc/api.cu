@@ -1461,19 +1461,6 @@ int ccdb_fit_model(ccdb_context* ctx, int64_t K, int32_t J, const int64_t* col_s
     return rc;
 }
 
-// Lockstep group size of the mixed-precision batched engine.  G = 4 packs the
-// group's state for one row into one 32-byte sector (a quarter of the DRAM
-// sectors G = 1 moves per instance), but gives one CTA G times the per-column
-// arithmetic and leaves ceil(n / G) CTAs for the SMs.  Take the largest G that
-// still gives every third SM a CTA.
-static int batch_group_size(const Matrix* m, int n, int n_sm) {
-    (void)m;
-    const int want = std::max(1, n_sm / 3);
-    for (int G : {4, 2})
-        if ((n + G - 1) / G >= want) return G;
-    return 1;
-}
-
 // Longest slice of a row-indexed column when C CTAs split the rows evenly.
 static int64_t batch_max_slice(const Matrix* m, int64_t K, int C) {
     int64_t mx = 0;
@@ -1504,10 +1491,10 @@ static int batch_cluster_size(const Matrix* m, int64_t K, int n_groups, int n_sm
     return 8;
 }
 
-// Whether the windowed engine serves a batch whose caller names no launch shape:
-// short columns, and a workspace within the context's memory budget.
+// Whether the windowed engine serves a batch whose caller names no launch shape: it
+// is the faster one, and its workspace is within the context's memory budget.
 static bool batch_windowed(Context* ctx, const Fit* f, int n, int ctas, bool mixed, int spill) {
-    if (f->batch_mean() > kBatchWindowMean) return false;
+    if (!batch_prefers_window({mixed, !(spill & 2), f->K, f->batch_mean(), n, ctx->n_sm})) return false;
     const size_t J = f->J, K = f->K, state = (spill & 1 ? 8 : 0) + (spill & 2 ? (mixed ? 4 : 8) : 0);
     const size_t bytes = ctas * ((sizeof(WinScal) + sizeof(double2)) * J + state * K) + sizeof(double) * J * n +
                          (sizeof(WinCol) + sizeof(WinSlice) + sizeof(int32_t)) * J + 4096;
@@ -1629,7 +1616,7 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
             check_cuda(cudaMemsetAsync(P.queue, 0, sizeof(int32_t), s), "batch queue");
             W.beta_out = P.beta = (double*)keep(ctx->alloc(sizeof(double) * (size_t)J * n));
         } else if (mixed) {
-            G = b->group ? b->group : batch_group_size(m, n, ctx->n_sm);
+            G = b->group ? b->group : batch_group_size(n, ctx->n_sm);
             if (G != 1 && G != 2 && G != 4) throw Error(CCDB_ERR_INVALID, "batch group must be 1, 2 or 4");
             n_groups = (n + G - 1) / G;
             P.group = G;

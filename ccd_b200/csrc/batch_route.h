@@ -33,11 +33,75 @@ struct BatchTeam {
 constexpr BatchTeam batch_team(int64_t mean) {
     return mean <= kBatchOneWarp ? BatchTeam{1, 128, 512} : BatchTeam{4, 320, 2048};
 }
-// Above this mean the sweeps that take one column at a time are the faster ones:
-// their gathers fill the memory pipe, and the lockstep groups read a row once for
-// four fits.  200 fits of 100,000 rows, windowed against one column at a time: mean
-// 200, FP64 7.4 against 14.1 ms and mixed 6.9 against 14.8; 500, 17.0 against 19.4
-// and 15.6 against 19.3; 1,000, 35.4 against 33.4 and 31.4 against 25.5.
-constexpr int64_t kBatchWindowMean = 640;
+// A batch as the choice between the engines sees it.
+struct BatchSize {
+    bool mixed;
+    bool share_in_shared;  // the rows' shares fit a CTA's shared memory
+    int64_t K, mean;
+    int n, n_sm;
+};
+
+// Lockstep group size of the mixed-precision batched engine.  G = 4 packs the
+// group's state for one row into one 32-byte sector (a quarter of the DRAM
+// sectors G = 1 moves per instance), but gives one CTA G times the per-column
+// arithmetic and leaves ceil(n / G) CTAs for the SMs.  Take the largest G that
+// still gives every third SM a CTA.
+constexpr int batch_group_size(int n, int n_sm) {
+    const int want = std::max(1, n_sm / 3);
+    for (int G : {4, 2})
+        if ((n + G - 1) / G >= want) return G;
+    return 1;
+}
+// The group, and the waves of CTAs when a cluster of up to eight gives every SM one.
+struct LockstepShape {
+    int group, cluster, waves;
+};
+constexpr LockstepShape lockstep_shape(int n, int n_sm) {
+    const int G = batch_group_size(n, n_sm), groups = (n + G - 1) / G;
+    int C = 1;
+    while (C < 8 && groups * C < n_sm) C *= 2;
+    return {G, C, (groups * C + n_sm - 1) / n_sm};
+}
+
+// Whether the windowed engine is the faster one.  It takes time like the columns'
+// mean and like n / SMs (a CTA takes the next fit when one ends); the sweeps that
+// step one column at a time fill the memory pipe with a long column's gathers, the
+// mixed ones read a row once for the up to four fits of a group, and their time
+// goes in whole waves.  So the line is a mean: 300 where the shares lie in global
+// memory, 480 in shared memory, for a wave of each, times the waves and what a group
+// costs more (of two 1.12; of four 1.45, 2 without a cluster), over n / SMs.
+// Up to 500 and 640 whatever the waves: above 508 entries a column is not all
+// copied ahead.  Time of the mixed engine over the windowed one, 600 columns:
+//   rows, fits: mean 200   300   350   450   500   560
+//   40,000,   4     2.25  1.38  1.16  1.11  0.99  0.83
+//   40,000, 450     2.28  1.55  1.30  1.20  1.03  0.85
+//   40,000, 1000    1.46  0.97  0.81  0.78  0.67  0.55
+//   100,000,   4    1.92  1.06  0.83  0.77  0.68  0.57
+//   100,000,  60    3.74  2.06  1.61  1.48  1.27  1.01
+//   100,000, 250    2.52  1.61  1.27  1.11  0.98  0.80
+//   100,000, 600    1.33  0.88  0.70  0.64  0.56  0.46
+// FP64 has one CTA a fit in both.  With the rows in shared memory the windowed one
+// is faster to the end (20,000 rows, mean 560: 1.13 to 1.67).  Else, up to one fit
+// an SM, the two are even from 360 to 450 and it loses above (100,000 rows, 148
+// fits: mean 300 1.11, 400 0.92; 40,000 rows: 400 1.07, 500 1.00, 560 0.87).  With
+// more fits it gains from the fits that end early while the running ones' state
+// fits L2 (40,000 rows, 200 fits: mean 500 1.27, 560 1.07), and less beyond (100,000
+// rows: 400 1.14, 500 1.02; 250,000 rows: 300 1.22, 400 1.00, 500 0.91).
+constexpr int64_t kBatchWindowMean = 640;  // above it never (100,000 rows, 200 fits, mean 1,000: 0.94, mixed 0.72)
+constexpr int64_t kBatchL2 = 100 << 20;    // of the 126 MB of L2, what the fits' rows may take
+
+constexpr bool batch_prefers_window(const BatchSize& b) {
+    if (b.mean > kBatchWindowMean) return false;
+    if (b.mixed) {
+        const LockstepShape s = lockstep_shape(b.n, b.n_sm);
+        const double turns = std::max(1.0, (double)b.n / b.n_sm);
+        const double group = s.group == 1 ? 1.0 : s.group == 2 ? 1.12 : s.cluster > 1 ? 1.45 : 2.0;
+        const double line = (b.share_in_shared ? 480 : 300) * s.waves * group / turns;
+        return b.mean <= std::min(line, b.share_in_shared ? 640.0 : 500.0);
+    }
+    if (b.share_in_shared) return true;
+    if (b.n <= b.n_sm) return b.mean <= 360;
+    return 16 * b.K * b.n_sm <= kBatchL2 || b.mean <= 450;
+}
 
 }  // namespace ccdb

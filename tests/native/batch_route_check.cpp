@@ -30,8 +30,45 @@ static void means() {
     check(batch_mean_entries(1, true, [](int) { return 7; }) == 0, "an offset alone");
 }
 
+// (fits, rows, mean) on 148 SMs where one engine was measured at least 5 % faster
+static void routes() {
+    struct {
+        bool mixed, shared;
+        int64_t K;
+        int n;
+        int64_t mean;
+        bool window;
+    } const at[] = {
+        {true, true, 40000, 4, 450, true},      {true, true, 40000, 4, 560, false},
+        {true, true, 40000, 60, 620, true},     {true, true, 40000, 148, 400, true},
+        {true, true, 40000, 250, 620, true},    {true, true, 40000, 600, 350, true},
+        {true, true, 40000, 1000, 200, true},   {true, true, 40000, 1000, 450, false},
+        {true, false, 100000, 4, 300, true},    {true, false, 100000, 4, 400, false},
+        {true, false, 100000, 60, 500, true},   {true, false, 100000, 80, 620, false},
+        {true, false, 100000, 148, 300, true},  {true, false, 100000, 148, 400, false},
+        {true, false, 100000, 200, 500, true},  {true, false, 100000, 300, 300, true},
+        {true, false, 100000, 300, 500, false}, {true, false, 100000, 450, 350, false},
+        {true, false, 100000, 600, 200, true},  {true, false, 100000, 600, 350, false},
+        {true, false, 100000, 1000, 300, false}, {true, false, 250000, 10, 300, true},
+        {true, false, 250000, 10, 400, false},  {true, false, 250000, 300, 500, false},
+        {false, true, 20000, 10, 560, true},    {false, true, 20000, 300, 560, true},
+        {false, false, 40000, 10, 200, true},   {false, false, 40000, 10, 560, false},
+        {false, false, 40000, 200, 500, true},  {false, false, 100000, 148, 300, true},
+        {false, false, 100000, 148, 500, false}, {false, false, 250000, 40, 500, false},
+        {false, false, 250000, 300, 300, true}, {false, false, 250000, 300, 500, false},
+        {true, true, 5000, 20, 1000, false},    {false, true, 5000, 20, 1000, false},
+    };
+    for (const auto& c : at) {
+        char what[128];
+        std::snprintf(what, sizeof what, "%s, %lld rows, %d fits, mean %lld", c.mixed ? "mixed" : "FP64", (long long)c.K, c.n,
+                      (long long)c.mean);
+        check(batch_prefers_window({c.mixed, c.shared, c.K, c.mean, c.n, 148}) == c.window, what);
+    }
+}
+
 int main() {
     means();
+    routes();
     if (!failures) std::printf("all routes as expected\n");
     return failures ? 1 : 0;
 }
