@@ -356,6 +356,7 @@ void Fit::ensure_group_window(int ctas, bool cluster) {
         c.flags = ((f == F_SPARSE || f == F_INDICATOR) ? 1 : 0) | ((f == F_SPARSE || f == F_DENSE) ? 2 : 0) |
                   ((f == F_INDICATOR || f == F_INTERCEPT) ? 4 : 0);
         window->any_vals |= (c.flags & 2) != 0;
+        window->any_long |= !is_cox() && c.n > kGroupLong;
         cols.push_back(c);
     }
     // Where a CTA's groups begin.  Cox: at the nearest start of a stratum, when no CTA
@@ -429,7 +430,8 @@ void Fit::ensure_group_window(int ctas, bool cluster) {
         window->tails = static_cast<double*>(ctx->alloc(sizeof(double) * 2 * ctas));
         window->heads = static_cast<double2*>(ctx->alloc(sizeof(double2) * 2 * ctas));
     }
-    check_cuda(launch_window_slices(m->d_rows, window->cols, (int32_t)n, window->cuts, ctas, window->slices, stream),
+    check_cuda(launch_window_slices(m->d_rows, window->cols, (int32_t)n, window->cuts, ctas, window->any_long, window->slices,
+                                    stream),
                "sweep plan");
     ++launches;
     check_cuda(ctx->wait(), "sweep plan");
@@ -529,6 +531,7 @@ void Fit::find_mode_group_window(const ccdb_mode_args& a, int* flag, int* iters,
     Q.ctas = window->ctas;
     Q.ll_fixed = ll_fixed;
     Q.any_vals = window->any_vals ? 1 : 0;
+    Q.any_long = window->any_long ? 1 : 0;
     Q.meet = window->meet ? 1 : 0;
     Q.chain = window->chain;
     Q.st = st;

@@ -131,7 +131,8 @@ struct DevWindow {
     bool cluster = false;
     int64_t grouping = -1;
     int64_t most_rows = 0, most_groups = 0;
-    bool meet = false;  // a stratum spans CTAs
+    bool any_long = false;  // a column may be too long for one warp
+    bool meet = false;      // a stratum spans CTAs
     int32_t chain = 1;
     GroupCut* cuts = nullptr;
     double2* part = nullptr;

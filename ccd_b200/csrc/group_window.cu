@@ -16,7 +16,13 @@
 //
 // Grouped models (GroupedData, ModelSpecifics.hpp:1101-1179): a stratum's run of
 // entries contributes t = numerator / denominator; a CTA's strata are whole, so a
-// column's partial sums are just (g, h).
+// column's partial sums are just (g, h).  A column with a slice of over kGroupLong
+// entries runs alone, on every warp: one warp that walked it was slower than the
+// kernel before this one where few CTAs shared the rows (300,000 rows, six dense
+// columns, on 1, 4, 8 CTAs: 197, 49, 22 ms; on every warp 30, 8.0, 3.9).  Alone
+// against one warp, 60 columns on 16 CTAs, slices of 600: 1.19 and 2.45 ms (L1), 1.46
+// and 4.23 (every step moves); of 300, on one CTA with hardly a step that moves, where
+// it gives up columns in flight: 0.64 and 0.42.
 //
 // Cox (cox.cu): g = sum n1 S1, h = sum n2 S1 - sum S2 (A^2 - A'^2) with A the
 // running sum of n1 within the stratum and A' the one before the entry.  A stratum
@@ -181,8 +187,10 @@ struct Owned {
     __device__ __forceinline__ bool last(int g) const { return WHERE != kGlobal ? strat_[g] & 2 : P->glast[g0 + g]; }
 };
 
-// MX: the mixed precision of the Cox engine.
-template <bool COX, int WHERE, bool CL, bool MX>
+// MX: the mixed precision of the Cox engine.  LONG: a grouped model has a column that
+// may be long; without it the code of one costs the others (26,000 x 500 conditional
+// logistic, no long column: 3.17 ms, 3.4 with it).
+template <bool COX, int WHERE, bool CL, bool MX, bool LONG>
 __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q) {
     __shared__ Rec s_rec[4][kWindow];  // by position: (position / kWindow) & 3, slot
     // cluster form, by exchange parity, column and CTA: Cox {G, HQ}, {B, T}, {H2, 0}, else {g, h}
@@ -388,14 +396,116 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     const Ahead ahead{Q.cols, Q.scal, Q.bh, slices, P.rows, P.vals, n_active};
     auto fetch = [&](int at, int l8) { ahead.record(at, rec_of(at), l8); };
     auto stage = [&](int at, int l8) { ahead.entries(at, rec_of(at), s_rows + stage_at(at), s_vals + stage_at(at), l8); };
+    // a column that runs alone, on every warp (grouped models); it is not copied ahead
+    auto long_column = [&](const Rec& r) { return LONG && (r.c.flags & 8); };
     // entry e of a record's slice: local row and value
     auto entry_row = [&](const Rec& r, int at, int e) {
-        if (e < kStage) return s_rows[stage_at(at) + e] - (int)own.row0;
+        if (e < kStage && !long_column(r)) return s_rows[stage_at(at) + e] - (int)own.row0;
         return ((r.c.flags & 1) ? __ldg(P.rows + r.c.cb + r.e.lo + e) : r.e.lo + e) - (int)own.row0;
     };
     auto entry_val = [&](const Rec& r, int at, int e) {
         if (!(r.c.flags & 2)) return 1.0;
-        return e < kStage ? s_vals[stage_at(at) + e] : __ldg(P.vals + r.c.vb + r.e.lo + e);
+        return e < kStage && !long_column(r) ? s_vals[stage_at(at) + e] : __ldg(P.vals + r.c.vb + r.e.lo + e);
+    };
+
+    // Grouped models: the sums of a long column over this CTA's slice, by all workers, in
+    // the warp that `takes` them.  Each warp walks sixteenths of the slice, whole passes of
+    // 32 entries; a run of entries that goes over its ends (a stratum met from both sides)
+    // is handed on in parts and put together at the end.
+    auto gather_alone = [&](const Rec& r, int at, bool takes) {
+        const int n = r.e.hi - r.e.lo, share = ((n + 32 * kWindow - 1) / (32 * kWindow)) * 32;
+        const int c0 = min(wid * share, n), c1 = min(c0 + share, n);
+        const bool ind = r.c.flags & 4;
+        // by warp: {g, h}, the part of a run that began before it, the part of one that goes on
+        // behind it; s_dg: 1 the former ends here, 2 it goes on, 4 there is a latter; and its stratum
+        double* const mine = s_dd + 6 * wid;
+        double g = 0.0, h = 0.0, run1 = 0.0, run2 = 0.0;
+        auto add_run = [&](int key, double a, double b) {
+            const double dn = own.den(key), ne = own.nev(key), t = a / dn, gg = ne * t;
+            g += gg;
+            h += ind ? gg * (1.0 - t) : ne * (b / dn - t * t);
+        };
+        int run_key = c0 > 0 && c0 < n ? own.group(entry_row(r, at, c0 - 1)) : -1;
+        bool joined = true;  // no run has begun in this warp's part so far
+        int parts = 0;
+#pragma unroll 1
+        for (int e0 = c0; e0 < c1; e0 += 32) {
+            const int e = e0 + lane;
+            const bool in = e < n;
+            int key = 0x7fffffff;
+            double a = 0.0, b = 0.0;
+            if (in) {
+                const int k = entry_row(r, at, e);
+                const double x = entry_val(r, at, e), ex = own.ex(k);
+                key = own.group(k);
+                a = ex * x;
+                if (!ind) b = ex * x * x;
+            }
+            int next = __shfl_down_sync(kFull, key, 1);
+            if (lane == 31) next = e + 1 < n ? own.group(entry_row(r, at, e + 1)) : -1;
+            int prev = __shfl_up_sync(kFull, key, 1);
+            if (lane == 0) prev = run_key;
+            const unsigned all_starts = __ballot_sync(kFull, key != prev);
+            const unsigned starts = all_starts & (kFull >> (31 - lane));
+            const int start = reach_down(all_starts, lane);
+#pragma unroll 1
+            for (int o = 1; o < 32; o <<= 1) {
+                const bool more = lane - o >= start;
+                if (!__any_sync(kFull, in && more)) break;  // no run is longer than o
+                const double y = __shfl_up_sync(kFull, a, o), z = __shfl_up_sync(kFull, b, o);
+                if (more) {
+                    a += y;
+                    b += z;
+                }
+            }
+            if (!starts) {
+                a += run1;
+                b += run2;
+            }
+            const bool ends = next != key || e + 1 >= n, before = joined && !starts;
+            const bool goes_on = !ends && e + 1 == c1;
+            if (__any_sync(kFull, in && before && ends)) parts |= 1;
+            if (__any_sync(kFull, in && before && goes_on)) parts |= 2;
+            if (__any_sync(kFull, in && !before && goes_on)) parts |= 4;
+            if (in && before && (ends || goes_on)) {
+                mine[2] = a;
+                mine[3] = b;
+                if (ends) s_dg[2 * wid + 1] = key;
+            } else if (in && ends) {
+                add_run(key, a, b);
+            } else if (in && goes_on) {
+                mine[4] = a;
+                mine[5] = b;
+            }
+            joined = joined && all_starts == 0;
+            run1 = __shfl_sync(kFull, a, 31);
+            run2 = __shfl_sync(kFull, b, 31);
+            run_key = __shfl_sync(kFull, key, 31);
+        }
+        const double2 gh = warp_sum_of_two(g, h);
+        if (lane == 0) {
+            mine[0] = gh.x;
+            mine[1] = gh.y;
+            s_dg[2 * wid] = parts;
+        }
+        workers_barrier();
+        if (!takes) return gh;
+        g = h = 0.0;
+        if (lane < kWindow) {  // lane w: warp w
+            if (s_dg[2 * lane] & 1) {
+                double a = s_dd[6 * lane + 2], b = s_dd[6 * lane + 3];
+                for (int w = lane - 1; w >= 0; --w) {
+                    const bool on = s_dg[2 * w] & 2;
+                    a += s_dd[6 * w + (on ? 2 : 4)];
+                    b += s_dd[6 * w + (on ? 3 : 5)];
+                    if (!on) break;
+                }
+                add_run(s_dg[2 * lane + 1], a, b);
+            }
+            g += s_dd[6 * lane];
+            h += s_dd[6 * lane + 1];
+        }
+        return warp_sum_of_two(g, h);
     };
 
     // a worker's groups [ga, gz), and how far the scans over them reach
@@ -468,13 +578,23 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
             ahead.done();
             unsigned moved_on = 0;  // the slots that took up a new column in the last round
             int width = kNarrow;
-            Turn t{0, min(width, n_active), 0, 0};
-            auto show_turn = [&]() {
+            Turn t{0, 0, 0, 0};
+            // what is in flight next, up to the next long column
+            auto next_turn = [&]() {
+                t.base = __reduce_min_sync(kFull, q);
+                t.limit = min(t.base + width, n_active);
+                if (LONG) {
+                    const int first = __reduce_min_sync(kFull, q < n_active && long_column(rec_of(q)) ? q : 0x7fffffff);
+                    t.alone = first == t.base;
+                    t.limit = t.alone ? t.base + 1 : min(t.limit, first);
+                }
                 if (me != 0 || lane != 0) return;
                 s_turn.base = t.base;
                 s_turn.limit = t.limit;
+                if (LONG) s_turn.alone = t.alone;
             };
-            show_turn();
+            if (LONG) __syncthreads();  // every helper's records
+            next_turn();
             __syncthreads();
             for (;;) {
                 if (t.base >= n_active) break;
@@ -490,7 +610,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 }
                 ++n_xch;
                 __syncthreads();
-                if (s_delta[kWindow] != 0.0) break;
+                const bool quit = s_delta[kWindow] != 0.0;
                 // ---- every column up to the first that moves is behind us
                 const unsigned to = __reduce_min_sync(kFull, flying && s_delta[lane & (kWindow - 1)] != 0.0 ? (unsigned)q : 0xffffffffu);
                 const bool moves = to != 0xffffffffu;
@@ -501,12 +621,10 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 if (COX && moves && Q.meet) n_xch += 2;
                 moved += moves;
                 ++rounds;
-                t.base = __reduce_min_sync(kFull, q);
-                t.limit = min(t.base + width, n_active);
-                show_turn();
+                next_turn();
                 ahead.done();
                 __syncthreads();
-                if (s_turn.stop) break;
+                if (quit | (s_turn.stop != 0)) break;
             }
             ahead.done();
         } else {
@@ -516,6 +634,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
             bool fresh = true;
             int ck = 0, cg = -1, ckey = 0x7fffffff;
             double cx = 1.0;
+            if (LONG) __syncthreads();
             __syncthreads();
             for (;;) {
                 const Turn now = s_turn;
@@ -523,7 +642,22 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 const bool mine = pos < now.limit;
                 const Rec& r = rec_of(pos);
                 double d = 0.0, hd = 0.0, b0 = 0.0, g = 0.0, h = 0.0;
-                if (mine) {
+                if (LONG && now.alone) {
+                    const double2 gh = gather_alone(rec_of(now.base), now.base, mine);
+                    if (mine) {
+                        b0 = r.bh.x;
+                        hd = r.bh.y;
+                        if (CL) {
+                            if (lane < C) {
+                                const unsigned par = n_xch & 1;
+                                send16(to_part + (par * kWindow + wid) * kColumnBytes + rank * (unsigned)sizeof(double2), to_bar + par * 8u,
+                                       gh.x, gh.y);
+                            }
+                        } else if (lane == 0) {
+                            __stcg(Q.part + ((size_t)((n_xch & 1) * kWindow + wid) * C + rank) * 3, gh);
+                        }
+                    }
+                } else if (mine) {
                     // ---- the column's sums over this CTA's slice
                     const int n = r.e.hi - r.e.lo;
                     const bool ind = r.c.flags & 4;
@@ -770,12 +904,13 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 __syncthreads();
                 // ---- every step up to the first that is not zero stands
                 int to;
+                bool quit;
                 {
                     const int slot = lane < kWindow ? (now.base + lane) & (kWindow - 1) : kWindow;
                     const bool here = lane < kWindow ? now.base + lane < now.limit : lane == kWindow;
                     const unsigned nz = __ballot_sync(kFull, here & (s_delta[slot] != 0.0));
-                    if (nz >> kWindow) break;
-                    to = nz ? now.base + __ffs(nz) - 1 : 0x7fffffff;
+                    quit = nz >> kWindow;
+                    to = nz - 1 < (1u << kWindow) - 1 ? now.base + __ffs(nz) - 1 : 0x7fffffff;
                 }
                 if (mine && pos <= to) {
                     if (rank == 0 && lane == 0) {  // the bound, and the coefficient where the step moved it
@@ -793,7 +928,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                     const Rec& mv = rec_of(to);
                     const double delta = s_delta[to & (kWindow - 1)];
                     const int n = mv.e.hi - mv.e.lo;
-                    if (n <= 32 && !P.weighted) {  // the column's own warp, which has its entries at hand
+                    if (n <= 32 && !P.weighted && !long_column(mv)) {  // the column's own warp, which has its entries at hand
                         if (wid == (to & (kWindow - 1))) {
                             double change = 0.0;
                             if (lane < n) {
@@ -955,6 +1090,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                     }
                 }
                 __syncthreads();
+                if (quit) break;
             }
         }
         gave_up = s_delta[kWindow] != 0.0 || s_turn.stop;
@@ -983,8 +1119,8 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
     }
 }
 
-__global__ void window_slices_kernel(const int32_t* rows, const WinCol* cols, int32_t n_active, const GroupCut* cuts, int ctas,
-                                     WinSlice* slices) {
+__global__ void window_slices_kernel(const int32_t* rows, WinCol* cols, int32_t n_active, const GroupCut* cuts, int ctas,
+                                     int32_t mark_long, WinSlice* slices) {
     const int64_t total = (int64_t)n_active * ctas;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int r = (int)(i / n_active);
@@ -1005,23 +1141,29 @@ __global__ void window_slices_kernel(const int32_t* rows, const WinCol* cols, in
             s.hi = find(k1);
         }
         slices[i] = s;
+        if (mark_long && s.hi - s.lo > kGroupLong)  // flags: the upper half of the word
+            atomicOr(reinterpret_cast<unsigned*>(&cols[i % n_active].conflict), 8u << 16);
     }
 }
 
 using Kernel = void (*)(GroupWindowParams);
 
-template <bool COX, bool CL, bool MX>
+template <bool COX, bool CL, bool MX, bool LONG>
 Kernel pick(int where) {
     switch (where) {
-    case kRowsShared: return group_window_kernel<COX, kRowsShared, CL, MX>;
-    case kGroupsShared: return group_window_kernel<COX, kGroupsShared, CL, MX>;
-    default: return group_window_kernel<COX, kGlobal, CL, MX>;
+    case kRowsShared: return group_window_kernel<COX, kRowsShared, CL, MX, LONG>;
+    case kGroupsShared: return group_window_kernel<COX, kGroupsShared, CL, MX, LONG>;
+    default: return group_window_kernel<COX, kGlobal, CL, MX, LONG>;
     }
 }
-Kernel pick(bool cox, int where, bool cl, bool mx) {
-    if (!cox) return cl ? pick<false, true, false>(where) : pick<false, false, false>(where);
-    if (mx) return cl ? pick<true, true, true>(where) : pick<true, false, true>(where);
-    return cl ? pick<true, true, false>(where) : pick<true, false, false>(where);
+// `form`: the mixed precision of Cox, or a grouped model's long columns
+Kernel pick(bool cox, int where, bool cl, bool form) {
+    if (cox) {
+        if (form) return cl ? pick<true, true, true, false>(where) : pick<true, false, true, false>(where);
+        return cl ? pick<true, true, false, false>(where) : pick<true, false, false, false>(where);
+    }
+    if (form) return cl ? pick<false, true, false, true>(where) : pick<false, false, false, true>(where);
+    return cl ? pick<false, true, false, false>(where) : pick<false, false, false, false>(where);
 }
 
 constexpr int64_t kStagedRows = 2 * kWindow * kStage * sizeof(int32_t);
@@ -1088,7 +1230,7 @@ cudaError_t group_window_limits(GroupWindowLimits* w) {
                 cudaLaunchAttribute at[1];
                 const cudaLaunchConfig_t cfg = config(C, (size_t)w->smem[1 + cox], 0, at);
                 int n = 0;
-                fits &= cudaOccupancyMaxActiveClusters(&n, pick(cox != 0, where, true, false), &cfg) == cudaSuccess && n >= 1;
+                fits &= cudaOccupancyMaxActiveClusters(&n, pick(cox != 0, where, true, cox == 0), &cfg) == cudaSuccess && n >= 1;
             }
         cudaGetLastError();  // a size the device rejects is not an error here: try the next
         if (fits) {
@@ -1099,11 +1241,11 @@ cudaError_t group_window_limits(GroupWindowLimits* w) {
     return cudaSuccess;
 }
 
-cudaError_t launch_window_slices(const int32_t* rows, const WinCol* cols, int32_t n_active, const GroupCut* cuts, int ctas,
-                                 WinSlice* slices, cudaStream_t stream) {
+cudaError_t launch_window_slices(const int32_t* rows, WinCol* cols, int32_t n_active, const GroupCut* cuts, int ctas,
+                                 bool mark_long, WinSlice* slices, cudaStream_t stream) {
     const int64_t total = (int64_t)n_active * ctas;
     window_slices_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 4096)), 256, 0, stream>>>(
-        rows, cols, n_active, cuts, ctas, slices);
+        rows, cols, n_active, cuts, ctas, mark_long ? 1 : 0, slices);
     return cudaGetLastError();
 }
 
@@ -1128,7 +1270,7 @@ cudaError_t launch_group_window(const GroupWindowParams& Q, bool cluster, int64_
     GroupWindowParams R = Q;
     R.vals_at = (int32_t)(kStagedRows + state);
     const size_t bytes = (size_t)(R.vals_at + vals);
-    const Kernel fn = pick(Q.cox != 0, where, cluster, Q.P.mixed != 0);
+    const Kernel fn = pick(Q.cox != 0, where, cluster, Q.cox ? Q.P.mixed != 0 : Q.any_long != 0);
     if (cluster) {
         cudaLaunchAttribute at[1];
         const cudaLaunchConfig_t cfg = config(C, bytes, stream, at);

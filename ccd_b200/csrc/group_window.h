@@ -13,6 +13,7 @@
 namespace ccdb {
 
 constexpr int kGroupWindowCtas = 160;  // most CTAs of the grid form
+constexpr int64_t kGroupLong = 512;    // a column with a larger slice runs alone (grouped models)
 
 // What one CTA owns: rows [row0, next row0) and groups [g0, next g0); a sentinel
 // follows the last CTA's.  Strata (Cox): `first` and `last` are those of its
@@ -43,6 +44,7 @@ struct GroupWindowParams {
     double tol;
     double ll_fixed;
     int32_t any_vals;  // some active column has values
+    int32_t any_long;  // some may be marked long (grouped models)
     int32_t meet;      // Cox: a stratum spans CTAs, which then exchange tail and head sums
     int32_t chain;     // lanes that a carry may pass over (1 + the CTAs within one stratum in a row)
     int32_t vals_at;   // where the staged values lie in shared memory (the launcher's)
@@ -66,9 +68,10 @@ struct GroupWindowLimits {
 cudaError_t group_window_limits(GroupWindowLimits* w);
 // Whether the groups that one of `ctas` CTAs owns fit in `smem` bytes.
 bool group_window_fits(bool cox, int64_t groups, int ctas, bool vals, int64_t smem);
-// Entry ranges of every column that each CTA owns, from the CTAs' first rows.
-cudaError_t launch_window_slices(const int32_t* rows, const WinCol* cols, int32_t n_active, const GroupCut* cuts,
-                                 int ctas, WinSlice* slices, cudaStream_t stream);
+// Entry ranges of every column that each CTA owns, from the CTAs' first rows; with
+// `mark_long`, a column of which a CTA owns more than kGroupLong entries is marked.
+cudaError_t launch_window_slices(const int32_t* rows, WinCol* cols, int32_t n_active, const GroupCut* cuts,
+                                 int ctas, bool mark_long, WinSlice* slices, cudaStream_t stream);
 // `most_rows`, `most_groups`: the most that one CTA owns.
 cudaError_t launch_group_window(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
                                 cudaStream_t stream);

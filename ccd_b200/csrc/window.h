@@ -2,6 +2,7 @@
 // plan that it walks (window_plan.cpp).
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <vector>
 
@@ -27,7 +28,8 @@ struct WinCol {
     uint16_t conflict, flags;
     int32_t pad;
 };
-static_assert(sizeof(WinCol) == 32, "WinCol layout");
+static_assert(sizeof(WinCol) == 32 && offsetof(WinCol, conflict) % 4 == 0 &&
+                  offsetof(WinCol, flags) == offsetof(WinCol, conflict) + 2, "WinCol layout");
 
 // Half-open range of a column's entries (of rows, for DENSE and INTERCEPT
 // columns) that one CTA owns.
