@@ -111,6 +111,16 @@ struct DevSchedule {
     double2* partials = nullptr;
 };
 
+// Parts of one allocation, each on a boundary of 256 bytes.
+struct Parts {
+    size_t bytes = 0;
+    size_t add(size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    }
+};
+
 // The plan of a windowed sweep on the device, and its per-position state.
 struct DevWindow {
     std::vector<uint8_t> fixed;
@@ -158,7 +168,8 @@ struct CoxDev {
     int64_t grouping = 0;  // changes when the rows are regrouped
     // Cox: runs of groups that end with events or with their stratum, the grouping
     // that the windowed sweep works on (block_rows); NB of them
-    int64_t NB = 0;
+    int64_t NB = 0, blocks = -1;  // the grouping that they belong to
+    void* block_mem = nullptr;    // what holds them all
     int32_t *blk = nullptr, *bgrp = nullptr;  // block of each row, first group of each block
     double *bden = nullptr, *bD = nullptr, *bS1 = nullptr, *bS2 = nullptr, *bnev = nullptr;
     uint8_t *bfirst = nullptr, *blast = nullptr;
@@ -217,6 +228,11 @@ struct Fit {
     std::vector<int32_t> pid0_h;
     std::vector<int64_t> cox_grow_h;    // first row of each stratum (grouped) or block (Cox), then K
     std::vector<int32_t> cox_bstrat_h;  // Cox: stratum of each block
+    struct {  // Cox: the group of each row (N: none); stratum, first row and weighted events of each group
+        std::vector<int32_t> row_group, stratum;
+        std::vector<int64_t> first_row;
+        std::vector<double> events;
+    } cox_groups_h;
     std::vector<int32_t> ptype_h;
     std::vector<uint8_t> fixed;
     bool weighted = false;
@@ -279,6 +295,7 @@ struct Fit {
     void cox_update(int j, double delta);
     // one findMode of the group engine in one launch (group_window.cu), and its plan
     void ensure_group_window(int ctas, bool cluster);
+    void ensure_cox_blocks();
     void find_mode_group_window(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms);
     // mode-finding variants (modes_host.cu): the MM cycle, the KKT swindle, and
     // the MM all-coordinate (g, h) into out[J] (fixed may be nullptr)
