@@ -114,6 +114,12 @@ int64_t Matrix::entries(int j) const {
     return col_start[j + 1] - col_start[j];
 }
 
+int64_t Matrix::total_entries() const {
+    int64_t total = 0;
+    for (int j = 0; j < J; ++j) total += entries(j);
+    return total;
+}
+
 Matrix::~Matrix() {
     for (void* p : {(void*)d_col_ptr, (void*)d_rows, (void*)d_val_ptr, (void*)d_vals, (void*)d_fmt,
                     (void*)d_row_ptr, (void*)d_csr_col, (void*)d_csr_val})
@@ -126,8 +132,7 @@ Matrix::~Matrix() {
 // entries is built on the host threads instead (csr_host.cpp, the same layout).
 void Matrix::ensure_csr(cudaStream_t s) {
     if (d_row_ptr) return;
-    int64_t total = 0;
-    for (int j = 0; j < J; ++j) total += entries(j);
+    const int64_t total = total_entries();
     CsrDeviceArgs a{K, J, d_col_ptr, d_rows, d_val_ptr, d_vals, d_fmt, val_start.back() > 0};
     auto* counts = static_cast<int32_t*>(ctx->alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(K, 1)));
     auto* cursor = static_cast<int64_t*>(ctx->alloc(sizeof(int64_t) * (size_t)std::max<int64_t>(K, 1)));

@@ -93,6 +93,7 @@ struct Matrix {
     double* d_csr_val = nullptr;
 
     int64_t entries(int j) const;
+    int64_t total_entries() const;
     // values of the row-major copy; NULL where every one is 1
     const double* csr_values() const { return val_start.back() > 0 ? d_csr_val : nullptr; }
     void ensure_csr(cudaStream_t s);

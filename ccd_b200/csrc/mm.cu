@@ -18,13 +18,20 @@ namespace {
 
 constexpr int kMT = 256;
 
+__device__ __forceinline__ double mm_share(const MMParams& P, int32_t grp, int64_t k) {
+    return P.nEv[grp] * P.xbe[k].y / P.denom[grp];
+}
+
 __global__ void __launch_bounds__(kMT) mm_share_kernel(MMParams P) {
     for (int64_t k = (int64_t)blockIdx.x * kMT + threadIdx.x; k < P.K; k += (int64_t)gridDim.x * kMT) {
         const int32_t grp = P.grp[k];
-        P.share[k] = P.nEv[grp] * P.xbe[k].y / P.denom[grp];
+        P.share[k] = mm_share(P, grp, k);
     }
 }
 
+// Small calls, and matrices with few entries for their rows, work the share out for
+// each entry: the launch before costs 3 us of some 30 (8 columns of 200 entries,
+// 20,000 rows: 28 us, with it 33; of 30,000 entries, 300,000 rows: 137 and 100).
 // incrementMMGradientAndHessian of the Survival models (ModelSpecifics.h:499-516,
 // the conditional and Cox models): weight = hNWeight and denominator =
 // denomPid of the row's group; indicator columns drop x.  Latency of the gathers:
@@ -46,7 +53,7 @@ __global__ void __launch_bounds__(kMT) mm_gh_kernel(MMParams P) {
 #pragma unroll 4
     for (int64_t p = threadIdx.x; p < n; p += kMT) {
         const int64_t k = has_rows ? (int64_t)__ldg(P.rows + cb + p) : p;
-        const double r = P.share[k];
+        const double r = P.share ? P.share[k] : mm_share(P, P.grp[k], k);
         if (ind) {
             g += r;
             h += r;
@@ -73,7 +80,7 @@ __global__ void __launch_bounds__(kMT) mm_gh_kernel(MMParams P) {
 cudaError_t launch_mm_gradient_hessian(const MMParams& P, cudaStream_t s) {
     if (P.J <= 0) return cudaSuccess;
     const int64_t blocks = (P.K + kMT - 1) / kMT;
-    mm_share_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), kMT, 0, s>>>(P);
+    if (P.share) mm_share_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), kMT, 0, s>>>(P);
     mm_gh_kernel<<<P.J, kMT, 0, s>>>(P);
     return cudaGetLastError();
 }

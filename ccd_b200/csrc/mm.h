@@ -23,7 +23,8 @@ struct MMParams {
     const int32_t* grp;
     const double* nEv;
     const double* denom;
-    double* share;         // K, scratch: events x offsExpXBeta / denominator of each row
+    double* share;         // K, scratch: events x offsExpXBeta / denominator of each row; nullptr:
+                           // worked out for each entry
     const double* xjy;
     const uint8_t* fixed;  // J flags (nullptr: none)
     // per column
@@ -33,7 +34,9 @@ struct MMParams {
     double2* gh;           // J outputs {gradient, Hessian bound}
 };
 
-// The rows' shares, then one CTA per column: the MM (gradient, Hessian bound), and with P.step the
+constexpr bool mm_shares_pay(int64_t entries, int64_t rows) { return entries > 4096 && 8 * entries >= rows; }
+
+// The rows' shares (if any), then one CTA per column: the MM (gradient, Hessian bound), and with P.step the
 // prior's step added to beta (no trust-region bound, as the reference's MM).
 cudaError_t launch_mm_gradient_hessian(const MMParams& P, cudaStream_t s);
 

@@ -51,9 +51,9 @@ void Fit::mm_gradient_hessian(const uint8_t* fixed_flags, double2* out) {
         P.ptype = ptype;
         P.pvar = pvar;
         P.gh = d_gh;
-        P.share = xb_tmp;  // free: no xBeta is pending
+        P.share = mm_shares_pay(m->total_entries(), K) ? xb_tmp : nullptr;  // free: no xBeta is pending
         check_cuda(launch_mm_gradient_hessian(P, stream), "mm gradient");
-        launches += 2;
+        launches += P.share ? 2 : 1;
         check_cuda(cudaMemcpyAsync(out, d_gh, sizeof(double2) * J, cudaMemcpyDeviceToHost, stream), "mm copy");
         check_cuda(ctx->wait(), "mm sync");
     } catch (...) {
@@ -114,7 +114,7 @@ void Fit::find_mode_mm(const ccdb_mode_args& a, int* flag, int* iters, double* o
         P.ptype = ptype;
         P.pvar = pvar;
         P.gh = d_gh;
-        P.share = xb_tmp;  // free until the cycle's xBeta is written
+        P.share = mm_shares_pay(m->total_entries(), K) ? xb_tmp : nullptr;  // free until the cycle's xBeta is written
         double t[4];
         objective_terms(t);
         double last = conv_objective(t, ll_fixed, a.convergence_type);
@@ -127,7 +127,7 @@ void Fit::find_mode_mm(const ccdb_mode_args& a, int* flag, int* iters, double* o
             P.nEv = cox.nEv;
             P.denom = cox.denom;
             check_cuda(launch_mm_gradient_hessian(P, stream), "mm step");
-            launches += 2;
+            launches += P.share ? 2 : 1;
             compute_xbeta_transpose();
             remaining_statistics();
             download_beta();
