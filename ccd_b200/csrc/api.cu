@@ -706,11 +706,27 @@ int Fit::window_ctas() {
 
 void Fit::release_window() {
     if (!window) return;
-    for (void* p : {(void*)window->cols, (void*)window->slices, (void*)window->scal,
-                    (void*)window->bh, (void*)window->share, (void*)window->cuts, (void*)window->part,
-                    (void*)window->tails, (void*)window->heads})
-        ctx->release(p);
+    ctx->release(window->mem);
     window.reset();
+}
+
+// The memory of a plan, and its two parts that the host has made.  Those of a small
+// plan are at the front and go up in one copy: a call of few columns had spent 8 us
+// on an allocation a part and two copies.  (A copy from pageable memory has read it
+// when the call returns.)
+void Fit::place_window(size_t bytes, PlanPart a, PlanPart b) {
+    window->mem = ctx->alloc(bytes);
+    char* const d = static_cast<char*>(window->mem);
+    const size_t front = b.at + b.bytes;
+    if (a.at == 0 && front <= 65536) {
+        std::vector<char> host(front);
+        std::memcpy(host.data(), a.host, a.bytes);
+        std::memcpy(host.data() + b.at, b.host, b.bytes);
+        check_cuda(cudaMemcpyAsync(d, host.data(), front, cudaMemcpyHostToDevice, stream), "sweep plan upload");
+        return;
+    }
+    check_cuda(cudaMemcpyAsync(d + a.at, a.host, a.bytes, cudaMemcpyHostToDevice, stream), "sweep plan upload");
+    check_cuda(cudaMemcpyAsync(d + b.at, b.host, b.bytes, cudaMemcpyHostToDevice, stream), "sweep plan upload");
 }
 
 void Fit::ensure_window(int ctas) {
@@ -721,14 +737,19 @@ void Fit::ensure_window(int ctas) {
     window.reset(new DevWindow());  // owned by the fit from here on, complete or not
     window->ctas = 0;               // not a plan to reuse until it is complete
     const size_t n = plan.cols.size();
-    window->cols = upload(ctx, plan.cols.data(), n, stream);
-    window->slices = upload(ctx, plan.slices.data(), plan.slices.size(), stream);
-    window->scal = static_cast<WinScal*>(ctx->alloc(sizeof(WinScal) * n));
-    window->bh = static_cast<double2*>(ctx->alloc(sizeof(double2) * n));
     for (const WinCol& c : plan.cols) window->any_vals |= (c.flags & 2) != 0;
-    if (!window_share_fits((K + ctas - 1) / ctas, window->any_vals, ctx->window_smem))
-        window->share = static_cast<double*>(ctx->alloc(sizeof(double) * K));
-    check_cuda(ctx->wait(), "sweep plan upload");
+    const bool share = !window_share_fits((K + ctas - 1) / ctas, window->any_vals, ctx->window_smem);
+    const size_t col_bytes = sizeof(WinCol) * n, slice_bytes = sizeof(WinSlice) * plan.slices.size();
+    Parts p;
+    const size_t at_cols = p.add(col_bytes), at_slices = p.add(slice_bytes), at_scal = p.add(sizeof(WinScal) * n),
+                 at_bh = p.add(sizeof(double2) * n), at_share = p.add(share ? sizeof(double) * K : 0);
+    place_window(p.bytes, {at_cols, col_bytes, plan.cols.data()}, {at_slices, slice_bytes, plan.slices.data()});
+    char* const d = static_cast<char*>(window->mem);
+    window->cols = reinterpret_cast<WinCol*>(d + at_cols);
+    window->slices = reinterpret_cast<WinSlice*>(d + at_slices);
+    window->scal = reinterpret_cast<WinScal*>(d + at_scal);
+    window->bh = reinterpret_cast<double2*>(d + at_bh);
+    window->share = share ? reinterpret_cast<double*>(d + at_share) : nullptr;
     window->n_active = (int32_t)n;
     window->fixed = fixed;
     window->ctas = ctas;

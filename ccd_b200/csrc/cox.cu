@@ -466,8 +466,12 @@ cudaError_t launch_cox_update(const CoxParams& P, int j, double delta, cudaStrea
     return cudaGetLastError();
 }
 
-cudaError_t launch_cox_remaining(const CoxParams& P, const double* fresh, cudaStream_t s) {
+cudaError_t launch_cox_exp(const CoxParams& P, const double* fresh, cudaStream_t s) {
     cox_exp_kernel<<<1184, 256, 0, s>>>(P, fresh);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_cox_denominators(const CoxParams& P, cudaStream_t s) {
     cox_denom_kernel<<<1184, 256, 0, s>>>(P);
     return cudaGetLastError();
 }
@@ -498,8 +502,7 @@ cudaError_t launch_grouped_update(const CoxParams& P, int j, double delta, cudaS
     return cudaGetLastError();
 }
 
-cudaError_t launch_grouped_remaining(const CoxParams& P, const double* fresh, cudaStream_t s) {
-    cox_exp_kernel<<<1184, 256, 0, s>>>(P, fresh);
+cudaError_t launch_grouped_denominators(const CoxParams& P, cudaStream_t s) {
     grouped_denom_kernel<<<1184, 256, 0, s>>>(P);
     return cudaGetLastError();
 }

@@ -45,7 +45,9 @@ size_t cox_tail_bytes();
 cudaError_t launch_cox_gh(const CoxParams& P, const int32_t* cols, int ncols, double2* out,
                           cudaStream_t s);
 cudaError_t launch_cox_update(const CoxParams& P, int j, double delta, cudaStream_t s);
-cudaError_t launch_cox_remaining(const CoxParams& P, const double* fresh, cudaStream_t s);
+// e = exp(xBeta) of every row, of both kinds of model; then the denominators
+cudaError_t launch_cox_exp(const CoxParams& P, const double* fresh, cudaStream_t s);
+cudaError_t launch_cox_denominators(const CoxParams& P, cudaStream_t s);
 // D from denom, then S1/S2 from D (two single-pass look-back scans); `epoch`
 // must differ from every earlier call on the same status arrays.
 cudaError_t launch_cox_scans(const CoxParams& P, unsigned* tickets, int* status, void* tails,
@@ -61,7 +63,7 @@ cudaError_t launch_cox_objective(const CoxParams& P, double2* red, int nblocks, 
 cudaError_t launch_grouped_gh(const CoxParams& P, const int32_t* cols, int ncols, double2* out,
                               cudaStream_t s);
 cudaError_t launch_grouped_update(const CoxParams& P, int j, double delta, cudaStream_t s);
-cudaError_t launch_grouped_remaining(const CoxParams& P, const double* fresh, cudaStream_t s);
+cudaError_t launch_grouped_denominators(const CoxParams& P, cudaStream_t s);
 cudaError_t launch_grouped_objective(const CoxParams& P, double2* red, int nblocks, cudaStream_t s);
 
 }  // namespace ccdb

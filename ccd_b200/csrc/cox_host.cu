@@ -290,7 +290,6 @@ void Fit::ensure_cox_blocks() {
     cox.bS2 = reinterpret_cast<double*>(d + at[3]);
     cox_grow_h.assign(brow, brow + NB + 1);
     cox_bstrat_h = std::move(bstrat);
-    check_cuda(ctx->wait(), "blocks");  // the host's copy may go
     cox.NB = NB;
     cox.blocks = cox.grouping;
 }
@@ -304,13 +303,18 @@ void Fit::cox_scans() {
 }
 
 // computeRemainingStatistics (ModelSpecifics.hpp:1588-1617) + the accumulated scans.
-void Fit::cox_remaining() {
+// `rows_done`: the rows' exp(xBeta) belongs to their xBeta, as a sweep leaves it.
+void Fit::cox_remaining(bool rows_done) {
     const double* const fresh = xb_pending ? xb_tmp : nullptr;  // xBeta computed into xb_tmp
     xb_pending = false;
     CoxParams P = cox_params();
-    if (is_cox()) check_cuda(launch_cox_remaining(P, fresh, stream), "cox remaining");
-    else check_cuda(launch_grouped_remaining(P, fresh, stream), "grouped remaining");
-    launches += 2;
+    if (!rows_done || fresh) {
+        check_cuda(launch_cox_exp(P, fresh, stream), "exp");
+        ++launches;
+    }
+    if (is_cox()) check_cuda(launch_cox_denominators(P, stream), "cox remaining");
+    else check_cuda(launch_grouped_denominators(P, stream), "grouped remaining");
+    ++launches;
     cox_scans();
     suff_known = true;
 }
@@ -439,26 +443,28 @@ void Fit::ensure_group_window(int ctas, bool cluster) {
         }
     }
     const size_t n = cols.size();
-    auto upload = [&](const void* h, size_t bytes) {
-        void* d = ctx->alloc(bytes);
-        check_cuda(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, stream), "sweep plan upload");
-        return d;
-    };
-    window->cols = static_cast<WinCol*>(upload(cols.data(), sizeof(WinCol) * n));
-    window->cuts = static_cast<GroupCut*>(upload(cuts.data(), sizeof(GroupCut) * cuts.size()));
-    window->slices = static_cast<WinSlice*>(ctx->alloc(sizeof(WinSlice) * n * ctas));
-    window->scal = static_cast<WinScal*>(ctx->alloc(sizeof(WinScal) * n));
-    window->bh = static_cast<double2*>(ctx->alloc(sizeof(double2) * n));
+    const size_t col_bytes = sizeof(WinCol) * n, cut_bytes = sizeof(GroupCut) * cuts.size(), grid = cluster ? 0 : 2 * ctas;
+    Parts p;
+    const size_t at_cols = p.add(col_bytes), at_cuts = p.add(cut_bytes), at_slices = p.add(sizeof(WinSlice) * n * ctas),
+                 at_scal = p.add(sizeof(WinScal) * n), at_bh = p.add(sizeof(double2) * n),
+                 at_part = p.add(sizeof(double2) * kWindow * 3 * grid), at_tails = p.add(sizeof(double) * grid),
+                 at_heads = p.add(sizeof(double2) * grid);
+    place_window(p.bytes, {at_cols, col_bytes, cols.data()}, {at_cuts, cut_bytes, cuts.data()});
+    char* const d = static_cast<char*>(window->mem);
+    window->cols = reinterpret_cast<WinCol*>(d + at_cols);
+    window->cuts = reinterpret_cast<GroupCut*>(d + at_cuts);
+    window->slices = reinterpret_cast<WinSlice*>(d + at_slices);
+    window->scal = reinterpret_cast<WinScal*>(d + at_scal);
+    window->bh = reinterpret_cast<double2*>(d + at_bh);
     if (!cluster) {
-        window->part = static_cast<double2*>(ctx->alloc(sizeof(double2) * 2 * kWindow * ctas * 3));
-        window->tails = static_cast<double*>(ctx->alloc(sizeof(double) * 2 * ctas));
-        window->heads = static_cast<double2*>(ctx->alloc(sizeof(double2) * 2 * ctas));
+        window->part = reinterpret_cast<double2*>(d + at_part);
+        window->tails = reinterpret_cast<double*>(d + at_tails);
+        window->heads = reinterpret_cast<double2*>(d + at_heads);
     }
     check_cuda(launch_window_slices(m->d_rows, window->cols, (int32_t)n, window->cuts, ctas, window->any_long, window->slices,
                                     stream),
                "sweep plan");
     ++launches;
-    check_cuda(ctx->wait(), "sweep plan");
     window->n_active = (int32_t)n;
     window->fixed = fixed;
     window->grouping = cox.grouping;
@@ -571,7 +577,7 @@ void Fit::find_mode_group_window(const ccdb_mode_args& a, int* flag, int* iters,
     check_cuda(launch_group_window(Q, use_cluster, window->most_rows, window->most_groups, stream), "group sweep launch");
     ++launches;
     check_cuda(cudaEventRecord(ctx->fev[1], stream), "event");
-    if (is_cox()) cox_remaining();  // the groups' own denominators and sums, for the calls that follow
+    if (is_cox()) cox_remaining(true);  // the groups' own denominators and sums, for the calls that follow
     check_cuda(ctx->wait(), "group sweep");  // the sweep is done before a copy is queued behind it
     DevStatus out{};
     int64_t cnt[2] = {0, 0};

@@ -132,6 +132,7 @@ struct DevWindow {
     int32_t n_long = 0, team = 1;
     int64_t entries = 0;
     int32_t* longs = nullptr;
+    void* mem = nullptr;  // what holds all of the following
     WinCol* cols = nullptr;
     WinSlice* slices = nullptr;
     WinScal* scal = nullptr;
@@ -272,6 +273,11 @@ struct Fit {
     int window_ctas();
     void ensure_window(int ctas);
     void release_window();
+    struct PlanPart {
+        size_t at, bytes;
+        const void* host;
+    };
+    void place_window(size_t bytes, PlanPart a, PlanPart b);
     int64_t batch_mean() const;  // entries of the columns that a batch steps (batch_route.h)
     void ensure_batch_window();
     void release_batch_window();
@@ -290,7 +296,7 @@ struct Fit {
     void cox_release();
     void cox_apply_weights();
     void cox_scans();
-    void cox_remaining();
+    void cox_remaining(bool rows_done = false);
     void cox_objective_terms(double* out4);
     void cox_gh_batch(const int32_t* cols, int n, double2* out);
     void cox_update(int j, double delta);
