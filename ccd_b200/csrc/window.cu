@@ -141,7 +141,11 @@ struct Rows {
     }
 };
 
-template <int MODEL, int WHERE, bool CL, bool WT>
+// FEW: no more columns than there are records in the buffers, 64; they stay there from
+// cycle to cycle, and the entries of up to 32 columns beside them (a cycle of 30
+// columns of a 1,000-row fit took 25.2 us, now 23.1; chosen when the kernel runs, it
+// cost the fits with more columns 1.5 %).
+template <int MODEL, int WHERE, bool CL, bool WT, bool FEW>
 __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
     __shared__ Rec s_rec[4][kWindow];  // by position: (position / kWindow) & 3, slot
     __shared__ double2 s_pair[2][kWindow][kWindowCluster];  // (g, h) by round parity, column and CTA
@@ -318,25 +322,31 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
             const int me = wid - kWindow;
             int q = lane < kWindow ? lane : 0x7fffffff;  // the slot's position
             const int l8 = lane & 7, mine = me + kHelpers * (lane >> 3);  // eight lanes a slot
-            for (int i = 0; i < 3; ++i) fetch(mine + i * kWindow, l8);
-            ahead.done();
-            stage(mine, l8);
-            stage(mine + kWindow, l8);
-            ahead.done();
+            const bool fetches = !FEW || iteration == 0;
+            const bool stages = !FEW || iteration == 0 || n_active > 2 * kWindow;
+            if (fetches) {
+                for (int i = 0; i < 3; ++i) fetch(mine + i * kWindow, l8);
+                ahead.done();
+            }
+            if (stages) {
+                stage(mine, l8);
+                stage(mine + kWindow, l8);
+                ahead.done();
+            }
             unsigned moved_on = 0;  // the slots that took up a new column in the last round
             int par = 0;
             // the bound of a column whose step was taken in the last round, and its
             // coefficient where the step moved it (lane l: slot l), off the warps' path
             auto settle = [&]() {
-                if (rank != 0 || me != kHelpers - 1 || !(moved_on >> lane & 1u)) return;
-                const Rec& r = rec_of(q - kWindow);
+                if ((rank != 0 && !FEW) || me != kHelpers - 1 || !(moved_on >> lane & 1u)) return;
+                Rec& r = rec_of(q - kWindow);
                 const double d = s_delta[par ^ 1][lane];
                 double2 bh = r.bh;
                 apply_bounds(d, bh.y);
-                if (d != 0.0) {
-                    bh.x += d;
-                    P.beta[r.c.j] = bh.x;
-                }
+                if (d != 0.0) bh.x += d;
+                if (FEW) r.bh = bh;
+                if (rank != 0) return;
+                if (d != 0.0) P.beta[r.c.j] = bh.x;
                 R.bh[q - kWindow] = bh;
             };
             Turn t{0, 0, 0, 0};
@@ -385,8 +395,8 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 }
                 const int at = __shfl_sync(kFull, q, mine);
                 if (moved_on >> mine & 1u) {
-                    stage(at + kWindow, l8);
-                    fetch(at + 2 * kWindow, l8);
+                    if (stages) stage(at + kWindow, l8);
+                    if (fetches) fetch(at + 2 * kWindow, l8);
                 }
                 settle();
                 if (CL) ++n_xch;
@@ -519,35 +529,29 @@ constexpr int64_t kStagedVals = 2 * kWindow * kStage * sizeof(double);
 
 using Kernel = void (*)(WindowParams);
 
+// Few columns have a kernel of their own where the rows are few too and have no
+// weights: a process's first fit loads them all, 0.3 ms each.
 template <int MODEL, int WHERE>
-Kernel pick(bool cl, bool wt) {
-    if constexpr (WHERE != kPairShared) {
-        if (cl) return wt ? window_sweep_kernel<MODEL, WHERE, true, true> : window_sweep_kernel<MODEL, WHERE, true, false>;
+Kernel pick(bool cl, bool wt, bool few) {
+    if constexpr (WHERE == kAllShared) {
+        if (few && !wt) return cl ? window_sweep_kernel<MODEL, WHERE, true, false, true> : window_sweep_kernel<MODEL, WHERE, false, false, true>;
     }
-    return wt ? window_sweep_kernel<MODEL, WHERE, false, true> : window_sweep_kernel<MODEL, WHERE, false, false>;
+    if constexpr (WHERE != kPairShared) {
+        if (cl) return wt ? window_sweep_kernel<MODEL, WHERE, true, true, false> : window_sweep_kernel<MODEL, WHERE, true, false, false>;
+    }
+    return wt ? window_sweep_kernel<MODEL, WHERE, false, true, false> : window_sweep_kernel<MODEL, WHERE, false, false, false>;
 }
 template <int MODEL>
-Kernel pick(int where, bool cl, bool wt) {
+Kernel pick(int where, bool cl, bool wt, bool few) {
     switch (where) {
-    case kAllShared: return pick<MODEL, kAllShared>(cl, wt);
-    case kShareShared: return pick<MODEL, kShareShared>(cl, wt);
-    case kGlobal: return pick<MODEL, kGlobal>(cl, wt);
-    default: return pick<MODEL, kPairShared>(false, wt);
+    case kAllShared: return pick<MODEL, kAllShared>(cl, wt, few);
+    case kShareShared: return pick<MODEL, kShareShared>(cl, wt, few);
+    case kGlobal: return pick<MODEL, kGlobal>(cl, wt, few);
+    default: return pick<MODEL, kPairShared>(false, wt, few);
     }
 }
-Kernel pick(int model, int where, bool cl, bool wt) {
-    return model == M_LOGISTIC ? pick<M_LOGISTIC>(where, cl, wt) : pick<M_POISSON>(where, cl, wt);
-}
-
-template <typename F>
-cudaError_t each_kernel(F&& f) {
-    for (int model : {(int)M_LOGISTIC, (int)M_POISSON})
-        for (int where : {(int)kAllShared, (int)kShareShared, (int)kGlobal, (int)kPairShared})
-            for (int v = 0; v < 4; ++v) {
-                const cudaError_t e = f(pick(model, where, v & 1, v & 2));
-                if (e != cudaSuccess) return e;
-            }
-    return cudaSuccess;
+Kernel pick(int model, int where, bool cl, bool wt, bool few) {
+    return model == M_LOGISTIC ? pick<M_LOGISTIC>(where, cl, wt, few) : pick<M_POISSON>(where, cl, wt, few);
 }
 
 cudaError_t smem_limit(int64_t* bytes) {
@@ -558,17 +562,15 @@ cudaError_t smem_limit(int64_t* bytes) {
     return e;
 }
 
-cudaError_t kernel_attrs() {
-    static std::atomic<uint64_t> done{0};
-    return once_per_device(done, [] {
+// A kernel's attributes, set before its first launch on a device.
+cudaError_t kernel_attrs(Kernel fn, int model, int where, bool cl, bool wt, bool few) {
+    static std::atomic<uint64_t> done[2][4][8];
+    return once_per_device(done[model == M_LOGISTIC][where][(cl ? 4 : 0) + (wt ? 2 : 0) + (few ? 1 : 0)], [&] {
         int64_t dyn = 0;
         cudaError_t e = smem_limit(&dyn);
-        if (e != cudaSuccess) return e;
-        return each_kernel([&](Kernel fn) {
-            cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-            if (r != cudaSuccess) return r;
-            return cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        });
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        return e;
     });
 }
 
@@ -597,19 +599,16 @@ bool window_share_fits(int64_t rows, bool vals, int64_t smem) {
 
 cudaError_t window_limits(int* cluster, int64_t* smem) {
     *cluster = 0;
+    // one for all: they have the same threads, and their shared memory is asked for in full
+    const Kernel fn = pick(M_LOGISTIC, kAllShared, true, false, false);
     cudaError_t e = smem_limit(smem);
-    if (e == cudaSuccess) e = kernel_attrs();
+    if (e == cudaSuccess) e = kernel_attrs(fn, M_LOGISTIC, kAllShared, true, false, false);
     if (e != cudaSuccess) return e;
     for (int C = kWindowCluster; C >= 1; C /= 2) {
-        int fits = 1;
-        e = each_kernel([&](Kernel fn) {
-            cudaLaunchAttribute at[1];
-            const cudaLaunchConfig_t cfg = config(C, (size_t)*smem, 0, at);
-            int n = 0;
-            const cudaError_t r = cudaOccupancyMaxActiveClusters(&n, fn, &cfg);
-            fits &= (r == cudaSuccess && n >= 1) ? 1 : 0;
-            return cudaSuccess;
-        });
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = config(C, (size_t)*smem, 0, at);
+        int n = 0;
+        const bool fits = cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n >= 1;
         cudaGetLastError();  // a size the device rejects is not an error here: try the next
         if (fits) {
             *cluster = C;
@@ -622,8 +621,6 @@ cudaError_t window_limits(int* cluster, int64_t* smem) {
 cudaError_t launch_window_sweep(const WindowParams& R, int64_t smem, cudaStream_t stream) {
     const int C = R.cluster;
     if (C < 1 || C > kWindowCluster) return cudaErrorInvalidValue;
-    cudaError_t e = kernel_attrs();
-    if (e != cudaSuccess) return e;
     const int64_t rows = (R.P.K + C - 1) / C;  // the most a CTA owns
     const int64_t vals = R.any_vals ? kStagedVals : 0;
     int where = kGlobal;
@@ -639,7 +636,10 @@ cudaError_t launch_window_sweep(const WindowParams& R, int64_t smem, cudaStream_
         state = 8 * ((rows + 1) & ~int64_t(1));
     }
     if (where == kGlobal && !R.share) return cudaErrorInvalidValue;
-    const Kernel fn = pick(R.P.model, where, C > 1, R.weighted != 0);
+    const bool few = R.n_active <= 4 * kWindow;
+    const Kernel fn = pick(R.P.model, where, C > 1, R.weighted != 0, few);
+    const cudaError_t e = kernel_attrs(fn, R.P.model, where, C > 1, R.weighted != 0, few);
+    if (e != cudaSuccess) return e;
     WindowParams Q = R;
     Q.vals_at = (int32_t)(kStagedRows + state);
     cudaLaunchAttribute at[1];
