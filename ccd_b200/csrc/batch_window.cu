@@ -665,27 +665,24 @@ cudaError_t batch_window_spill(int64_t K, bool mixed, bool vals, int* spill) {
 }
 
 cudaError_t launch_batch_window(const BatchWindowParams& R, cudaStream_t stream) {
-    static std::atomic<uint64_t> done{0};
-    cudaError_t e = once_per_device(done, [] {
-        int64_t dyn = 0;
-        cudaError_t r = smem_limit(&dyn);
-        for (int model : {(int)M_LOGISTIC, (int)M_POISSON})
-            for (int team : {1, 4})
-                for (int v = 0; v < 6 && r == cudaSuccess; ++v)
-                    r = cudaFuncSetAttribute(pick(model, v & 1, v >> 1, team), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)dyn);
-        return r;
-    });
-    if (e != cudaSuccess) return e;
     int where = kNone;
     int64_t state = 0;
-    e = placement(R.P.K, R.mixed != 0, R.any_vals != 0, &where, &state);
+    cudaError_t e = placement(R.P.K, R.mixed != 0, R.any_vals != 0, &where, &state);
     if (e != cudaSuccess) return e;
     if ((where != kBoth && !R.xbeta) || (where == kNone && !R.share)) return cudaErrorInvalidValue;
     BatchWindowParams Q = R;
     Q.vals_at = (int32_t)(kStagedRows + state);
     const size_t smem = (size_t)(Q.vals_at + (R.any_vals ? kStagedVals : 0));
-    pick(R.P.model, R.mixed != 0, where, R.team)<<<R.ctas, kT, smem, stream>>>(Q);
+    const Kernel fn = pick(R.P.model, R.mixed != 0, where, R.team);
+    static std::atomic<uint64_t> done[2][3][4];  // the attribute, before a kernel's first launch on a device
+    e = once_per_device(done[R.P.model == M_LOGISTIC][where][(R.mixed ? 2 : 0) + (R.team == 1 ? 1 : 0)], [&] {
+        int64_t dyn = 0;
+        cudaError_t r = smem_limit(&dyn);
+        if (r == cudaSuccess) r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+        return r;
+    });
+    if (e != cudaSuccess) return e;
+    fn<<<R.ctas, kT, smem, stream>>>(Q);
     return cudaGetLastError();
 }
 

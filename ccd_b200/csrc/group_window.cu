@@ -1173,28 +1173,25 @@ int64_t group_bytes(bool cox, int64_t groups) { return (cox ? 36 : 16) * groups;
 int64_t row_bytes(int64_t rows) { return 20 * rows; }
 int64_t even(int64_t b) { return (b + 15) & ~int64_t(15); }
 
-// Dynamic shared memory that the kernels of a form may hold -- grid, cluster of a
-// grouped model, cluster of Cox -- set once per device.
-cudaError_t kernel_attrs(int64_t smem[3]) {
-    static std::atomic<uint64_t> done{0};
+// Dynamic shared memory that the kernels of a form may hold: grid, cluster of a
+// grouped model, cluster of Cox.
+cudaError_t smem_limits(int64_t smem[3]) {
     int dev = 0, optin = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (e != cudaSuccess) return e;
     // the kernels' static shared memory stays below these
     constexpr int64_t kStatic[3] = {16384, 24576, 45056};
     for (int c = 0; c < 3; ++c) smem[c] = std::max<int64_t>(0, optin - kStatic[c]);
-    return once_per_device(done, [&] {
-        for (int cox = 0; cox < 2; ++cox)
-            for (int where : {(int)kRowsShared, (int)kGroupsShared, (int)kGlobal})
-                for (int v = 0; v < 4; ++v) {
-                    const int cl = v & 1;
-                    const Kernel fn = pick(cox != 0, where, cl != 0, (v & 2) != 0);
-                    cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[cl ? 1 + cox : 0]);
-                    if (r == cudaSuccess && cl) r = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-                    if (r != cudaSuccess) return r;
-                }
-        return cudaSuccess;
+    return e;
+}
+
+// A kernel's attributes, set before its first launch on a device.
+cudaError_t kernel_attrs(Kernel fn, bool cox, int where, bool cl, bool form, int64_t smem) {
+    static std::atomic<uint64_t> done[2][3][4];
+    return once_per_device(done[cox][where][(cl ? 2 : 0) + (form ? 1 : 0)], [&] {
+        cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (r == cudaSuccess && cl) r = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        return r;
     });
 }
 
@@ -1221,17 +1218,16 @@ bool group_window_fits(bool cox, int64_t groups, int ctas, bool vals, int64_t sm
 
 cudaError_t group_window_limits(GroupWindowLimits* w) {
     w->cluster = 0;
-    cudaError_t e = kernel_attrs(w->smem);
+    cudaError_t e = smem_limits(w->smem);
+    // one for all: they have the same threads, and their shared memory is asked for in full
+    const Kernel fn = pick(false, kRowsShared, true, false);
+    if (e == cudaSuccess) e = kernel_attrs(fn, false, kRowsShared, true, false, w->smem[1]);
     if (e != cudaSuccess) return e;
     for (int C = kWindowCluster; C >= 1; C /= 2) {
-        bool fits = true;
-        for (int cox = 0; cox < 2; ++cox)
-            for (int where : {(int)kRowsShared, (int)kGroupsShared, (int)kGlobal}) {
-                cudaLaunchAttribute at[1];
-                const cudaLaunchConfig_t cfg = config(C, (size_t)w->smem[1 + cox], 0, at);
-                int n = 0;
-                fits &= cudaOccupancyMaxActiveClusters(&n, pick(cox != 0, where, true, cox == 0), &cfg) == cudaSuccess && n >= 1;
-            }
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = config(C, (size_t)w->smem[1], 0, at);
+        int n = 0;
+        const bool fits = cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n >= 1;
         cudaGetLastError();  // a size the device rejects is not an error here: try the next
         if (fits) {
             w->cluster = C;
@@ -1254,7 +1250,7 @@ cudaError_t launch_group_window(const GroupWindowParams& Q, bool cluster, int64_
     const int C = Q.ctas;
     if (C < 1 || C > (cluster ? kWindowCluster : kGroupWindowCtas)) return cudaErrorInvalidValue;
     int64_t limits[3];
-    cudaError_t e = kernel_attrs(limits);
+    cudaError_t e = smem_limits(limits);
     if (e != cudaSuccess) return e;
     const int64_t smem = limits[cluster ? 1 + (Q.cox != 0) : 0];
     const int64_t vals = Q.any_vals ? kStagedVals : 0, groups = group_bytes(Q.cox != 0, most_groups);
@@ -1270,7 +1266,10 @@ cudaError_t launch_group_window(const GroupWindowParams& Q, bool cluster, int64_
     GroupWindowParams R = Q;
     R.vals_at = (int32_t)(kStagedRows + state);
     const size_t bytes = (size_t)(R.vals_at + vals);
-    const Kernel fn = pick(Q.cox != 0, where, cluster, Q.cox ? Q.P.mixed != 0 : Q.any_long != 0);
+    const bool form = Q.cox ? Q.P.mixed != 0 : Q.any_long != 0;
+    const Kernel fn = pick(Q.cox != 0, where, cluster, form);
+    e = kernel_attrs(fn, Q.cox != 0, where, cluster, form, smem);
+    if (e != cudaSuccess) return e;
     if (cluster) {
         cudaLaunchAttribute at[1];
         const cudaLaunchConfig_t cfg = config(C, bytes, stream, at);
