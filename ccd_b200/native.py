@@ -239,7 +239,8 @@ class Matrix:
 
     def close(self):
         if getattr(self, "h", None):
-            lib().ccdb_matrix_destroy(self.h)
+            if self.ctx.h:  # the collector may have taken the context first, and all that is on it
+                lib().ccdb_matrix_destroy(self.h)
             self.h = None
 
     def __del__(self):
@@ -283,7 +284,8 @@ class Fit:
 
     def close(self):
         if getattr(self, "h", None):
-            lib().ccdb_fit_destroy(self.h)
+            if self.ctx.h:
+                lib().ccdb_fit_destroy(self.h)
             self.h = None
 
     def __del__(self):
