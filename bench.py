@@ -93,8 +93,9 @@ def parse():
     ap.add_argument("--strategy", choices=["auto", "levels", "speculative", "grid_levels", "resident"], default="auto",
                     help="sweep strategy of the independent-row engine (CCDB_SWEEP_*)")
     ap.add_argument("--trace", default=None,
-                    help="write a per-level timestamp trace of the last timed findMode's first "
-                         "sweep to this file (summarise with python -m ccd_b200.trace)")
+                    help="write a timestamp trace of the last timed findMode to this file: its first rounds "
+                         "(python -m ccd_b200.trace --rounds), or with --strategy grid_levels its first "
+                         "sweep by level (python -m ccd_b200.trace)")
     return ap.parse_args()
 
 

@@ -796,6 +796,23 @@ void Fit::release_batch_window() {
     batch_window.reset();
 }
 
+RoundTrace::RoundTrace(Context* c) : ctx(c), path(std::getenv("CCDB_TRACE_FILE")) {
+    if (!path) return;
+    d = static_cast<RoundStamp*>(ctx->alloc(sizeof(RoundStamp) * kTracedRounds));
+    check_cuda(cudaMemsetAsync(d, 0, sizeof(RoundStamp) * kTracedRounds, ctx->stream), "trace");
+}
+
+void RoundTrace::write() {
+    if (!d) return;
+    std::vector<RoundStamp> s(kTracedRounds);
+    check_cuda(cudaMemcpyAsync(s.data(), d, sizeof(RoundStamp) * s.size(), cudaMemcpyDeviceToHost, ctx->stream), "trace copy");
+    check_cuda(ctx->wait(), "trace copy");
+    if (FILE* fh = std::fopen(path, "wb")) {
+        std::fwrite(s.data(), sizeof(RoundStamp), s.size(), fh);
+        std::fclose(fh);
+    }
+}
+
 void Fit::find_mode_window(const ccdb_mode_args& a, int* flag, int* iters, double* obj, float* ms) {
     if (std::find(fixed.begin(), fixed.end(), uint8_t(0)) == fixed.end()) {
         // every coordinate is fixed: each cycle changes nothing, so the first
@@ -825,8 +842,10 @@ void Fit::find_mode_window(const ccdb_mode_args& a, int* flag, int* iters, doubl
     R.weighted = weighted ? 1 : 0;
     R.any_vals = window->any_vals ? 1 : 0;
     R.cluster = window->ctas;
+    RoundTrace trace(ctx);
+    R.trace = trace.d;
     check_cuda(cudaEventRecord(ctx->fev[0], stream), "event");
-    check_cuda(launch_window_sweep(R, ctx->window_smem, stream), "sweep launch");
+    check_cuda((trace.d ? launch_window_sweep_traced : launch_window_sweep)(R, ctx->window_smem, stream), "sweep launch");
     ++launches;
     check_cuda(cudaEventRecord(ctx->fev[1], stream), "event");
     // the host waits for the sweep before it queues the copy back: a device-to-host
@@ -837,6 +856,7 @@ void Fit::find_mode_window(const ccdb_mode_args& a, int* flag, int* iters, doubl
     check_cuda(cudaMemcpyAsync(&out, st, sizeof(out), cudaMemcpyDeviceToHost, stream), "status");
     check_cuda(ctx->wait(), "sweep");
     check_cuda(cudaEventElapsedTime(ms, ctx->fev[0], ctx->fev[1]), "elapsed");
+    trace.write();
     if (out.error != E_NONE)
         throw Error(CCDB_ERR_TIMEOUT, "device wait timed out (code " + std::to_string(out.error) +
                                           " at " + std::to_string(out.error_where) + ")");

@@ -142,7 +142,7 @@ void Fit::cox_release() {
     for (void* p : {(void*)cox.xbe, (void*)cox.grp, (void*)cox.rstrat, (void*)cox.denom, (void*)cox.D,
                     (void*)cox.S1, (void*)cox.S2, (void*)cox.nEv, (void*)cox.gfirst, (void*)cox.glast,
                     (void*)cox.grow, (void*)cox.tickets, (void*)cox.status, cox.tails,
-                    (void*)cox.batch_cols, (void*)cox.batch_out, (void*)cox.counters, cox.block_mem})
+                    (void*)cox.batch_cols, (void*)cox.batch_out, cox.block_mem})
         ctx->release(p);
 }
 
@@ -521,13 +521,11 @@ void Fit::find_mode_group_window(const ccdb_mode_args& a, int* flag, int* iters,
         while (n_cta < most && !group_window_fits(is_cox(), N, n_cta, any_vals, smem_grid)) ++n_cta;
     }
     ensure_group_window(n_cta, use_cluster);
-    if (!cox.counters) cox.counters = static_cast<int64_t*>(ctx->alloc(sizeof(int64_t) * 2));
     if (!beta_dirty_host) upload_beta();
     DevStatus zero{};
     zero.flag = R_FAIL;
     check_cuda(cudaMemcpyAsync(st, &zero, sizeof(zero), cudaMemcpyHostToDevice, stream), "status");
     check_cuda(cudaMemsetAsync(grid_bar, 0, sizeof(unsigned), stream), "barrier");
-    check_cuda(cudaMemsetAsync(cox.counters, 0, sizeof(int64_t) * 2, stream), "counters");
     GroupWindowParams Q{};
     Q.P = cox_params();
     Q.cox = is_cox() ? 1 : 0;
@@ -572,23 +570,25 @@ void Fit::find_mode_group_window(const ccdb_mode_args& a, int* flag, int* iters,
     Q.red = red;
     Q.grid_bar = grid_bar;
     Q.wait_limit_ns = wait_limit_ns;
-    Q.counters = cox.counters;
+    RoundTrace trace(ctx);
+    Q.trace = trace.d;
     check_cuda(cudaEventRecord(ctx->fev[0], stream), "event");
-    check_cuda(launch_group_window(Q, use_cluster, window->most_rows, window->most_groups, stream), "group sweep launch");
+    check_cuda((trace.d ? launch_group_window_traced : launch_group_window)(Q, use_cluster, window->most_rows,
+                                                                            window->most_groups, stream),
+               "group sweep launch");
     ++launches;
     check_cuda(cudaEventRecord(ctx->fev[1], stream), "event");
     if (is_cox()) cox_remaining(true);  // the groups' own denominators and sums, for the calls that follow
     check_cuda(ctx->wait(), "group sweep");  // the sweep is done before a copy is queued behind it
     DevStatus out{};
-    int64_t cnt[2] = {0, 0};
     check_cuda(cudaMemcpyAsync(&out, st, sizeof(out), cudaMemcpyDeviceToHost, stream), "status");
-    check_cuda(cudaMemcpyAsync(cnt, cox.counters, sizeof(cnt), cudaMemcpyDeviceToHost, stream), "counters");
     check_cuda(ctx->wait(), "group sweep");
     check_cuda(cudaEventElapsedTime(ms, ctx->fev[0], ctx->fev[1]), "elapsed");
+    trace.write();
     if (out.error != E_NONE)
         throw Error(CCDB_ERR_TIMEOUT, "device wait timed out (code " + std::to_string(out.error) + " at " +
                                           std::to_string(out.error_where) + ")");
-    nz_steps += cnt[0];
+    nz_steps += (int64_t)out.nonzero_steps;
     *flag = out.flag;
     *iters = out.iterations;
     *obj = out.objective;

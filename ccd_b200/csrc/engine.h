@@ -152,6 +152,17 @@ struct DevWindow {
     double2* heads = nullptr;
 };
 
+// CCDB_TRACE_FILE=<path>: the first rounds of a windowed sweep, written to the file
+// as they are (profiling aid; off by default).
+struct RoundTrace {
+    Context* ctx;
+    const char* path;
+    RoundStamp* d = nullptr;
+    explicit RoundTrace(Context* c);
+    ~RoundTrace() { ctx->release(d); }
+    void write();
+};
+
 // Device tables of the Breslow Cox engine (cox.cu).
 struct CoxDev {
     int64_t N = 0;  // risk-set groups
@@ -176,7 +187,6 @@ struct CoxDev {
     double *bden = nullptr, *bD = nullptr, *bS1 = nullptr, *bS2 = nullptr, *bnev = nullptr;
     uint8_t *bfirst = nullptr, *blast = nullptr;
     int64_t* brow = nullptr;
-    int64_t* counters = nullptr;  // nonzero steps and rounds of the windowed sweep
 };
 
 int64_t cox_group_rows(const std::vector<int32_t>& pid0, const std::vector<double>& time,

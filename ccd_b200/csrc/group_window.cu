@@ -539,6 +539,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
 
     double last = 0.0;
     long long moved = 0, rounds = 0;
+    Tracer tracer{Q.trace, rank == 0 && tid == kWorkers + 32};
     bool gave_up = false;  // a wait of this CTA ran out
 
     for (int iteration = 0;; ++iteration) {
@@ -599,6 +600,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
             for (;;) {
                 if (t.base >= n_active) break;
                 const bool flying = q < t.limit;
+                tracer.begin(t.base, t.limit - t.base, t.alone);
                 if (CL && me == 0) {
                     const unsigned bytes = __reduce_add_sync(kFull, flying ? pair_bytes(q, rec_of(q)) : 0u);
                     if (lane == 0) expect_sums(bytes);
@@ -610,6 +612,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 }
                 ++n_xch;
                 __syncthreads();
+                tracer.steps();
                 const bool quit = s_delta[kWindow] != 0.0;
                 // ---- every column up to the first that moves is behind us
                 const unsigned to = __reduce_min_sync(kFull, flying && s_delta[lane & (kWindow - 1)] != 0.0 ? (unsigned)q : 0xffffffffu);
@@ -624,6 +627,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 next_turn();
                 ahead.done();
                 __syncthreads();
+                tracer.end(__popc(moved_on), moves);
                 if (quit | (s_turn.stop != 0)) break;
             }
             ahead.done();
@@ -1112,9 +1116,8 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
         __syncthreads();
         for (int p = tid; p < n_active; p += kT) Q.hdelta[Q.cols[p].j] = Q.bh[p].y;
         if (wid == kWindow && lane == 0) {
-            Q.counters[0] = moved;
-            Q.counters[1] = rounds;
             Q.st->nonzero_steps = (unsigned long long)moved;
+            Q.st->rounds = (unsigned long long)rounds;
         }
     }
 }
@@ -1212,6 +1215,7 @@ cudaLaunchConfig_t config(int C, size_t smem, cudaStream_t stream, cudaLaunchAtt
 
 }  // namespace
 
+#ifndef CCDB_TRACE_ROUNDS
 bool group_window_fits(bool cox, int64_t groups, int ctas, bool vals, int64_t smem) {
     return kStagedRows + even(group_bytes(cox, (groups + ctas - 1) / ctas)) + (vals ? kStagedVals : 0) <= smem;
 }
@@ -1247,6 +1251,10 @@ cudaError_t launch_window_slices(const int32_t* rows, WinCol* cols, int32_t n_ac
 
 cudaError_t launch_group_window(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
                                 cudaStream_t stream) {
+#else
+cudaError_t launch_group_window_traced(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
+                                       cudaStream_t stream) {
+#endif
     const int C = Q.ctas;
     if (C < 1 || C > (cluster ? kWindowCluster : kGroupWindowCtas)) return cudaErrorInvalidValue;
     int64_t limits[3];

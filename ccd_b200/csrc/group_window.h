@@ -56,7 +56,7 @@ struct GroupWindowParams {
     double2* red;    // 2 x ctas: objective partials
     unsigned* grid_bar;
     long long wait_limit_ns;  // bound on any single wait for the other CTAs
-    int64_t* counters;  // [0]: nonzero steps, [1]: rounds
+    RoundStamp* trace;  // kTracedRounds, of a traced launch
 };
 
 // The largest cluster (16, 8, 4, 2, 1) that can be resident (0 if none), and the
@@ -75,5 +75,8 @@ cudaError_t launch_window_slices(const int32_t* rows, WinCol* cols, int32_t n_ac
 // `most_rows`, `most_groups`: the most that one CTA owns.
 cudaError_t launch_group_window(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
                                 cudaStream_t stream);
+// with Q.trace filled (group_window_trace.cu)
+cudaError_t launch_group_window_traced(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
+                                       cudaStream_t stream);
 
 }  // namespace ccdb

@@ -49,7 +49,7 @@ struct DevStatus {
     double loglik;
     double log_prior;
     unsigned long long nonzero_steps;  // coordinate steps that moved a coefficient (device sweeps)
-    unsigned long long pad2;
+    unsigned long long rounds;         // of a group model's windowed sweep
 };
 
 }  // namespace ccdb

@@ -290,6 +290,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
 
     double last = 0.0;
     unsigned long long moved = 0;
+    Tracer tracer{R.trace, rank == 0 && tid == kWorkers + 32};
     bool gave_up = false;  // a wait of this CTA ran out
 
     for (int iteration = 0;; ++iteration) {
@@ -372,6 +373,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 if (t.base >= n_active || t.stop) break;
                 const bool flying = q < t.limit;
                 const unsigned slots = __ballot_sync(kFull, flying);
+                tracer.begin(t.base, __popc(slots), t.alone);
                 const int turn = t.base & (kWindow - 1);
                 if (me == 0) {
                     if (CL && lane == 0) {
@@ -401,6 +403,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 settle();
                 if (CL) ++n_xch;
                 __syncthreads();
+                tracer.steps();
                 // ---- which steps stand, and what is in flight next
                 const unsigned moves = __ballot_sync(kFull, flying && s_delta[par][lane & (kWindow - 1)] != 0.0);
                 bool stands = flying && (s_holders[lane & (kWindow - 1)] & moves) == 0;
@@ -415,6 +418,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
                 next_turn();
                 ahead.done();
                 __syncthreads();
+                tracer.end(__popc(taken), __popc(taken & moves));
             }
             settle();
         } else {
@@ -593,6 +597,7 @@ int64_t all_bytes(int model, int64_t rows) { return (model == M_LOGISTIC ? 16 : 
 
 }  // namespace
 
+#ifndef CCDB_TRACE_ROUNDS
 bool window_share_fits(int64_t rows, bool vals, int64_t smem) {
     return kStagedRows + 8 * ((rows + 1) & ~int64_t(1)) + (vals ? kStagedVals : 0) <= smem;
 }
@@ -619,6 +624,9 @@ cudaError_t window_limits(int* cluster, int64_t* smem) {
 }
 
 cudaError_t launch_window_sweep(const WindowParams& R, int64_t smem, cudaStream_t stream) {
+#else
+cudaError_t launch_window_sweep_traced(const WindowParams& R, int64_t smem, cudaStream_t stream) {
+#endif
     const int C = R.cluster;
     if (C < 1 || C > kWindowCluster) return cudaErrorInvalidValue;
     const int64_t rows = (R.P.K + C - 1) / C;  // the most a CTA owns
@@ -631,7 +639,7 @@ cudaError_t launch_window_sweep(const WindowParams& R, int64_t smem, cudaStream_
     } else if (C == 1 && kStagedRows + 16 * rows + vals <= smem) {
         where = kPairShared;
         state = 16 * rows;
-    } else if (window_share_fits(rows, R.any_vals != 0, smem)) {
+    } else if (ccdb::window_share_fits(rows, R.any_vals != 0, smem)) {
         where = kShareShared;
         state = 8 * ((rows + 1) & ~int64_t(1));
     }

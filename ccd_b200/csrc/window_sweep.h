@@ -8,6 +8,14 @@
 
 namespace ccdb {
 
+// A round of a traced sweep (CTA 0's SM clock): its beginning, its steps known, its
+// end; the first position in flight, the columns in flight, taken, and moved, and
+// whether one ran alone.
+struct RoundStamp {
+    int64_t begin, steps, end, base, flying, taken, moved, alone;
+};
+constexpr int kTracedRounds = 4096;  // the first ones of a sweep
+
 // What a column's step needs beside its entries, by position.
 struct WinScal {
     double xjy, pvar, lambda, inv_var;  // sqrt(2 / pvar) of a Laplace prior, 1 / pvar of a normal one
@@ -28,6 +36,7 @@ struct WindowParams {
     int32_t vals_at;         // where the staged values lie in shared memory (the launcher's)
     int32_t cluster;         // CTAs
     int32_t pad;
+    RoundStamp* trace;       // kTracedRounds, of a traced launch
 };
 
 // The largest cluster (16, 8, 4, 2, 1) that can be resident with the most
@@ -37,5 +46,7 @@ cudaError_t window_limits(int* cluster, int64_t* smem);
 // (then `share` may be nullptr).
 bool window_share_fits(int64_t rows, bool vals, int64_t smem);
 cudaError_t launch_window_sweep(const WindowParams& R, int64_t smem, cudaStream_t stream);
+// with R.trace filled (window_trace.cu)
+cudaError_t launch_window_sweep_traced(const WindowParams& R, int64_t smem, cudaStream_t stream);
 
 }  // namespace ccdb

@@ -1,7 +1,11 @@
 """Summarise a sweep timestamp trace written by the engine.
 
-Setting ``CCDB_TRACE_FILE=<path>`` before a grid-wide level sweep makes libccdb write,
-for the first sweep, the schedule (segments, tasks) and per CTA segment the
+Setting ``CCDB_TRACE_FILE=<path>`` makes libccdb trace a fit's sweeps, each findMode
+attempt over the one before.  Of a windowed sweep, the default, the file holds CTA
+0's SM clock at three points of the first 4,096 rounds and what the round did;
+``python -m ccd_b200.trace --rounds <path> [sm_mhz]`` prints where a round's time
+goes and how many columns it takes.  Of a grid-wide level sweep it holds, for the
+first sweep, the schedule (segments, tasks) and per CTA segment the
 global timer at: wait start, level open, end of the CTA-wide phase, end of
 the warp phase, arrival.  ``python -m ccd_b200.trace <path>`` prints where the
 time of a sweep goes: level-to-level detection, per-level span, and the phase
@@ -72,6 +76,28 @@ def summarise(path: str) -> str:
     return "\n".join(out)
 
 
+ROUND = np.dtype([(n, "i8") for n in ("begin", "steps", "end", "base", "flying", "taken", "moved", "alone")])
+
+
+def summarise_rounds(path: str, sm_mhz: float = 1965.0) -> str:
+    t = np.fromfile(path, ROUND)
+    t = t[t["end"] != 0]
+    us = 1.0 / sm_mhz
+    cycle = np.flatnonzero(np.diff(t["base"]) < 0)
+    out = [f"rounds traced: {len(t)}, cycles ended: {len(cycle)}; columns taken {int(t['taken'].sum())}, "
+           f"moved {int(t['moved'].sum())}; {t['taken'].mean():.2f} taken of {t['flying'].mean():.2f} in flight a round"]
+    for name, sel in (("several columns", t["alone"] == 0), ("one column alone", t["alone"] != 0)):
+        s = t[sel]
+        if not len(s):
+            continue
+        moves = s["moved"] > 0
+        out.append(f"  {name}: {len(s)} rounds, median {np.median(s['end'] - s['begin']) * us:.2f} us: to the steps "
+                   f"{np.median(s['steps'] - s['begin']) * us:.2f}, to the end "
+                   f"{np.median((s['end'] - s['steps'])[moves]) * us if moves.any() else 0:.2f} where one moves, "
+                   f"{np.median((s['end'] - s['steps'])[~moves]) * us if (~moves).any() else 0:.2f} where none does")
+    return "\n".join(out)
+
+
 BATCH_PHASES = ("issue (stage, prefetch, metadata)", "gather + FP32 terms", "group reduction",
                 "step + update", "cp.async wait + barrier")
 
@@ -94,5 +120,7 @@ def summarise_batch(path: str, sm_mhz: float = 1965.0) -> str:
 if __name__ == "__main__":
     if sys.argv[1] == "--batch":
         print(summarise_batch(sys.argv[2], *(float(a) for a in sys.argv[3:4])))
+    elif sys.argv[1] == "--rounds":
+        print(summarise_rounds(sys.argv[2], *(float(a) for a in sys.argv[3:4])))
     else:
         print(summarise(sys.argv[1]))
