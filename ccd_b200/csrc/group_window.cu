@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
 
     double last = 0.0;
     long long moved = 0, rounds = 0;
-    Tracer tracer{Q.trace, rank == 0 && tid == kWorkers + 32};
+    Tracer tracer{Q.trace, rank == 0 && tid == kWorkers + 32, &s_turn.base};
     bool gave_up = false;  // a wait of this CTA ran out
 
     for (int iteration = 0;; ++iteration) {

@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
 
     double last = 0.0;
     unsigned long long moved = 0;
-    Tracer tracer{R.trace, rank == 0 && tid == kWorkers + 32};
+    Tracer tracer{R.trace, rank == 0 && tid == kWorkers + 32, &s_turn.base};
     bool gave_up = false;  // a wait of this CTA ran out
 
     for (int iteration = 0;; ++iteration) {

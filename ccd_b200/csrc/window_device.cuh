@@ -192,17 +192,21 @@ struct Ahead {
 struct Tracer {
     RoundStamp* to;
     bool mine;
+    const volatile int* gate;  // a word of shared memory, not below 0
     int n = 0;
     RoundStamp s{};
+    // the clock behind the last barrier: its reading depends on a word that is read there
+    // (by itself it moved in front of the barrier)
+    __device__ long long now() const { return *gate >= 0 ? clock64() : 0; }
     __device__ void begin(int base, int flying, int alone) {
-        s.begin = clock64();
+        s.begin = now();
         s.base = base;
         s.flying = flying;
         s.alone = alone;
     }
-    __device__ void steps() { s.steps = clock64(); }
+    __device__ void steps() { s.steps = now(); }
     __device__ void end(int taken, int moved) {
-        s.end = clock64();
+        s.end = now();
         s.taken = taken;
         s.moved = moved;
         if (mine && n < kTracedRounds) to[n] = s;
@@ -213,6 +217,7 @@ struct Tracer {
 struct Tracer {
     RoundStamp* to;
     bool mine;
+    const volatile int* gate;
     __device__ __forceinline__ void begin(int, int, int) {}
     __device__ __forceinline__ void steps() {}
     __device__ __forceinline__ void end(int, int) {}
