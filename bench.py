@@ -926,11 +926,8 @@ def run_cv(args, world, rank, local, collect=False):
     byts = cv_bytes(d, res_all)
     achieved = byts / (t / args.steps) / 1e9
     sweeps = [r["iterations"] for r in res_all]
-    lens = np.sort(np.diff(d.col_start))[:-1]
-    if mixed and group or lens.mean() > 640:  # the engine's rule for columns too long to step side by side
-        kernel = "batch_mixed_kernel<LOGISTIC>" if mixed else "batch_sweep_kernel<LOGISTIC>"
-    else:
-        kernel = "batch_window_kernel<LOGISTIC>"
+    kernel = {native.BATCH_WINDOWED: "batch_window_kernel<LOGISTIC>", native.BATCH_LOCKSTEP: "batch_mixed_kernel<LOGISTIC>",
+              native.BATCH_COLUMNS: "batch_sweep_kernel<LOGISTIC>"}[f.batch_engine(len(var), group, cluster)]
     line = {
         "metric": "converged fits/s", "value": fits / t, "unit": "fits/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * t / args.steps,
@@ -1412,7 +1409,7 @@ def run_variant(args, world, rank, local):
         """Device seconds, launches and cycles of one step."""
         if name == "fisher_l1":
             f.compute_fisher_information(cols)
-            return f.last_call_seconds(), 2 * ((len(cols) + 7) // 8), 1
+            return f.last_call_seconds(), 1, 1  # 10,000 rows fit in shared memory: one launch
         f.set_beta(cold)
         r = f.find_mode(margs)
         return r.device_seconds, r.kernel_launches, r.iterations
@@ -1470,7 +1467,7 @@ def run_variant(args, world, rank, local):
             b = fisher_bytes(d, cols)
             ach = b * args.steps / dev_t / 1e9
             roofline = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                        "peak_source": peak_kind, "algorithmic_bytes_per_launch": b / (2 * ((len(cols) + 7) // 8)),
+                        "peak_source": peak_kind, "algorithmic_bytes_per_launch": b,
                         "kernel": "fisher_dense_kernel (one launch a call)", "traffic": None}
         elif name == "mm_clr":
             b = mm_cycle_bytes(d) * cycles

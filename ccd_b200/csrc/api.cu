@@ -1548,6 +1548,35 @@ static bool batch_windowed(Context* ctx, const Fit* f, int n, int ctas, bool mix
     return !ctx->budget || ctx->in_use + bytes <= ctx->budget;
 }
 
+// The engine of a batch, and what its choice has found out.
+struct BatchRoute {
+    int32_t engine;
+    bool any_vals = false;
+    int ctas = 0, spill = 0;  // of the windowed engine
+};
+
+static BatchRoute batch_route(const Fit* f, const ccdb_batch_desc* b) {
+    const bool mixed = f->precision == CCDB_PRECISION_MIXED;
+    BatchRoute r{mixed ? CCDB_BATCH_LOCKSTEP : CCDB_BATCH_COLUMNS};
+    for (int j = f->offset_col0 ? 1 : 0; j < f->J; ++j) r.any_vals |= f->m->fmt[j] == F_SPARSE || f->m->fmt[j] == F_DENSE;
+    r.ctas = std::min(b->n_instances, f->ctx->n_sm);
+    check_cuda(batch_window_spill(f->K, mixed, r.any_vals, &r.spill), "batch sweep");
+    // a launch shape, and the trace of a column's phases, ask for the lockstep engine
+    if (mixed && (b->group || b->cluster || std::getenv("CCDB_BATCH_TRACE_FILE"))) return r;
+    if (batch_windowed(f->ctx, f, b->n_instances, r.ctas, mixed, r.spill)) r.engine = CCDB_BATCH_WINDOWED;
+    return r;
+}
+
+int ccdb_batch_engine(ccdb_fit* f, const ccdb_batch_desc* b, int32_t* engine) {
+    return guard([&] {
+        require(f && b && engine && b->n_instances > 0, "NULL argument");
+        if (f->model != M_LOGISTIC && f->model != M_POISSON)
+            throw Error(CCDB_ERR_UNSUPPORTED, "batched fits: logistic and Poisson models");
+        check_cuda(cudaSetDevice(f->ctx->device), "cudaSetDevice");
+        *engine = batch_route(f, b).engine;
+    });
+}
+
 int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_args* a, double* beta_out,
                          ccdb_batch_result* results, double* device_seconds) {
     return guard([&] {
@@ -1633,13 +1662,8 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
             if (hold[i] >= kKeyNoFold)
                 throw Error(CCDB_ERR_UNSUPPORTED, "mixed batched fits: held-out fold ids below 127");
         BatchWindowParams W{};
-        bool any_vals = false;
-        for (int j = f->offset_col0 ? 1 : 0; j < J; ++j) any_vals |= m->fmt[j] == F_SPARSE || m->fmt[j] == F_DENSE;
-        const int ctas = std::min(n, ctx->n_sm);
-        int spill = 0;
-        check_cuda(batch_window_spill(K, mixed, any_vals, &spill), "batch sweep");
-        const bool shaped = mixed && (b->group || b->cluster || trace_path);  // asks for the lockstep engine
-        const bool windowed = !shaped && batch_windowed(ctx, f, n, ctas, mixed, spill);
+        const BatchRoute route = batch_route(f, b);
+        const bool windowed = route.engine == CCDB_BATCH_WINDOWED;
         if (windowed) {
             f->ensure_batch_window();
             const DevWindow& w = *f->batch_window;
@@ -1652,12 +1676,12 @@ int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* b, const ccdb_mode_
             W.any_vals = w.any_vals ? 1 : 0;
             W.mixed = mixed ? 1 : 0;
             W.team = w.team;
-            W.ctas = ctas;
+            W.ctas = route.ctas;
             const size_t cols = (size_t)W.ctas * std::max(W.n_active, 1);
             W.scal = (WinScal*)keep(ctx->alloc(sizeof(WinScal) * cols));
             W.bh = (double2*)keep(ctx->alloc(sizeof(double2) * cols));
-            if (spill & 1) W.xbeta = (double*)keep(ctx->alloc(sizeof(double) * (size_t)K * W.ctas));
-            if (spill & 2) W.share = (double*)keep(ctx->alloc((mixed ? 4 : 8) * (size_t)K * W.ctas));
+            if (route.spill & 1) W.xbeta = (double*)keep(ctx->alloc(sizeof(double) * (size_t)K * W.ctas));
+            if (route.spill & 2) W.share = (double*)keep(ctx->alloc((mixed ? 4 : 8) * (size_t)K * W.ctas));
             P.queue = (int32_t*)keep(ctx->alloc(sizeof(int32_t)));
             check_cuda(cudaMemsetAsync(P.queue, 0, sizeof(int32_t), s), "batch queue");
             W.beta_out = P.beta = (double*)keep(ctx->alloc(sizeof(double) * (size_t)J * n));

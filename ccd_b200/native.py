@@ -27,6 +27,7 @@ ERR_INVALID, ERR_CUDA, ERR_UNSUPPORTED, ERR_BUDGET, ERR_TIMEOUT = -1, -2, -3, -4
 ALGORITHM_CCD, ALGORITHM_MM = 0, 1
 PRECISION_FP64, PRECISION_MIXED = 0, 1
 SWEEP_AUTO, SWEEP_LEVELS, SWEEP_SPECULATIVE, SWEEP_GRID_LEVELS, SWEEP_RESIDENT = 0, 1, 2, 3, 4
+BATCH_COLUMNS, BATCH_LOCKSTEP, BATCH_WINDOWED = 0, 1, 2
 
 
 class CcdbError(RuntimeError):
@@ -137,6 +138,7 @@ def lib() -> C.CDLL:
         L.ccdb_fit_model.argtypes = [_P, C.c_int64, C.c_int32, _P, _P, _P, _P, _P, C.POINTER(_FitDesc),
                                      _P, C.POINTER(_ModeArgs), _P, C.POINTER(_FitResult)]
         L.ccdb_batch_find_mode.argtypes = [_P, C.POINTER(_BatchDesc), C.POINTER(_ModeArgs), _P, _P, _P]
+        L.ccdb_batch_engine.argtypes = [_P, C.POINTER(_BatchDesc), C.POINTER(C.c_int32)]
         L.ccdb_column_gradient_hessian_noalloc.argtypes = [C.c_int32, C.c_int32, C.c_int64, _P, _P, _P,
                                                            C.c_double, _P, _P]
         L.ccdb_sweep_levels.argtypes = [C.c_int64, C.c_int32, _P, _P, _P, _P, _P, _P]
@@ -417,6 +419,14 @@ class Fit:
                 "updates": r.updates, "update_entries": r.update_entries,
                 "gradient_entries": r.gradient_entries} for r in res]
         return beta, out, secs.value
+
+    def batch_engine(self, n: int, group: int = 0, cluster: int = 0) -> int:
+        """The engine that batch_find_mode runs n instances on (BATCH_COLUMNS,
+        BATCH_LOCKSTEP or BATCH_WINDOWED)."""
+        bd = _BatchDesc(int(n), None, None, None, int(group), int(cluster))
+        e = C.c_int32()
+        _check(lib().ccdb_batch_engine(self.h, C.byref(bd), C.byref(e)))
+        return e.value
 
     def fold_instances(self, variances, holdout, row_fold, args: Optional[ModeFindingArguments] = None):
         """Cross-validation instances as standalone fits on this handle, for

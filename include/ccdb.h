@@ -285,11 +285,18 @@ typedef struct {
  * Each instance runs the sequential sweep of a standalone fit; instances do not
  * interact.  Logistic and Poisson models.  beta_out: n_instances x J.
  * Fits with short columns run the windowed sweep, one CTA an instance.  A
- * CCDB_PRECISION_MIXED fit with long columns, or whose caller gives a group or a
- * cluster, steps lockstep groups of batch->group instances through the columns
+ * CCDB_PRECISION_MIXED fit with long columns (how long depends on the instances
+ * and rows: ccdb_batch_engine), or whose caller gives a group or a cluster, steps lockstep groups of batch->group instances through the columns
  * (mixed fits: at most 16,777,215 rows; held-out fold ids below 127). */
 int ccdb_batch_find_mode(ccdb_fit* f, const ccdb_batch_desc* batch, const ccdb_mode_args* args,
                          double* beta_out, ccdb_batch_result* results, double* device_seconds);
+
+/* The engine that ccdb_batch_find_mode runs this batch on, by the fits, their columns
+ * and the context's memory as they are now. */
+#define CCDB_BATCH_COLUMNS 0  /* FP64, one column at a time */
+#define CCDB_BATCH_LOCKSTEP 1 /* mixed precision, groups of instances in lockstep */
+#define CCDB_BATCH_WINDOWED 2 /* several columns in flight */
+int ccdb_batch_engine(ccdb_fit* f, const ccdb_batch_desc* batch, int32_t* engine);
 
 /* --- allocation-free gradient (no reference counterpart) -------------------- */
 
