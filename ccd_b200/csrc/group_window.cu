@@ -75,6 +75,12 @@ using namespace win;
 // what shared memory holds: rows and groups, groups, neither
 enum Where : int { kRowsShared = 0, kGroupsShared = 1, kGlobal = 2 };
 
+// Cox: a Hessian below this part of the moment that it is left of is what rounding
+// leaves of zero: a column that is constant within every risk set carries no
+// information and gives (0, 0), which the reference's quotients have exactly and which
+// ends an unpenalised fit as ill-conditioned.
+constexpr double kCoxNoise = 256 * 2.220446049250313e-16;
+
 constexpr int kNarrow = 4;  // columns in flight after a step that moved; zero rounds double them
 
 // exp of a row's xBeta: FP64, or in the mixed precision of the Cox engine FP32.
@@ -843,6 +849,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                     if (CL) wait_sums(s_delta[kWindow]);
                     g = 0.0;
                     h = 0.0;
+                    double second = 0.0;  // Cox, a column with values: the sum of H2
                     if (CL) {  // lane l: CTA l
                         const double2* const from = &s_part[n_xch & 1][wid][0][0];
                         if (COX) {
@@ -857,6 +864,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                             if (lane < C) {
                                 g = gq.x;
                                 h = h2.x - (gq.y + 2.0 * carry * bt.x);
+                                second = h2.x;
                             }
                         } else if (lane < C) {
                             g = from[lane].x;
@@ -888,6 +896,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                                 const double h2 = ind ? gq.x : __ldcg(from + 3 * c + 2).x, carry = (s_flags[c] & 1) ? in : 0.0;
                                 g += gq.x;
                                 h += h2 - (gq.y + 2.0 * carry * bt.x);
+                                second += h2;
                                 in = s_flags[c] == 3 ? in + bt.y : bt.y;
                             } else {
                                 g += gq.x;
@@ -898,7 +907,14 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                     const double2 gh = warp_sum_of_two(g, h);
                     g = gh.x;
                     h = gh.y;
-                    if (r.c.n > 0) g -= r.s.xjy;
+                    bool noise = false;
+                    if (COX && !MX) {
+                        if (ind) second = g;
+                        else second = warp_sum_of_two(second, 0.0).x;
+                        noise = second > 0.0 && fabs(h) <= kCoxNoise * second && fabs(h) <= 1.7976931348623157e308;
+                    }
+                    if (noise) g = h = 0.0;
+                    else if (r.c.n > 0) g -= r.s.xjy;
                     else g = h = 0.0;  // an empty column gives (0, 0) (ModelSpecifics.hpp:720-723)
                     d = newton_quotient_step(g, h, b0, r.s.ptype, r.s.pvar, r.s.lambda, r.s.inv_var, b_var);
                     d = (d < -hd) ? -hd : (d > hd ? hd : d);  // apply_bounds; its new bound is not needed yet
