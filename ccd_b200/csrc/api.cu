@@ -742,14 +742,14 @@ void Fit::ensure_window(int ctas) {
     const size_t col_bytes = sizeof(WinCol) * n, slice_bytes = sizeof(WinSlice) * plan.slices.size();
     Parts p;
     const size_t at_cols = p.add(col_bytes), at_slices = p.add(slice_bytes), at_scal = p.add(sizeof(WinScal) * n),
-                 at_bh = p.add(sizeof(double2) * n), at_share = p.add(share ? sizeof(double) * K : 0);
+                 at_bh = p.add(sizeof(double2) * n);
     place_window(p.bytes, {at_cols, col_bytes, plan.cols.data()}, {at_slices, slice_bytes, plan.slices.data()});
     char* const d = static_cast<char*>(window->mem);
     window->cols = reinterpret_cast<WinCol*>(d + at_cols);
     window->slices = reinterpret_cast<WinSlice*>(d + at_slices);
     window->scal = reinterpret_cast<WinScal*>(d + at_scal);
     window->bh = reinterpret_cast<double2*>(d + at_bh);
-    window->share = share ? reinterpret_cast<double*>(d + at_share) : nullptr;
+    window->share = share ? xb_tmp : nullptr;  // free during a sweep: no xBeta is pending
     window->n_active = (int32_t)n;
     window->fixed = fixed;
     window->ctas = ctas;

@@ -137,7 +137,7 @@ struct DevWindow {
     WinSlice* slices = nullptr;
     WinScal* scal = nullptr;
     double2* bh = nullptr;
-    double* share = nullptr;  // K, where a CTA's rows do not fit its shared memory
+    double* share = nullptr;  // K (the fit's xb_tmp), where a CTA's rows do not fit its shared memory
     // group models: the CTAs' cuts, of the grouping that was current, and the grid
     // form's exchange buffers
     bool cluster = false;
