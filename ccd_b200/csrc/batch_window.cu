@@ -673,16 +673,19 @@ cudaError_t launch_batch_window(const BatchWindowParams& R, cudaStream_t stream)
     BatchWindowParams Q = R;
     Q.vals_at = (int32_t)(kStagedRows + state);
     const size_t smem = (size_t)(Q.vals_at + (R.any_vals ? kStagedVals : 0));
-    const Kernel fn = pick(R.P.model, R.mixed != 0, where, R.team);
-    static std::atomic<uint64_t> done[2][3][4];  // the attribute, before a kernel's first launch on a device
-    e = once_per_device(done[R.P.model == M_LOGISTIC][where][(R.mixed ? 2 : 0) + (R.team == 1 ? 1 : 0)], [&] {
+    static std::atomic<uint64_t> done{0};
+    e = once_per_device(done, [] {  // of all kernels (why: window.cu)
         int64_t dyn = 0;
         cudaError_t r = smem_limit(&dyn);
-        if (r == cudaSuccess) r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+        for (int model : {(int)M_LOGISTIC, (int)M_POISSON})
+            for (int team : {1, 4})
+                for (int v = 0; v < 6 && r == cudaSuccess; ++v)
+                    r = cudaFuncSetAttribute(pick(model, v & 1, v >> 1, team), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)dyn);
         return r;
     });
     if (e != cudaSuccess) return e;
-    fn<<<R.ctas, kT, smem, stream>>>(Q);
+    pick(R.P.model, R.mixed != 0, where, R.team)<<<R.ctas, kT, smem, stream>>>(Q);
     return cudaGetLastError();
 }
 

@@ -1204,12 +1204,19 @@ cudaError_t smem_limits(int64_t smem[3]) {
     return e;
 }
 
-// A kernel's attributes, set before its first launch on a device.
-cudaError_t kernel_attrs(Kernel fn, bool cox, int where, bool cl, bool form, int64_t smem) {
-    static std::atomic<uint64_t> done[2][3][4];
-    return once_per_device(done[cox][where][(cl ? 2 : 0) + (form ? 1 : 0)], [&] {
-        cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (r == cudaSuccess && cl) r = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+// The attributes of all kernels at the first launch on a device (why all: window.cu).
+cudaError_t kernel_attrs(const int64_t smem[3]) {
+    static std::atomic<uint64_t> done{0};
+    return once_per_device(done, [&] {
+        cudaError_t r = cudaSuccess;
+        for (int cox = 0; cox < 2; ++cox)
+            for (int where : {(int)kRowsShared, (int)kGroupsShared, (int)kGlobal})
+                for (int v = 0; v < 4 && r == cudaSuccess; ++v) {
+                    const int cl = v & 1;
+                    const Kernel fn = pick(cox != 0, where, cl != 0, (v & 2) != 0);
+                    r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[cl ? 1 + cox : 0]);
+                    if (r == cudaSuccess && cl) r = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                }
         return r;
     });
 }
@@ -1241,7 +1248,7 @@ cudaError_t group_window_limits(GroupWindowLimits* w) {
     cudaError_t e = smem_limits(w->smem);
     // one for all: they have the same threads, and their shared memory is asked for in full
     const Kernel fn = pick(false, kRowsShared, true, false);
-    if (e == cudaSuccess) e = kernel_attrs(fn, false, kRowsShared, true, false, w->smem[1]);
+    if (e == cudaSuccess) e = kernel_attrs(w->smem);
     if (e != cudaSuccess) return e;
     for (int C = kWindowCluster; C >= 1; C /= 2) {
         cudaLaunchAttribute at[1];
@@ -1292,7 +1299,7 @@ cudaError_t launch_group_window_traced(const GroupWindowParams& Q, bool cluster,
     const size_t bytes = (size_t)(R.vals_at + vals);
     const bool form = Q.cox ? Q.P.mixed != 0 : Q.any_long != 0;
     const Kernel fn = pick(Q.cox != 0, where, cluster, form);
-    e = kernel_attrs(fn, Q.cox != 0, where, cluster, form, smem);
+    e = kernel_attrs(limits);
     if (e != cudaSuccess) return e;
     if (cluster) {
         cudaLaunchAttribute at[1];

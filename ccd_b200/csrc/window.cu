@@ -566,14 +566,21 @@ cudaError_t smem_limit(int64_t* bytes) {
     return e;
 }
 
-// A kernel's attributes, set before its first launch on a device.
-cudaError_t kernel_attrs(Kernel fn, int model, int where, bool cl, bool wt, bool few) {
-    static std::atomic<uint64_t> done[2][4][8];
-    return once_per_device(done[model == M_LOGISTIC][where][(cl ? 4 : 0) + (wt ? 2 : 0) + (few ? 1 : 0)], [&] {
+// The attributes of all kernels at the first launch on a device: one that is set, and
+// its kernel loaded, while other contexts' sweeps run waits for them (a replay of 200
+// requests: p50 8 ms, 340 to 760 with each kernel's at its own first launch).
+cudaError_t kernel_attrs() {
+    static std::atomic<uint64_t> done{0};
+    return once_per_device(done, [] {
         int64_t dyn = 0;
         cudaError_t e = smem_limit(&dyn);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        for (int model : {(int)M_LOGISTIC, (int)M_POISSON})
+            for (int where : {(int)kAllShared, (int)kShareShared, (int)kGlobal, (int)kPairShared})
+                for (int v = 0; v < 8 && e == cudaSuccess; ++v) {
+                    const Kernel fn = pick(model, where, v & 1, v & 2, v & 4);
+                    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+                    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                }
         return e;
     });
 }
@@ -607,7 +614,7 @@ cudaError_t window_limits(int* cluster, int64_t* smem) {
     // one for all: they have the same threads, and their shared memory is asked for in full
     const Kernel fn = pick(M_LOGISTIC, kAllShared, true, false, false);
     cudaError_t e = smem_limit(smem);
-    if (e == cudaSuccess) e = kernel_attrs(fn, M_LOGISTIC, kAllShared, true, false, false);
+    if (e == cudaSuccess) e = kernel_attrs();
     if (e != cudaSuccess) return e;
     for (int C = kWindowCluster; C >= 1; C /= 2) {
         cudaLaunchAttribute at[1];
@@ -644,9 +651,8 @@ cudaError_t launch_window_sweep_traced(const WindowParams& R, int64_t smem, cuda
         state = 8 * ((rows + 1) & ~int64_t(1));
     }
     if (where == kGlobal && !R.share) return cudaErrorInvalidValue;
-    const bool few = R.n_active <= 4 * kWindow;
-    const Kernel fn = pick(R.P.model, where, C > 1, R.weighted != 0, few);
-    const cudaError_t e = kernel_attrs(fn, R.P.model, where, C > 1, R.weighted != 0, few);
+    const Kernel fn = pick(R.P.model, where, C > 1, R.weighted != 0, R.n_active <= 4 * kWindow);
+    const cudaError_t e = kernel_attrs();
     if (e != cudaSuccess) return e;
     WindowParams Q = R;
     Q.vals_at = (int32_t)(kStagedRows + state);
