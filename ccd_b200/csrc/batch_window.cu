@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kT, 1) batch_window_kernel(BatchWindowParams R
     };
     auto staged_all = [&](unsigned& phase) {
         if (phase < 2) return true;
-        const bool ok = __all_sync(kFull, wait_bytes(&s_bar[wid - kWindow], phase & 1, P.xch_wait_ns));
+        const bool ok = wait_bytes(&s_bar[wid - kWindow], phase & 1, P.xch_wait_ns);
         if (!ok) drain(&s_bar[wid - kWindow], phase & 1);  // what is under way lands before the CTA leaves
         phase = (phase & 1) ^ 1;
         return ok;

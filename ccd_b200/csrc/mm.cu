@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(kMT) mm_share_kernel(MMParams P) {
 // the conditional and Cox models): weight = hNWeight and denominator =
 // denomPid of the row's group; indicator columns drop x.  Latency of the gathers:
 // 2.6 million entries over 130,000 rows 25 us and the shares 4, 41 before.
+template <bool SHARES>
 __global__ void __launch_bounds__(kMT) mm_gh_kernel(MMParams P) {
     __shared__ double2 s_red[kMT / 32];
     const int j = blockIdx.x;
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(kMT) mm_gh_kernel(MMParams P) {
 #pragma unroll 4
     for (int64_t p = threadIdx.x; p < n; p += kMT) {
         const int64_t k = has_rows ? (int64_t)__ldg(P.rows + cb + p) : p;
-        const double r = P.share ? P.share[k] : mm_share(P, P.grp[k], k);
+        const double r = SHARES ? P.share[k] : mm_share(P, P.grp[k], k);
         if (ind) {
             g += r;
             h += r;
@@ -80,8 +81,12 @@ __global__ void __launch_bounds__(kMT) mm_gh_kernel(MMParams P) {
 cudaError_t launch_mm_gradient_hessian(const MMParams& P, cudaStream_t s) {
     if (P.J <= 0) return cudaSuccess;
     const int64_t blocks = (P.K + kMT - 1) / kMT;
-    if (P.share) mm_share_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), kMT, 0, s>>>(P);
-    mm_gh_kernel<<<P.J, kMT, 0, s>>>(P);
+    if (P.share) {
+        mm_share_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), kMT, 0, s>>>(P);
+        mm_gh_kernel<true><<<P.J, kMT, 0, s>>>(P);
+    } else {
+        mm_gh_kernel<false><<<P.J, kMT, 0, s>>>(P);
+    }
     return cudaGetLastError();
 }
 
