@@ -52,6 +52,10 @@ using namespace win;
 using bm::two_sum;
 
 constexpr int kLane = 4;  // staged entries per lane
+// A copy under way in a helper's `phase`: 2, and this too where the bound is below one
+// sleep of a wait, so that the test for a copy is the test for such a bound (one more
+// in front of each wait had cost 0.5 %).
+constexpr unsigned kBriefStep = 1u << 16;
 
 // A column has a team of T warps, so kWindow / T columns are in flight.
 template <int T>
@@ -214,11 +218,13 @@ __global__ void __launch_bounds__(kT, 1) batch_window_kernel(BatchWindowParams R
         const int to = stage_at<kStaged, W>(at);
         if (nr) bulk_copy(s_rows + to, P.rows + (r.c.cb & ~int64_t(3)), nr, bar);
         if (nv) bulk_copy(s_vals + to, P.vals + (r.c.vb & ~int64_t(1)), nv, bar);
-        phase += 2;  // bit 0: the parity to wait for; above: copies under way
+        phase += R.step;  // bit 0: the parity to wait for; above: copies under way
     };
     auto staged_all = [&](unsigned& phase) {
-        if (phase < 2) return true;
-        const bool ok = wait_bytes(&s_bar[wid - kWindow], phase & 1, P.xch_wait_ns);
+        bool ok;
+        if (phase - 2 < kBriefStep - 2) ok = wait_sleeping(&s_bar[wid - kWindow], phase & 1, P.xch_wait_ns);
+        else if (phase < 2) return true;
+        else ok = wait_looking(&s_bar[wid - kWindow], phase & 1, P.xch_wait_ns);
         if (!ok) drain(&s_bar[wid - kWindow], phase & 1);  // what is under way lands before the CTA leaves
         phase = (phase & 1) ^ 1;
         return ok;
@@ -671,6 +677,7 @@ cudaError_t launch_batch_window(const BatchWindowParams& R, cudaStream_t stream)
     if (e != cudaSuccess) return e;
     if ((where != kBoth && !R.xbeta) || (where == kNone && !R.share)) return cudaErrorInvalidValue;
     BatchWindowParams Q = R;
+    Q.step = 2 + (R.P.xch_wait_ns < win::kLookNs ? kBriefStep : 0);
     Q.vals_at = (int32_t)(kStagedRows + state);
     const size_t smem = (size_t)(Q.vals_at + (R.any_vals ? kStagedVals : 0));
     static std::atomic<uint64_t> done{0};

@@ -27,7 +27,7 @@ struct BatchWindowParams {
     int32_t mixed;
     int32_t ctas;           // instances that run at once
     int32_t team;           // warps to a column: 1 or 4
-    int32_t pad;
+    uint32_t step;          // what a copy under way adds to a helper's phase (the launcher's)
 };
 
 // What of a row's state does not fit in shared memory: bit 0 its xBeta, bit 1 its share.

@@ -94,18 +94,28 @@ __device__ __forceinline__ bool arrived(const uint64_t* bar, unsigned parity) {
         : "memory");
     return done != 0;
 }
-// false when the bytes have not all come within limit_ns
-__device__ __forceinline__ bool wait_bytes(const uint64_t* bar, unsigned parity, long long limit_ns) {
-    const bool brief = limit_ns < kLookNs;  // a bound below one sleep is kept by looks alone
-    if (!brief && arrived(bar, parity)) return true;  // nearly always; without this line a Poisson fit took 1.2 % longer
-    unsigned long long t0 = brief ? global_ns() : 0;
-    for (unsigned n = 0; !(brief ? landed(bar, parity) : arrived(bar, parity)); ++n)
-        if (brief || (n & 15u) == 15u) {
+// false when the bytes have not all come within limit_ns, by looks that sleep
+__device__ __forceinline__ bool wait_sleeping(const uint64_t* bar, unsigned parity, long long limit_ns) {
+    unsigned long long t0 = 0;
+    for (unsigned n = 0; !arrived(bar, parity); ++n)
+        if ((n & 15u) == 15u) {
             const unsigned long long t = global_ns();
             if (t0 == 0) t0 = t;
             if ((long long)(t - t0) > limit_ns) return false;
         }
     return true;
+}
+// the same for a bound below one sleep
+__device__ __forceinline__ bool wait_looking(const uint64_t* bar, unsigned parity, long long limit_ns) {
+    const unsigned long long t0 = global_ns();
+    while (!landed(bar, parity))
+        if ((long long)(global_ns() - t0) > limit_ns) return false;
+    return true;
+}
+__device__ __forceinline__ bool wait_bytes(const uint64_t* bar, unsigned parity, long long limit_ns) {
+    const bool brief = limit_ns < kLookNs;
+    if (!brief && arrived(bar, parity)) return true;  // nearly always; without this line a Poisson fit took 1.2 % longer
+    return brief ? wait_looking(bar, parity, limit_ns) : wait_sleeping(bar, parity, limit_ns);
 }
 __device__ __forceinline__ void init_bars(uint64_t* bars, int n) {
     for (int i = 0; i < n; ++i)
