@@ -389,7 +389,9 @@ void Fit::ensure_group_window(int ctas, bool cluster) {
     }
     // Where a CTA's groups begin.  Cox: at the nearest start of a stratum, when no CTA
     // then owns a quarter more than its even share, so that no stratum spans CTAs and
-    // a step needs no tail and head sums; else in even shares.
+    // a step needs no tail and head sums; else in even shares.  (The line weighs balance
+    // alone.  With fewer blocks a CTA than worker threads, 512, the longer share costs the
+    // scans nothing, and the two exchanges, 1,300 to 1,800 clocks each, are paid for it.)
     std::vector<GroupCut> cuts(ctas + 1);
     const int64_t N = is_cox() ? cox.NB : cox.N;
     std::vector<int64_t> first_group(ctas + 1);
@@ -497,7 +499,10 @@ void Fit::find_mode_group_window(const ccdb_mode_args& a, int* flag, int* iters,
     // 8, 16 and a grid of 32, 64, 148: conditional logistic, 4,000 sets, 512 entries a
     // column: 4.60 3.27 2.82 3.13 3.41 4.74; 20,000 sets, 2,601 entries: 26.8 14.3 4.78
     // 4.22 3.84 4.14; Cox, 20,000 rows, 199 entries: 2.75 2.94 2.52 4.47 4.73 6.35;
-    // 200,000 rows, 2,001 entries: 17.7 11.0 7.62 6.68 6.55 7.84.
+    // 200,000 rows, 2,001 entries: 17.7 11.0 7.62 6.68 6.55 7.84.  The line of 128 lies
+    // above where the forms cross.  200,000 rows, cluster of 16 and grid of 64, Cox: mean
+    // 800 7.13 and 7.58, 1,200 7.88 and 7.75, 2,000 9.98 and 8.76; conditional logistic:
+    // 200 1.00 and 1.37, 400 0.95 and 0.98, 800 1.58 and 1.21, 2,000 4.47 and 2.45.
     const int64_t N = is_cox() ? cox.NB : cox.N;
     int64_t total = 0, active = 0;
     for (int j = 0; j < J; ++j)
