@@ -76,7 +76,9 @@ __device__ __forceinline__ void add_terms(bool ind, bool weighted, double x, dou
         if (ind) h += wt * (1.0 - t);
         else h += weighted ? w * (t * x - t * t) : t * x - t * t;
     } else {
-        h += ind ? wt : wt * x;
+        // the weight last, as in the reference: a row of weight zero whose term overflows
+        // is not a number there either
+        h += ind ? wt : weighted ? w * (t * x) : t * x;
     }
 }
 
