@@ -26,8 +26,9 @@
 // The share is all that a gradient gathers: one 8-byte word, no exp and no
 // division per entry, computed once where the row changes.  It lives in shared
 // memory when the CTA's rows fit (8 bytes a row), with xBeta and the
-// denominator beside it when they fit too (24 bytes a row); otherwise they stay
-// in global memory, where only their CTA touches them.
+// denominator beside it when they fit too (24 bytes a row, 32 of a logistic fit, which
+// keeps exp(xBeta) as well), and the weights when there is room for these besides (8
+// more); otherwise they stay in global memory, where only their CTA touches them.
 //
 // Beside the sixteen warps with columns, four helper warps take everything that
 // looks ahead off the round's path: they copy a warp's next entries and records
@@ -100,6 +101,8 @@ struct Rows {
     double* ex;      // exp(xBeta), shared form of a logistic fit (a Poisson share is it)
     double2* xd;     // {xBeta, denominator}, shared form
     double2* row;    // the engine's row words of the CTA's first row
+    const double* wt;  // weights, wt_step words apart: beside the state, or in the row words
+    int wt_step;
 
     static constexpr bool kPair = WHERE == kAllShared || WHERE == kPairShared;  // xd holds the row
     __device__ __forceinline__ double p(int k) const {
@@ -108,7 +111,12 @@ struct Rows {
         const double e = exp(s.x);
         return (MODEL == M_LOGISTIC) ? e / s.y : e;
     }
-    __device__ __forceinline__ double weight(int k) const { return WT ? row[2 * (int64_t)k + 1].y : 1.0; }
+    // In shared memory where they fit beside the rest (8 bytes a row): read from the row
+    // words, a second cache line an entry, they cost weighted fits whose columns nearly all
+    // move more than the windows gave them (1,500 rows, 70 columns of 450 entries, normal
+    // prior: logistic 4.51 ms, from shared memory 4.40, Poisson 4.16 and 4.06; 3,000 rows,
+    // columns of 1,800: 6.3 and 5.7).
+    __device__ __forceinline__ double weight(int k) const { return WT ? wt[(int64_t)k * wt_step] : 1.0; }
     // the row words that an update will read, on their way to L1 ahead of it
     __device__ __forceinline__ void expect(int k) const {
         if (!kPair) asm volatile("prefetch.global.L1 [%0];" ::"l"(row + 2 * (int64_t)k));
@@ -180,6 +188,10 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
     const int even = (n_rows + 1) & ~1;
     rows.ex = s_state + even;
     rows.xd = reinterpret_cast<double2*>(s_state + (WHERE == kPairShared ? 0 : MODEL == M_LOGISTIC ? 2 : 1) * even);
+    const bool own_wt = WT && WHERE == kAllShared && R.weights_shared;
+    double* const s_wt = reinterpret_cast<double*>(rows.xd + n_rows);
+    rows.wt = own_wt ? s_wt : &rows.row[1].y;
+    rows.wt_step = own_wt ? 1 : 4;
     const WinSlice* const slices = R.slices + (int64_t)rank * n_active;
 
     // ---- the state of the rows, the records of the columns
@@ -190,6 +202,7 @@ __global__ void __launch_bounds__(kT, 1) window_sweep_kernel(WindowParams R) {
         if (WHERE != kPairShared) rows.share[k] = (MODEL == M_LOGISTIC) ? a.y / d : a.y;
         if (rows.kPair) rows.xd[k] = make_double2(a.x, d);
         if (WHERE == kAllShared && MODEL == M_LOGISTIC) rows.ex[k] = a.y;
+        if (own_wt) s_wt[k] = rows.row[2 * (int64_t)k + 1].y;
     }
 #pragma unroll 1
     for (int q = rank * kT + tid; q < n_active; q += C * kT) {
@@ -642,9 +655,13 @@ cudaError_t launch_window_sweep_traced(const WindowParams& R, int64_t smem, cuda
     const int64_t vals = R.any_vals ? kStagedVals : 0;
     int where = kGlobal;
     int64_t state = 0;
+    bool weights_shared = false;
     if (kStagedRows + all_bytes(R.P.model, rows) + vals <= smem) {
         where = kAllShared;
         state = all_bytes(R.P.model, rows);
+        const int64_t weights = 8 * ((rows + 1) & ~int64_t(1));
+        weights_shared = R.weighted && kStagedRows + state + weights + vals <= smem;
+        if (weights_shared) state += weights;
     } else if (C == 1 && kStagedRows + 16 * rows + vals <= smem) {
         where = kPairShared;
         state = 16 * rows;
@@ -658,6 +675,7 @@ cudaError_t launch_window_sweep_traced(const WindowParams& R, int64_t smem, cuda
     if (e != cudaSuccess) return e;
     WindowParams Q = R;
     Q.vals_at = (int32_t)(kStagedRows + state);
+    Q.weights_shared = weights_shared ? 1 : 0;
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = config(C, (size_t)(Q.vals_at + vals), stream, at);
     return cudaLaunchKernelEx(&cfg, fn, Q);

@@ -35,7 +35,7 @@ struct WindowParams {
     int32_t any_vals;        // some active column has values
     int32_t vals_at;         // where the staged values lie in shared memory (the launcher's)
     int32_t cluster;         // CTAs
-    int32_t pad;
+    int32_t weights_shared;  // the weights lie beside the rest of a row (the launcher's)
     RoundStamp* trace;       // kTracedRounds, of a traced launch
 };
 
