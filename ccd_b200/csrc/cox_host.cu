@@ -444,6 +444,9 @@ void Fit::ensure_group_window(int ctas, bool cluster) {
             while (c.hi + 1 < ctas && (cuts[c.hi].flags & 2) && (cuts[c.hi + 1].flags & 1)) ++c.hi;
         }
     }
+    // Cox: by a column's even share of the fullest CTA's rows (which columns are marked
+    // long, their true slices say)
+    for (const WinCol& c : cols) window->any_long |= is_cox() && c.n * window->most_rows > kGroupLong * K;
     const size_t n = cols.size();
     const size_t col_bytes = sizeof(WinCol) * n, cut_bytes = sizeof(GroupCut) * cuts.size(), grid = cluster ? 0 : 2 * ctas;
     Parts p;
@@ -578,9 +581,10 @@ void Fit::find_mode_group_window(const ccdb_mode_args& a, int* flag, int* iters,
     RoundTrace trace(ctx);
     Q.trace = trace.d;
     check_cuda(cudaEventRecord(ctx->fev[0], stream), "event");
-    check_cuda((trace.d ? launch_group_window_traced : launch_group_window)(Q, use_cluster, window->most_rows,
-                                                                            window->most_groups, stream),
-               "group sweep launch");
+    const auto launch = trace.d                         ? launch_group_window_traced
+                        : is_cox() && window->any_long ? launch_group_window_long
+                                                       : launch_group_window;
+    check_cuda(launch(Q, use_cluster, window->most_rows, window->most_groups, stream), "group sweep launch");
     ++launches;
     check_cuda(cudaEventRecord(ctx->fev[1], stream), "event");
     if (is_cox()) cox_remaining(true);  // the groups' own denominators and sums, for the calls that follow

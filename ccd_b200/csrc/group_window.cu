@@ -36,6 +36,15 @@
 // denominators: each thread takes a contiguous run of the CTA's groups, and the
 // CTAs exchange one tail sum, then one pair of head sums.
 //
+// Long columns run alone there too, but only while steps move (the last round's did, or
+// the column is not held at zero): a Cox column at rest is cheaper beside fifteen others
+// on one warp.  A warp's part of a slice misses a carry as a CTA's does.  And the rows of
+// a long column fall into one tie group by the hundred, whose changes its first entry
+// added one by one: a warp of one group hands its sum over.  150,637 rows, one stratum,
+// days as ties, 50 columns up to dense, 9 cycles: 43 ms; one warp a column 539, the kernel
+// before this one 203.  18,498 rows, 18 columns, six dense: 2.25 ms, 5.14, 7.7; 150,000
+// rows, 198 sparse columns and two dense: 3.10, 3.77, 42.7.
+//
 // Cox works on blocks, runs of groups up to one with events or to their stratum's
 // end: D counts only where there are events and S1, S2 change only there (cox_host.cu
 // builds them).  "Group" below is a block.
@@ -193,9 +202,9 @@ struct Owned {
     __device__ __forceinline__ bool last(int g) const { return WHERE != kGlobal ? strat_[g] & 2 : P->glast[g0 + g]; }
 };
 
-// MX: the mixed precision of the Cox engine.  LONG: a grouped model has a column that
-// may be long; without it the code of one costs the others (26,000 x 500 conditional
-// logistic, no long column: 3.17 ms, 3.4 with it).
+// MX: the mixed precision of the Cox engine.  LONG: a column may be long; without it the
+// code of one costs the others (26,000 x 500 conditional logistic, no long column: 3.17
+// ms, 3.4 with it; Cox, 12,000 x 60: 3.09 and 3.17).
 template <bool COX, int WHERE, bool CL, bool MX, bool LONG>
 __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q) {
     __shared__ Rec s_rec[4][kWindow];  // by position: (position / kWindow) & 3, slot
@@ -514,6 +523,125 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
         return warp_sum_of_two(g, h);
     };
 
+    // A column's partial sums of this CTA, Cox, from the warp that has them to every CTA.
+    auto send_cox = [&](double2 gq, double2 bt, double h2, bool ind) {
+        if (CL) {
+            if (lane < C) {
+                const unsigned par = n_xch & 1, bar = to_bar + par * 8u;
+                const unsigned a = to_part + (par * kWindow + wid) * kColumnBytes + rank * (unsigned)sizeof(double2);
+                send16(a, bar, gq.x, gq.y);
+                send16(a + kSumBytes, bar, bt.x, bt.y);
+                if (!ind) send16(a + 2 * kSumBytes, bar, h2, 0.0);
+            }
+        } else if (lane == 0) {
+            double2* to = Q.part + ((size_t)((n_xch & 1) * kWindow + wid) * C + rank) * 3;
+            __stcg(to, gq);
+            __stcg(to + 1, bt);
+            __stcg(to + 2, make_double2(h2, 0.0));
+        }
+    };
+
+    // Cox: the same of a long column, by all workers, sent by the warp that `takes` it.
+    // Each warp walks a part of whole passes of 32 entries with running sums that begin at
+    // its own first entry; what they miss of a stratum that the warps before it have begun
+    // is a carry, as it is from CTA to CTA: HQ grows by 2 c times the sum of S2 n1 over that
+    // stratum's entries here.
+    auto cox_alone = [&](const Rec& r, int at, bool takes) {
+        const int n = r.e.hi - r.e.lo, share = ((n + 32 * kWindow - 1) / (32 * kWindow)) * 32;
+        const int c0 = min(wid * share, n), c1 = min(c0 + share, n);
+        const bool ind = r.c.flags & 4;
+        const int first = (cut.flags & 1) ? cut.first : -2;
+        auto key_of = [&](int e) {
+            const int k = entry_row(r, at, e);
+            return own.stratum(k, own.group(k));
+        };
+        const int before = c0 > 0 && c0 < c1 ? key_of(c0 - 1) : -1;  // the stratum that the warp below ends in
+        double G = 0.0, H2 = 0.0, HQ = 0.0, B = 0.0, BW = 0.0, run = 0.0, A = 0.0;
+        float gs = 0.f, gc = 0.f, hs = 0.f, hc = 0.f;  // mixed: FP32 TwoSum partials of G and H2
+        int run_key = -1, key = -1;
+        bool joined = false;
+#pragma unroll 1
+        for (int e0 = c0; e0 < c1; e0 += 32) {
+            const int e = e0 + lane;
+            const bool in = e < c1;
+            double n1 = 0.0, n2 = 0.0, s1 = 0.0, s2 = 0.0;
+            float n1f = 0.f, n2f = 0.f;
+            key = 0x7fffffff;
+            if (in) {
+                const int k = entry_row(r, at, e), gr = own.group(k);
+                const double x = entry_val(r, at, e), ex = own.ex(k), w = P.weighted ? P.w[own.row0 + k] : 1.0;
+                key = own.stratum(k, gr);
+                if (gr >= 0) {
+                    s1 = own.s1(gr);
+                    s2 = own.s2(gr);
+                }
+                if (MX) {
+                    const float xf = (float)x, ef = (float)ex;
+                    n1f = P.weighted ? (float)w * (ef * xf) : ef * xf;
+                    if (!ind) n2f = n1f * xf;
+                    n1 = (double)n1f;
+                } else {
+                    n1 = P.weighted ? w * (ex * x) : ex * x;
+                    if (!ind) n2 = P.weighted ? w * (ex * x * x) : ex * x * x;
+                }
+            }
+            int prev = __shfl_up_sync(kFull, key, 1);
+            if (lane == 0) prev = run_key;
+            const unsigned starts = __ballot_sync(kFull, key != prev);
+            A = scan_up(n1, reach_down(starts, lane), 32);
+            if (!(starts & (kFull >> (31 - lane)))) A += run;
+            const double before_it = A - n1;
+            if (MX) {
+                const float s1f = (float)s1;
+                two_sum_f(gs, gc, n1f * s1f);
+                two_sum_f(hs, hc, n2f * s1f);
+            } else {
+                G += n1 * s1;
+                H2 += n2 * s1;
+            }
+            if (in) HQ += s2 * (A * A - before_it * before_it);  // risk-set sums: FP64
+            if (key == first) B += s2 * n1;
+            if (key == before) BW += s2 * n1;
+            if (e0 == c0) joined = __shfl_sync(kFull, key, 0) == before;
+            if (e0 + 32 < c1) {
+                run = __shfl_sync(kFull, A, 31);
+                run_key = __shfl_sync(kFull, key, 31);
+            }
+        }
+        if (MX) {
+            G = (double)gs + (double)gc;
+            H2 = (double)hs + (double)hc;
+        }
+        const int end = (c1 - c0 + 31) & 31;  // the part's last entry's lane
+        const double T = c0 < c1 ? __shfl_sync(kFull, A, end) : 0.0;
+        const int last_key = __shfl_sync(kFull, key, end);
+        const double s = warp_sum_of_four(G, H2, HQ, B), bw = warp_sum_of_two(BW, 0.0).x;
+        // by warp: G, H2, HQ, B, BW, T; s_dg: 1 the part begins within a stratum, 2 it lies in it; the last key
+        double* const mine = s_dd + 6 * wid;
+        if ((lane & 7) == 0) mine[lane >> 3] = s;
+        if (lane == 0) {
+            mine[4] = bw;
+            mine[5] = T;
+            s_dg[2 * wid] = joined ? (last_key == before ? 3 : 1) : 0;
+            s_dg[2 * wid + 1] = last_key;
+        }
+        workers_barrier();
+        if (!takes) return;
+        // lane w: warp w; what a part passes on, and what comes in to it
+        const double* const of = s_dd + 6 * (lane & (kWindow - 1));
+        const int fl = lane < kWindow ? s_dg[2 * lane] : 0, parts = n > 0 ? (n - 1) / share : 0;  // the last part
+        const unsigned starts = __ballot_sync(kFull, fl != 3);
+        const double pass = scan_up(of[5], reach_down(starts, lane), kWindow);
+        const double in = __shfl_up_sync(kFull, pass, 1), t = __shfl_sync(kFull, pass, parts);
+        const double carry = (fl & 1) ? in : 0.0;
+        const bool have = lane < kWindow;
+        const double u = warp_sum_of_four(have ? of[0] : 0.0, have ? of[1] : 0.0, have ? of[2] + 2.0 * carry * of[4] : 0.0,
+                                          have ? of[3] : 0.0);
+        const double2 gq = make_double2(__shfl_sync(kFull, u, 0), __shfl_sync(kFull, u, 16));
+        const double2 bt = make_double2(__shfl_sync(kFull, u, 24), n > 0 && s_dg[2 * parts + 1] == cut.last ? t : 0.0);
+        send_cox(gq, bt, __shfl_sync(kFull, u, 8), ind);
+    };
+
     // a worker's groups [ga, gz), and how far the scans over them reach
     const int per_worker = ((own.n_groups + kWorkers - 1) / kWorkers) | 1;  // odd: no bank conflicts
     const int ga = min(tid * per_worker, own.n_groups), gz = wid < kWindow ? min(ga + per_worker, own.n_groups) : ga;
@@ -591,7 +719,12 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 t.base = __reduce_min_sync(kFull, q);
                 t.limit = min(t.base + width, n_active);
                 if (LONG) {
-                    const int first = __reduce_min_sync(kFull, q < n_active && long_column(rec_of(q)) ? q : 0x7fffffff);
+                    bool alone = false;
+                    if (q < n_active && long_column(rec_of(q))) {
+                        const Rec& r = rec_of(q);
+                        alone = !COX || width == kNarrow || r.s.ptype != 1 || r.bh.x != 0.0;
+                    }
+                    const int first = __reduce_min_sync(kFull, alone ? q : 0x7fffffff);
                     t.alone = first == t.base;
                     t.limit = t.alone ? t.base + 1 : min(t.limit, first);
                 }
@@ -652,7 +785,13 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                 const bool mine = pos < now.limit;
                 const Rec& r = rec_of(pos);
                 double d = 0.0, hd = 0.0, b0 = 0.0, g = 0.0, h = 0.0;
-                if (LONG && now.alone) {
+                if (LONG && COX && now.alone) {
+                    cox_alone(rec_of(now.base), now.base, mine);
+                    if (mine) {
+                        b0 = r.bh.x;
+                        hd = r.bh.y;
+                    }
+                } else if (LONG && now.alone) {
                     const double2 gh = gather_alone(rec_of(now.base), now.base, mine);
                     if (mine) {
                         b0 = r.bh.x;
@@ -760,20 +899,7 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                         const double Bv = __shfl_sync(kFull, other, 8);
                         const double2 gq = make_double2(__shfl_sync(kFull, s, 0), __shfl_sync(kFull, other, 0));
                         const double h2 = __shfl_sync(kFull, s, 8);
-                        if (CL) {
-                            if (lane < C) {
-                                const unsigned par = n_xch & 1, bar = to_bar + par * 8u;
-                                const unsigned a = to_part + (par * kWindow + wid) * kColumnBytes + rank * (unsigned)sizeof(double2);
-                                send16(a, bar, gq.x, gq.y);
-                                send16(a + kSumBytes, bar, Bv, T);
-                                if (!ind) send16(a + 2 * kSumBytes, bar, h2, 0.0);
-                            }
-                        } else if (lane == 0) {
-                            double2* to = Q.part + ((size_t)((n_xch & 1) * kWindow + wid) * C + rank) * 3;
-                            __stcg(to, gq);
-                            __stcg(to + 1, make_double2(Bv, T));
-                            __stcg(to + 2, make_double2(h2, 0.0));
-                        }
+                        send_cox(gq, make_double2(Bv, T), h2, ind);
                     } else {
                         double run1 = 0.0, run2 = 0.0;
                         int run_key = -1;
@@ -986,6 +1112,15 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                             }
                         }
                         s_dg[tid] = gr;
+                        if (LONG) {  // a warp within one group has its sum ready for the head of the run
+                            const int gr0 = __shfl_sync(kFull, gr, 0);
+                            const bool one = __all_sync(kFull, gr >= 0 && gr == gr0);
+                            if (one) {
+                                const double t = warp_sum_of_two(s_dd[tid], 0.0).x;
+                                if (lane == 0) s_run[wid] = t;
+                            }
+                            if (lane == 0) s_first[wid] = one ? gr : -1;
+                        }
                         workers_barrier();
                         if (gr >= 0) {
                             int b = tid - 1;
@@ -994,6 +1129,11 @@ __global__ void __launch_bounds__(kT, 1) group_window_kernel(GroupWindowParams Q
                                 double v = own.den(gr);
                                 const int most = min(kWorkers, n - e0);
                                 for (int i = tid; i < most; ++i) {
+                                    if (LONG && (i & 31) == 0 && s_first[i >> 5] == gr) {
+                                        v = v + s_run[i >> 5];
+                                        i += 31;
+                                        continue;
+                                    }
                                     if (s_dg[i] < 0) continue;
                                     if (s_dg[i] != gr) break;
                                     v = v + s_dd[i];
@@ -1168,21 +1308,29 @@ __global__ void window_slices_kernel(const int32_t* rows, WinCol* cols, int32_t 
 using Kernel = void (*)(GroupWindowParams);
 
 template <bool COX, bool CL, bool MX, bool LONG>
-Kernel pick(int where) {
+Kernel pick_where(int where) {
     switch (where) {
     case kRowsShared: return group_window_kernel<COX, kRowsShared, CL, MX, LONG>;
     case kGroupsShared: return group_window_kernel<COX, kGroupsShared, CL, MX, LONG>;
     default: return group_window_kernel<COX, kGlobal, CL, MX, LONG>;
     }
 }
-// `form`: the mixed precision of Cox, or a grouped model's long columns
-Kernel pick(bool cox, int where, bool cl, bool form) {
-    if (cox) {
-        if (form) return cl ? pick<true, true, true, false>(where) : pick<true, false, true, false>(where);
-        return cl ? pick<true, true, false, false>(where) : pick<true, false, false, false>(where);
-    }
-    if (form) return cl ? pick<false, true, false, true>(where) : pick<false, false, false, true>(where);
-    return cl ? pick<false, true, false, false>(where) : pick<false, false, false, false>(where);
+template <bool COX, bool MX, bool LONG>
+Kernel pick_form(int where, bool cl) {
+    return cl ? pick_where<COX, true, MX, LONG>(where) : pick_where<COX, false, MX, LONG>(where);
+}
+// `mixed`: the mixed precision of Cox; `longs`: a column may be long.  The kernels of Cox
+// fits with long columns are a compilation of their own (group_window_long.cu): loaded
+// with the others they cost every process's first group fit 12 ms.
+Kernel pick(bool cox, int where, bool cl, bool mixed, bool longs) {
+#ifndef CCDB_COX_LONG
+    if (!cox) return longs ? pick_form<false, false, true>(where, cl) : pick_form<false, false, false>(where, cl);
+    if (!longs) return mixed ? pick_form<true, true, false>(where, cl) : pick_form<true, false, false>(where, cl);
+#endif
+#if defined(CCDB_COX_LONG) || defined(CCDB_TRACE_ROUNDS)
+    if (cox && longs) return mixed ? pick_form<true, true, true>(where, cl) : pick_form<true, false, true>(where, cl);
+#endif
+    return nullptr;
 }
 
 constexpr int64_t kStagedRows = 2 * kWindow * kStage * sizeof(int32_t);
@@ -1211,9 +1359,10 @@ cudaError_t kernel_attrs(const int64_t smem[3]) {
         cudaError_t r = cudaSuccess;
         for (int cox = 0; cox < 2; ++cox)
             for (int where : {(int)kRowsShared, (int)kGroupsShared, (int)kGlobal})
-                for (int v = 0; v < 4 && r == cudaSuccess; ++v) {
+                for (int v = 0; v < (cox ? 8 : 4) && r == cudaSuccess; ++v) {
                     const int cl = v & 1;
-                    const Kernel fn = pick(cox != 0, where, cl != 0, (v & 2) != 0);
+                    const Kernel fn = pick(cox != 0, where, cl != 0, (v & 4) != 0, (v & 2) != 0);
+                    if (!fn) continue;
                     r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[cl ? 1 + cox : 0]);
                     if (r == cudaSuccess && cl) r = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
                 }
@@ -1238,7 +1387,7 @@ cudaLaunchConfig_t config(int C, size_t smem, cudaStream_t stream, cudaLaunchAtt
 
 }  // namespace
 
-#ifndef CCDB_TRACE_ROUNDS
+#if !defined(CCDB_TRACE_ROUNDS) && !defined(CCDB_COX_LONG)
 bool group_window_fits(bool cox, int64_t groups, int ctas, bool vals, int64_t smem) {
     return kStagedRows + even(group_bytes(cox, (groups + ctas - 1) / ctas)) + (vals ? kStagedVals : 0) <= smem;
 }
@@ -1247,7 +1396,7 @@ cudaError_t group_window_limits(GroupWindowLimits* w) {
     w->cluster = 0;
     cudaError_t e = smem_limits(w->smem);
     // one for all: they have the same threads, and their shared memory is asked for in full
-    const Kernel fn = pick(false, kRowsShared, true, false);
+    const Kernel fn = pick(false, kRowsShared, true, false, false);
     if (e == cudaSuccess) e = kernel_attrs(w->smem);
     if (e != cudaSuccess) return e;
     for (int C = kWindowCluster; C >= 1; C /= 2) {
@@ -1274,6 +1423,9 @@ cudaError_t launch_window_slices(const int32_t* rows, WinCol* cols, int32_t n_ac
 
 cudaError_t launch_group_window(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
                                 cudaStream_t stream) {
+#elif defined(CCDB_COX_LONG)
+cudaError_t launch_group_window_long(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
+                                     cudaStream_t stream) {
 #else
 cudaError_t launch_group_window_traced(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
                                        cudaStream_t stream) {
@@ -1297,8 +1449,8 @@ cudaError_t launch_group_window_traced(const GroupWindowParams& Q, bool cluster,
     GroupWindowParams R = Q;
     R.vals_at = (int32_t)(kStagedRows + state);
     const size_t bytes = (size_t)(R.vals_at + vals);
-    const bool form = Q.cox ? Q.P.mixed != 0 : Q.any_long != 0;
-    const Kernel fn = pick(Q.cox != 0, where, cluster, form);
+    const Kernel fn = pick(Q.cox != 0, where, cluster, Q.P.mixed != 0, Q.any_long != 0);
+    if (!fn) return cudaErrorInvalidValue;
     e = kernel_attrs(limits);
     if (e != cudaSuccess) return e;
     if (cluster) {

@@ -13,7 +13,7 @@
 namespace ccdb {
 
 constexpr int kGroupWindowCtas = 160;  // most CTAs of the grid form
-constexpr int64_t kGroupLong = 512;    // a column with a larger slice runs alone (grouped models)
+constexpr int64_t kGroupLong = 512;    // a column with a larger slice may run alone
 
 // What one CTA owns: rows [row0, next row0) and groups [g0, next g0); a sentinel
 // follows the last CTA's.  Strata (Cox): `first` and `last` are those of its
@@ -44,7 +44,7 @@ struct GroupWindowParams {
     double tol;
     double ll_fixed;
     int32_t any_vals;  // some active column has values
-    int32_t any_long;  // some may be marked long (grouped models)
+    int32_t any_long;  // some may be marked long
     int32_t meet;      // Cox: a stratum spans CTAs, which then exchange tail and head sums
     int32_t chain;     // lanes that a carry may pass over (1 + the CTAs within one stratum in a row)
     int32_t vals_at;   // where the staged values lie in shared memory (the launcher's)
@@ -75,6 +75,9 @@ cudaError_t launch_window_slices(const int32_t* rows, WinCol* cols, int32_t n_ac
 // `most_rows`, `most_groups`: the most that one CTA owns.
 cudaError_t launch_group_window(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
                                 cudaStream_t stream);
+// Cox with Q.any_long (group_window_long.cu)
+cudaError_t launch_group_window_long(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
+                                     cudaStream_t stream);
 // with Q.trace filled (group_window_trace.cu)
 cudaError_t launch_group_window_traced(const GroupWindowParams& Q, bool cluster, int64_t most_rows, int64_t most_groups,
                                        cudaStream_t stream);
